@@ -197,6 +197,19 @@ __host__ __device__ __forceinline__ double own_exp(double x) {
     return ldexp(p, (int)kf);
 }
 
+// The pieces of a bounded wait on a word in global memory.
+__device__ __forceinline__ uint64_t global_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // Non-negative doubles order like their bit patterns.
 __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *addr, double v) {
     if (!(v >= 0.0)) return;
@@ -302,6 +315,8 @@ struct cw_lattice_s {
     int build_plans();
 };
 
+namespace cw { struct Resident64; }
+
 struct cw_field_s {
     cw::HandleStream hs;             // its stream and last error
     cw::Geom g;
@@ -322,6 +337,7 @@ struct cw_field_s {
     void *stats = nullptr;           // per-history solve state (device)
     cw::Span *d_span = nullptr;
     void *dc_cache = nullptr;        // plans and solver of the FP32 solve (field.cu)
+    cw::Resident64 *resident = nullptr;  // tilings and scratch of the FP64 solve on chip (field64.cu)
     cw_field_s *adjoint = nullptr;   // twin of cw_field_relax_adjoint, made on its first call
     cw::Plan inflow_plan;            // every site, for the inflow enqueued inside a step
     int alloc_fp32();

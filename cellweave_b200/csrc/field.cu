@@ -24,27 +24,6 @@ using namespace cw;
 
 namespace {
 
-struct RelaxState {
-    unsigned long long moved[2];  // max |change| of the red and the black half-sweep
-    unsigned long long resid;     // max projected residual
-    double omega;
-    double tol;
-    int64_t sweeps;               // sweeps taken, final once done
-    int32_t done;                 // 0 running, 1 converged
-    int32_t stop;
-    double last_change;
-    double last_resid;
-    int64_t inner;                // FP32 sweeps taken (defect correction)
-    // the error estimate of the defect-correction solve (the wide sweeps'
-    // apply): the largest |correction| of the last outer iteration and the
-    // largest |c| it left, as the bits of non-negative doubles (atomic max),
-    // the previous iteration's largest correction, and the bound asked
-    unsigned long long corr;
-    unsigned long long cmax;
-    double prev_corr;
-    double etol;
-};
-
 // (a history holds fewer than 2^31 pixels: 32-bit division is enough)
 __device__ __forceinline__ void locate(const int4 dm, int64_t local, int &x, int &y, int &z) {
     const uint32_t l = (uint32_t)local, w = (uint32_t)dm.x, h = (uint32_t)dm.y;
@@ -1253,6 +1232,7 @@ int cw_field_destroy(cw_field f) {
     dfree(st);
     if (f->adjoint) cw_field_destroy(f->adjoint);
     f->inflow_plan.release();
+    resident64_release(f);
     f->g.release();
     f->hs.release();
     delete f;
@@ -1470,13 +1450,18 @@ int cw::field_relax(cw_field_s *f, const cw_relax_opts *opts, const double *omeg
     }
     RelaxState *d_st = (RelaxState *)f->stats;
     CW_CUDA(cudaMemcpyAsync(d_st, hs.data(), sizeof(RelaxState) * nh, cudaMemcpyHostToDevice, stream()));
-    if (o.precision == CW_FP64) rc = relax_fp64(f, o, spans, d_st, hs);
-    else rc = relax_fp32dc(f, o, d_st, hs);
+    bool resident = false;
+    if (o.precision == CW_FP64) {
+        rc = relax64_resident(f, o, spans, d_st, hs, &resident);
+        if (rc == CW_OK && !resident) rc = relax_fp64(f, o, spans, d_st, hs);
+    } else {
+        rc = relax_fp32dc(f, o, d_st, hs);
+    }
     if (rc != CW_OK) return rc;
     // final residual of every history, for the report (the defect-correction
-    // loop ends on one it has just computed)
+    // loop and the resident FP64 solve end on one they have just computed)
     std::vector<double> res(nh);
-    if (o.precision == CW_FP32_DC) {
+    if (o.precision == CW_FP32_DC || resident) {
         for (uint32_t k = 0; k < nh; ++k) res[k] = hs[k].last_resid;
     } else if ((rc = cw_field_residual(f, res.data())) != CW_OK) {
         return rc;

@@ -17,7 +17,34 @@ struct FieldView {
     int floor;  // 1: updates floored at zero, residual projected (the reference); 0: a linear solve
 };
 
+// The state of one history's solve, on the device.
+struct RelaxState {
+    unsigned long long moved[2];  // max |change| of the red and the black half-sweep
+    unsigned long long resid;     // max projected residual
+    double omega;
+    double tol;
+    int64_t sweeps;               // sweeps taken, final once done
+    int32_t done;                 // 0 running, 1 converged
+    int32_t stop;
+    double last_change;
+    double last_resid;
+    int64_t inner;                // FP32 sweeps taken (defect correction)
+    // the error estimate of the defect-correction solve (the wide sweeps'
+    // apply): the largest |correction| of the last outer iteration and the
+    // largest |c| it left, as the bits of non-negative doubles (atomic max),
+    // the previous iteration's largest correction, and the bound asked
+    unsigned long long corr;
+    unsigned long long cmax;
+    double prev_corr;
+    double etol;
+};
+
 FieldView view(cw_field_s *f);
+// The FP64 relax kept on chip (field64.cu), where every history's tiles are
+// resident on the device at once; *served false: they are not, nothing has run.
+int relax64_resident(cw_field_s *f, const cw_relax_opts &o, const std::vector<Span> &spans, RelaxState *d_st,
+                     std::vector<RelaxState> &hs, bool *served);
+void resident64_release(cw_field_s *f);
 int field_hold_bath_device(cw_field_s *f, const uint8_t *d_open, int hist, double value);
 
 // The source side of a pixel's balance after `t` (d*sum or d*lap - decay*c):

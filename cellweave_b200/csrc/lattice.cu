@@ -340,18 +340,6 @@ struct PassScratch {
 // third; then the pass keys
 enum { CTL_COUNT = 0, CTL_BAR = 3, CTL_GEN = 32, CTL_ERR = 48, CTL_ROUNDS = 49, CTL_SEQ = 50, CTL_KEYS = 64 };
 
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
 // A barrier over the whole (co-resident, cooperatively launched) grid whose
 // wait gives up after S.barrier_ns; false then, on every thread of the block.
 // The block S.withhold (a failure test) never arrives and returns false.
