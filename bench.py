@@ -522,14 +522,14 @@ def shape_record(L, cfg, steps, warm, peak):
     tuned = sim.tuning()
     sites = int(sum(w * h * d for w, h, d in cfg["dims"]))
     volume = any(d > 1 for _, _, d in cfg["dims"])
-    depth = 2 if volume else tuned["depth"]
+    depth = tuned["depth"]
     lm = sor_launch_ms(L, sim.field_handle(0), depth, tuned["window"])
-    # a volume's launch is one sweep (two half-sweeps) of tiles marched along
-    # z (k_sor32_vol); a plane's, `depth` half-sweeps on chip: 16 B per site a launch
+    # a launch is `depth` half-sweeps: of tiles marched along z in a volume
+    # (k_sor32_vol), of windows on chip in a plane: 16 B per site a launch
     alg = sites * SOR_BYTES_PER_SITE_PASS
     gbs = alg / (lm / 1e3) / 1e9
-    rec["sor"] = {"kernel": ("k_sor32_vol<2, %d> (64x%d tiles marched along z, one sweep per launch)" %
-                             ((16, 16) if tuned["window"] == 1 else (32, 32))) if volume else
+    rec["sor"] = {"kernel": ("k_sor32_vol (64x%d tiles marched along z, %d half-sweeps per launch)" %
+                             (16 if tuned["window"] == 1 else 32, depth)) if volume else
                   f"k_sor32_wide<{depth}> ({depth} half-sweeps per launch on chip)",
                   "launch_ms": round(lm, 4), "alg_bytes_per_launch": int(alg), "achieved_gbs": round(gbs, 1),
                   "frac": round(gbs / peak, 3)}

@@ -423,36 +423,74 @@ __global__ void k_sor32_half(float *__restrict__ dlt, const float *__restrict__ 
 // ------------------------------------------------------------------ volumes, blocked
 
 // Temporal blocking in a volume (2.5-D: tiles across x and y marched along
-// z).  A block takes a VX x VY tile of a history's columns over a chunk of
-// its slices [z0, z1) and runs S <= D half-sweeps on it in one pass along z:
-// at step t, stage s (the s-th half-sweep) updates slice t - 2 (s - 1), its
-// pixels of that half-sweep's colour, in place in a ring of slices in shared
-// memory.  Two slices between stages keep every read at the right level:
-// stage s reads slices p - 1, p, p + 1 after stage s - 1 (slice p + 1 was
-// done a step ago, slice p - 1 holds stage s's own colour, which stage s
-// does not read), and no slice a stage reads is written in the same step.
-// The tile's halo is D pixels across x and y and D slices along z beyond
-// the chunk; what lies beyond the loaded slices or the tile reads as zero,
-// exact at the history's border and an error that moves in one ring per
-// half-sweep inside it, so every pixel D or more from such an edge equals S
-// in-place half-sweeps of the whole history (as k_sor32_half gives them,
-// to the bit: the same sums in the same order).  A thread owns a pair of
-// columns (one pixel of each colour per slice); the next slice is brought
-// into registers while the stages run, then into the ring, one barrier a
-// step.  The stage's coefficients are read from global memory (L1 keeps a
-// slice's for the S steps that use it).
+// z).  A block takes a VX x 2 NW tile of a history's columns over a chunk of
+// its slices [z0, z1) and runs S <= VD half-sweeps on it in one pass along z:
+// at step t, stage s (the s-th half-sweep) updates slice t - (s - 1), the
+// pixels of that half-sweep's colour.  A thread owns a pair of columns in two
+// rows and keeps the slices in use, t - VD to t + 1, and their coefficients in
+// registers, so that a pixel's neighbours along z are its own (slice p + 1 has
+// had stage s - 1 in the same step, slice p - 1 a step ago), along x a shuffle,
+// along y the thread's other row or the neighbouring warp's: as loaded for the
+// first stage, then published in shared memory after each stage for the next
+// step.  One barrier a step.  The slices' slots and the colour of each row's
+// pixel are known at compile time (steps unrolled over the slots, an even
+// number; tiles start at even x, y and z): at step K of the unrolled loop every
+// stage updates column (row + K) mod 2 of the pair.
+//
+// Slices come into a ring in shared memory by asynchronous copies of ALIGN
+// bytes (16, 8 or 4, as the histories' rows allow), four slices ahead of the
+// one a step reads: with the slices loaded into registers two ahead, waiting
+// for them was the first stall.
+//
+// The tile's halo is VD pixels across x and y and VD slices along z beyond the
+// chunk; what lies outside the history or beyond the loaded slices has zero
+// coefficients and stays zero: exact at the history's border, and an error
+// that moves in one ring per half-sweep inside it, so every pixel VD or more
+// from such an edge equals S in-place half-sweeps of the whole history (as
+// k_sor32_half gives them, to the bit: the same sums in the same order).
+//
+// Measured on an oxygen field of 256^3 voxels (16-byte copies): 140 -> 41 us a
+// sweep against the kernel before, which kept the slices in shared memory, two
+// steps apart, and took 223 thread instructions an update (20 now); its HBM
+// floor at two sweeps a launch is 20 us, and the shared-memory pipe is busy 75 %
+// of the time.  255^3 (4-byte copies) 140 -> 56, 181^3 53 -> 26, 97^3 22.7 ->
+// 10.4, 96^3 21.7 -> 7.4.
 constexpr int VX = 64;  // tile columns: 32 lanes x 2
+constexpr int VD = 4;   // half-sweeps a launch at most
+constexpr int VSLOTS = VD + 2;  // slices in registers, and in the ring
 
-template <int D, int VY>
-__global__ void __launch_bounds__(32 * VY) k_sor32_vol(const float *__restrict__ src, float *__restrict__ dst,
-                                                       const float *__restrict__ rhs, const float *__restrict__ inv,
-                                                       const int4 *__restrict__ dims, const int64_t *__restrict__ off,
-                                                       const int4 *__restrict__ tiles, int vz,
-                                                       const float *__restrict__ omega, const int32_t *done,
-                                                       int done_stride, int nhalf, int start_colour, int zero_start,
-                                                       double *__restrict__ apply_c, int floor) {
-    constexpr int R = 2 * D + 2;  // ring slots: slices t - 2 D + 1 .. t + 2 in use at step t
-    extern __shared__ __align__(16) float ring[];  // [R][VY][VX]
+constexpr size_t vol_smem(int nw) {
+    return sizeof(float) * ((size_t)VSLOTS * 3 * VX * 2 * nw + 2 * (VD - 1) * (nw + 2) * 64);
+}
+
+// ALIGN bytes into shared memory at `to`; zeros where the chunk is not live.
+template <int ALIGN>
+__device__ __forceinline__ void copy_async(uint32_t to, const float *from, bool live) {
+    const int bytes = live ? ALIGN : 0;
+    if (ALIGN == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(to), "l"(from), "n"(ALIGN), "r"(bytes)
+                     : "memory");
+}
+
+// FULL: VD half-sweeps, neither a first launch nor a last one (most of a
+// correction's launches: without the other cases' code the unrolled steps fit
+// the instruction cache; 89 -> 62 us a sweep of 256^3 before the ring).
+template <int NW, int ALIGN, bool FULL>
+__global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
+    k_sor32_vol(const float *__restrict__ src, float *__restrict__ dst, const float *__restrict__ rhs,
+                const float *__restrict__ inv, const int4 *__restrict__ dims, const int64_t *__restrict__ off,
+                const int4 *__restrict__ tiles, int vz, const float *__restrict__ omega, const int32_t *done,
+                int done_stride, int nhalf, int zero_start, double *__restrict__ apply_c, int floor) {
+    constexpr int D = VD, NS = VSLOTS;
+    static_assert(NS % 2 == 0, "the steps' parity repeats with the slots");
+    constexpr int VY = 2 * NW, ARR = VX * VY, SLICE = 3 * ARR;
+    extern __shared__ __align__(16) float vsm[];
+    // the ring: [slot][correction, b, a][row][column]; then the published rows:
+    // [step parity][stage 1 .. D - 1][warp + 1][row][lane], a warp of zeros at either end
+    float *const edge = vsm + NS * SLICE;
+    constexpr int EWARP = 64, ESTAGE = (NW + 2) * EWARP, EBUF = (D - 1) * ESTAGE;
     const int4 tl = tiles[blockIdx.x];
     const int h = tl.x;
     if (done[(int64_t)h * done_stride]) return;
@@ -460,108 +498,155 @@ __global__ void __launch_bounds__(32 * VY) k_sor32_vol(const float *__restrict__
     const int x0 = tl.y, y0 = tl.z, z0 = tl.w;
     const int z1 = min(z0 + vz, dm.z);
     const int zlo = max(z0 - D, 0), zhi = min(z1 + D, dm.z);
-    const int S = nhalf;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int lx = 2 * tx, gx = x0 + lx, gy = y0 + ty;
-    const bool in0 = gx < dm.x && gy < dm.y, in1 = gx + 1 < dm.x && gy < dm.y;
+    const int S = FULL ? D : nhalf;
+    if (FULL) {
+        zero_start = 0;
+        apply_c = nullptr;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int gx = x0 + 2 * lane, gy = y0 + 2 * warp;
     // offsets inside the history in 32 bits (a history holds fewer than 2^31
     // pixels), its arrays from their first pixel
     const int plane = dm.x * dm.y;
-    const int col = gy * dm.x + gx;  // this thread's first pixel in slice 0
     const int64_t base = off[h];
-    const float *hsrc = src + base, *hrhs = rhs + base, *hinv = inv + base;
+    const float *const from[3] = {src + base, rhs + base, inv + base};
     float *hdst = dst + base;
     double *hc = apply_c ? apply_c + base : nullptr;
     const float omc = 1.f - omega[h];
+    const float lm = lane == 0 ? 0.f : 1.f, rm = lane == 31 ? 0.f : 1.f;
     // the output interior of the tile (a window edge on the history's border makes no error)
     const int ix0 = x0 == 0 ? 0 : x0 + D, ix1 = x0 + VX >= dm.x ? dm.x : x0 + VX - D;
     const int iy0 = y0 == 0 ? 0 : y0 + D, iy1 = y0 + VY >= dm.y ? dm.y : y0 + VY - D;
-    const bool out_y = gy >= iy0 && gy < iy1;
-    const bool out0 = in0 && out_y && gx >= ix0 && gx < ix1, out1 = in1 && out_y && gx + 1 >= ix0 && gx + 1 < ix1;
-    // this thread's pair in ring slot k
-    float2 *const mine = (float2 *)(ring + ty * VX) + tx;
-    auto at = [&](int k) -> float2 * { return mine + k * (VY * VX / 2); };
-    auto wrap = [](int k) { return k < 0 ? k + R : (k >= R ? k - R : k); };
-    auto load = [&](int o, float &v0, float &v1) {  // o: the slice's offset
-        v0 = v1 = 0.f;
-        if (!zero_start) {
-            if (in0) v0 = __ldg(hsrc + o + col);
-            if (in1) v1 = __ldg(hsrc + o + col + 1);
+    bool out0[2], out1[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const bool oy = gy + j >= iy0 && gy + j < iy1;
+        out0[j] = oy && gx >= ix0 && gx < ix1;
+        out1[j] = oy && gx + 1 >= ix0 && gx + 1 < ix1;
+    }
+    // the chunks of a slice this thread copies of each array: 16 / ALIGN of them
+    constexpr int CH = 16 / ALIGN, PER_ROW = VX * 4 / ALIGN, RSTEP = 32 * NW / PER_ROW;
+    const int crow = threadIdx.x / PER_ROW, ccol = threadIdx.x % PER_ROW * (ALIGN / 4);
+    const uint32_t ring0 = sh_addr(vsm) + 4u * (uint32_t)(crow * VX + ccol);
+    const int cfirst = (y0 + crow) * dm.x + x0 + ccol;
+    // slice z into slot k of the ring
+    auto fetch = [&](int z, int k) {
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+            const bool live = x0 + ccol < dm.x && z < zhi && y0 + crow + q * RSTEP < dm.y;
+            const int i = live ? z * plane + cfirst + q * RSTEP * dm.x : 0;
+#pragma unroll
+            for (int m = 0; m < 3; ++m)
+                copy_async<ALIGN>(ring0 + 4u * (uint32_t)(k * SLICE + m * ARR + q * RSTEP * VX), from[m] + i,
+                                  live && !(m == 0 && zero_start));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int i = threadIdx.x; i < 2 * EBUF; i += 32 * NW) edge[i] = 0.f;
+#pragma unroll
+    for (int k = 0; k < NS - 1; ++k) fetch(zlo + k, k);
+    float2 v[NS][2], b[NS][2], a[NS][2];
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) v[k][j] = b[k][j] = a[k][j] = make_float2(0.f, 0.f);
+    const float *const mine = vsm + 2 * warp * VX + 2 * lane;
+    float *const my_edge = edge + (warp + 1) * EWARP + lane;
+    auto take = [&](int k, float2 (&V)[2], float2 (&B)[2], float2 (&A)[2]) {
+        const float *p = mine + k * SLICE;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            V[j] = *(const float2 *)(p + j * VX);
+            B[j] = *(const float2 *)(p + ARR + j * VX);
+            A[j] = *(const float2 *)(p + 2 * ARR + j * VX);
         }
     };
-    // the first two slices
-    for (int z = zlo; z < min(zlo + 2, zhi); ++z) {
-        float v0, v1;
-        load(z * plane, v0, v1);
-        *at(z % R) = make_float2(v0, v1);
-    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
     __syncthreads();
-    const int tend = zhi - 1 + 2 * (S - 1);
-    int rt = zlo % R;     // ring slot of slice t
-    int toff = zlo * plane;  // offset of slice t
-    for (int t = zlo; t <= tend; ++t, rt = wrap(rt + 1), toff += plane) {
-        // the slice after next into registers while the stages run
-        const int zn = t + 2;
-        float n0 = 0.f, n1 = 0.f;
-        if (zn < zhi) load(toff + 2 * plane, n0, n1);
+    take(0, v[0], b[0], a[0]);
+    const int tend = zhi - 1 + (S - 1);
+    for (int t0 = zlo; t0 <= tend; t0 += NS) {
 #pragma unroll
-        for (int s = 1; s <= D; ++s) {
-            if (s > S) break;
-            const int p = t - 2 * (s - 1);  // the same for the whole block
-            if (p < zlo || p >= zhi) continue;
-            const int c = (start_colour + s - 1) & 1;
-            // the pixel of colour c in this thread's pair ((x + y + z) mod 2 == c,
-            // x0 even): the same e for a warp, which holds one row
-            const int e = (c + gy + p) & 1;
-            const int k = wrap(rt - 2 * (s - 1));
-            float2 *row = at(k);
-            const float2 me = *row;
-            // x neighbours: the left pair's second pixel, the right pair's first
-            const float left = __shfl_up_sync(0xffffffffu, me.y, 1);
-            const float right = __shfl_down_sync(0xffffffffu, me.x, 1);
-            const float2 z2 = make_float2(0.f, 0.f);
-            const float2 ym2 = ty > 0 ? row[-VX / 2] : z2, yp2 = ty + 1 < VY ? row[VX / 2] : z2;
-            const float2 zm2 = p - 1 >= zlo ? *at(wrap(k - 1)) : z2;
-            const float2 zp2 = p + 1 < zhi ? *at(wrap(k + 1)) : z2;
-            if (!(e ? in1 : in0)) continue;  // outside the history: stays zero
-            float xm, xp, ym, yp, zm, zp, cur;
-            if (e == 0) {
-                xm = tx > 0 ? left : 0.f; xp = me.y; ym = ym2.x; yp = yp2.x; zm = zm2.x; zp = zp2.x; cur = me.x;
-            } else {
-                xm = me.x; xp = tx < 31 ? right : 0.f; ym = ym2.y; yp = yp2.y; zm = zm2.y; zp = zp2.y; cur = me.y;
-            }
-            // k_sor32_half's sums, in its order
-            float sum = (xm + xp) + (ym + yp);
-            sum += (zm + zp);
-            const int i = toff - 2 * (s - 1) * plane + col + e;
-            const float v = fmaf(__ldg(hinv + i), sum, fmaf(omc, cur, __ldg(hrhs + i)));
-            *row = e == 0 ? make_float2(v, me.y) : make_float2(me.x, v);
-        }
-        // slice t - 2 (S - 1) has had every half-sweep: its interior out
-        const int pf = t - 2 * (S - 1);
-        if (pf >= z0 && pf < z1) {
-            const float2 q = *at(wrap(rt - 2 * (S - 1)));
-            const int i = toff - 2 * (S - 1) * plane + col;
-            if (hc) {
-                // the last launch of a correction: c += d on the free pixels
-                // (a held pixel has a = 0 and d = 0 throughout), floored as
-                // the reference's update is (pde.rs:395)
-                if (out0 && (q.x != 0.f || __ldg(hinv + i) != 0.f)) {
-                    const double v = hc[i] + (double)q.x;
-                    hc[i] = floor ? fmax(v, 0.0) : v;
+        for (int K = 0; K < NS; ++K) {
+            const int t = t0 + K;
+            if (t > tend) break;  // the same for the whole block
+            // slice t + 1 has landed for every thread; slice t - 1 has been read
+            // by all, its slot takes slice t + NS - 1
+            asm volatile("cp.async.wait_group %0;" ::"n"(NS - 3) : "memory");
+            __syncthreads();
+            fetch(t + NS - 1, (K + NS - 1) % NS);
+            take((K + 1) % NS, v[(K + 1) % NS], b[(K + 1) % NS], a[(K + 1) % NS]);
+            // the pixels above and below as loaded, for the first stage
+            float above0 = 0.f, below0 = 0.f;
+            if (warp > 0) above0 = mine[K * SLICE - VX + (K & 1)];
+            if (warp < NW - 1) below0 = mine[K * SLICE + 2 * VX + ((K + 1) & 1)];
+            const float *ein = my_edge + (K & 1) * EBUF;
+            float *eout = my_edge + ((K + 1) & 1) * EBUF;
+#pragma unroll
+            for (int s = 1; s <= D; ++s) {
+                if (s > S) break;
+                const int p = (K - (s - 1) + NS) % NS, pm = (p + NS - 1) % NS, pp = (p + 1) % NS;
+                // the across-lane neighbours of both rows first
+                float side[2], next[2];
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    side[j] = ((j + K) & 1) == 0 ? __shfl_up_sync(0xffffffffu, v[p][j].y, 1)
+                                                 : __shfl_down_sync(0xffffffffu, v[p][j].x, 1);
+                const float above = s == 1 ? above0 : ein[(s - 2) * ESTAGE - EWARP + 32];
+                const float below = s == 1 ? below0 : ein[(s - 2) * ESTAGE + EWARP];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    // k_sor32_half's sums, in its order
+                    const float2 other = v[p][1 - j];
+                    if (((j + K) & 1) == 0) {
+                        const float ym = j == 0 ? above : other.x, yp = j == 0 ? other.x : below;
+                        float sum = fmaf(lm, side[j], v[p][j].y) + (ym + yp);
+                        sum += v[pm][j].x + v[pp][j].x;
+                        next[j] = fmaf(a[p][j].x, sum, fmaf(omc, v[p][j].x, b[p][j].x));
+                    } else {
+                        const float ym = j == 0 ? above : other.y, yp = j == 0 ? other.y : below;
+                        float sum = fmaf(rm, side[j], v[p][j].x) + (ym + yp);
+                        sum += v[pm][j].y + v[pp][j].y;
+                        next[j] = fmaf(a[p][j].y, sum, fmaf(omc, v[p][j].y, b[p][j].y));
+                    }
                 }
-                if (out1 && (q.y != 0.f || __ldg(hinv + i + 1) != 0.f)) {
-                    const double v = hc[i + 1] + (double)q.y;
-                    hc[i + 1] = floor ? fmax(v, 0.0) : v;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (((j + K) & 1) == 0) v[p][j].x = next[j];
+                    else v[p][j].y = next[j];
+                    if (s < D) eout[(s - 1) * ESTAGE + 32 * j] = next[j];
                 }
-            } else {
-                if (out0) hdst[i] = q.x;
-                if (out1) hdst[i + 1] = q.y;
+                // slice t - (S - 1) has had every half-sweep: its interior out
+                const int pf = t - (s - 1);
+                if (s == S && pf >= z0 && pf < z1) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int i = pf * plane + (gy + j) * dm.x + gx;
+                        const float2 q = v[p][j];
+                        if (hc) {
+                            // the last launch of a correction: c += d on the free
+                            // pixels (a held pixel has a = 0 and d = 0 throughout),
+                            // floored as the reference's update is (pde.rs:395)
+                            if (out0[j] && (q.x != 0.f || a[p][j].x != 0.f)) {
+                                const double c = hc[i] + (double)q.x;
+                                hc[i] = floor ? fmax(c, 0.0) : c;
+                            }
+                            if (out1[j] && (q.y != 0.f || a[p][j].y != 0.f)) {
+                                const double c = hc[i + 1] + (double)q.y;
+                                hc[i + 1] = floor ? fmax(c, 0.0) : c;
+                            }
+                        } else if (ALIGN >= 8 && out0[j] && out1[j]) {
+                            *(float2 *)(hdst + i) = q;
+                        } else {
+                            if (out0[j]) hdst[i] = q.x;
+                            if (out1[j]) hdst[i + 1] = q.y;
+                        }
+                    }
+                }
             }
         }
-        if (zn < zhi) *at(wrap(rt + 2)) = make_float2(n0, n1);
-        __syncthreads();
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 typedef void (*TbKernel)(const float *, float *, const float *, const float *, const int4 *, const int64_t *,
@@ -590,14 +675,17 @@ WideKernel wide_kernel_of(int depth) {
 }
 
 typedef void (*VolKernel)(const float *, float *, const float *, const float *, const int4 *, const int64_t *,
-                          const int4 *, int, const float *, const int32_t *, int, int, int, int, double *, int);
+                          const int4 *, int, const float *, const int32_t *, int, int, int, double *, int);
 
-VolKernel vol_kernel(int depth, int vy) {
-    if (vy == 16) return depth >= 4 ? k_sor32_vol<4, 16> : k_sor32_vol<2, 16>;
-    return depth >= 4 ? k_sor32_vol<4, 32> : k_sor32_vol<2, 32>;
+template <int NW, bool FULL>
+VolKernel vol_kernel_of(int align) {
+    return align == 16 ? k_sor32_vol<NW, 16, FULL> : align == 8 ? k_sor32_vol<NW, 8, FULL> : k_sor32_vol<NW, 4, FULL>;
 }
 
-size_t vol_smem(int depth, int vy) { return (size_t)(2 * depth + 2) * vy * VX * sizeof(float); }
+VolKernel vol_kernel(int vy, int align, bool full) {
+    return vy == 16 ? (full ? vol_kernel_of<8, true>(align) : vol_kernel_of<8, false>(align))
+                    : (full ? vol_kernel_of<16, true>(align) : vol_kernel_of<16, false>(align));
+}
 
 WideKernel wide_kernel(int depth, int warps) { return warps == 16 ? wide_kernel_of<16>(depth) : wide_kernel_of<8>(depth); }
 
@@ -671,48 +759,56 @@ int wide_init(Sor32 &s, cw_field_s *f, int warps) {
     return CW_OK;
 }
 
-// The volume kernel's tiles: VX x vy columns (halo `depth`) by chunks of vz
-// slices, vz the largest of 64, 32, 16 that still gives the device three
-// tiles for every block it holds at once.
+// The volume kernel's tiles: VX x vy columns (halo VD) by chunks of vz slices,
+// an even number: the count of chunks whose waves of tiles march the fewest
+// slices, halo and pipeline included (256^3: 440 tiles of 32 slices, three full
+// waves of 148).
 int vol_init(Sor32 &s, cw_field_s *f, int window) {
     s.vol = false;
     const Geom &g = f->g;
-    for (uint32_t k = 0; k < g.nh; ++k)
+    int most = 0;
+    s.valign = 16;
+    for (uint32_t k = 0; k < g.nh; ++k) {
         if (g.d[k] < 2) return CW_OK;
-    s.vdepth = s.depth >= 4 ? 4 : 2;
+        most = std::max(most, (int)g.d[k]);
+        for (int64_t n : {(int64_t)g.w[k], g.off[k]})
+            while (n * 4 % s.valign) s.valign /= 2;
+    }
+    s.vdepth = s.depth >= VD ? VD : 2;
     s.vy = window == CW_WINDOW_64 ? 16 : 32;
-    VolKernel kern = vol_kernel(s.vdepth, s.vy);
-    const size_t smem = vol_smem(s.vdepth, s.vy);
-    CW_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = vol_smem(s.vy / 2);
+    for (bool full : {true, false})
+        CW_CUDA(cudaFuncSetAttribute((const void *)vol_kernel(s.vy, s.valign, full),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0, dev = 0, nsm = 0;
-    CW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)kern, 32 * s.vy, smem));
+    CW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)vol_kernel(s.vy, s.valign, true),
+                                                          16 * s.vy, smem));
     if (per_sm < 1) return CW_OK;  // one half-sweep per launch serves
     CW_CUDA(cudaGetDevice(&dev));
     CW_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     std::vector<int> xs, ys;
     std::vector<int64_t> columns(g.nh);
     for (uint32_t k = 0; k < g.nh; ++k) {
-        axis_starts(g.w[k], VX, s.vdepth, xs);
-        axis_starts(g.h[k], s.vy, s.vdepth, ys);
+        axis_starts(g.w[k], VX, VD, xs);
+        axis_starts(g.h[k], s.vy, VD, ys);
         columns[k] = (int64_t)xs.size() * ys.size();
     }
-    // chunks: the longest of 64, 32, 16 slices that still gives three tiles
-    // for every block the device holds at once (one tile a block, for less of
-    // the z halo's redundant work, measured 11 % slower on the 256^3 spheroid)
-    const int64_t want = 3LL * per_sm * nsm;
-    s.vz = 16;
-    for (int vz : {64, 32}) {
+    const int64_t resident = (int64_t)per_sm * nsm;
+    int64_t best = -1;
+    for (int chunks = 1; chunks <= (most + 7) / 8; ++chunks) {
+        const int vz = ((most + chunks - 1) / chunks + 1) / 2 * 2;
         int64_t n = 0;
         for (uint32_t k = 0; k < g.nh; ++k) n += columns[k] * ((g.d[k] + vz - 1) / vz);
-        if (n >= want) {
+        const int64_t cost = (n + resident - 1) / resident * (std::min(vz + 2 * VD, most) + VD + 2);
+        if (best < 0 || cost < best) {
+            best = cost;
             s.vz = vz;
-            break;
         }
     }
     std::vector<int4> tiles;
     for (uint32_t k = 0; k < g.nh; ++k) {
-        axis_starts(g.w[k], VX, s.vdepth, xs);
-        axis_starts(g.h[k], s.vy, s.vdepth, ys);
+        axis_starts(g.w[k], VX, VD, xs);
+        axis_starts(g.h[k], s.vy, VD, ys);
         for (int z = 0; z < g.d[k]; z += s.vz)
             for (int y : ys)
                 for (int x : xs) tiles.push_back(make_int4((int)k, x, y, z));
@@ -775,16 +871,14 @@ int Sor32::sweeps(cw_field_s *f, int n, const int32_t *done, int done_stride, fl
         // between the buffers; the first launch starts from zero
         float *a = ping, *b = pong;
         int remaining = 2 * n, done_half = 0;
-        VolKernel kern = vol_kernel(vdepth, vy);
-        const size_t smem = vol_smem(vdepth, vy);
         while (remaining > 0) {
             const int dd = remaining < vdepth ? remaining : vdepth;
             // with `apply` the last launch adds its correction to the field
             const bool last = remaining == dd;
-            kern<<<nvtiles, 32 * vy, smem, stream()>>>(a, b, f->r32, f->inv32, f->g.d_dims, f->g.d_off, vtiles, vz,
-                                                       omega, done, done_stride, dd, done_half & 1,
-                                                       done_half == 0 ? 1 : 0, apply && last ? f->c : nullptr,
-                                                       f->floor ? 1 : 0);
+            const bool full = dd == VD && done_half > 0 && !(apply && last);
+            vol_kernel(vy, valign, full)<<<nvtiles, 16 * vy, vol_smem(vy / 2), stream()>>>(
+                a, b, f->r32, f->inv32, f->g.d_dims, f->g.d_off, vtiles, vz, omega, done, done_stride, dd,
+                done_half == 0 ? 1 : 0, apply && last ? f->c : nullptr, f->floor ? 1 : 0);
             CW_LAUNCHED();
             remaining -= dd;
             done_half += dd;
