@@ -291,10 +291,15 @@ struct cw_lattice_s {
     int8_t reach[3 * 124] = {0};
     double across = 1.0;
     int32_t *d_flag = nullptr;       // scratch flag / counters
-    // scratch of the sublattice passes (lattice.cu): claims, pending lists, control words
+    // scratch of the sublattice passes (lattice.cu): claims, attempts, the cells' lists, control words
     unsigned long long *claim = nullptr;  // 2 * ncells
-    uint4 *plist = nullptr;               // plist_cap attempts of 3 uint4 (lattice.cu)
-    uint32_t *pidx = nullptr;             // 2 * plist_cap pending-attempt indices
+    uint4 *plist = nullptr;               // plist_cap attempts of 8 uint4
+    ulonglong2 *pmail = nullptr;          // plist_cap mailboxes
+    uint32_t *pidx = nullptr;             // 2 * plist_cap attempt indices
+    uint32_t *pcount = nullptr;           // ncells: attempts listed
+    unsigned long long *pchain = nullptr; // ncells lists of entries (null: passes by rounds)
+    int32_t useg = 1;                     // pixels of a row a lane reads at once
+    bool chain_tried = false;             // room for the lists was asked for
     int64_t plist_cap = 0;
     int32_t *d_vplan = nullptr;           // nh + 1: the pass plan (first chunk of each history)
     uint32_t *pctl = nullptr;             // control words, then 27 pass keys per history (lattice.cu)
@@ -313,6 +318,7 @@ struct cw_lattice_s {
     int32_t *bath_label = nullptr;        // the bath's union-find labels, one per site (bath.cu)
     uint8_t *bath_mark = nullptr;         // roots that reach the outer layer (bath.cu)
     int build_plans();
+    int ensure_scratch();
 };
 
 namespace cw { struct Resident64; }

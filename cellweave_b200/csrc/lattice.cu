@@ -10,7 +10,7 @@
 // only through the volume and surface records of cells they share.  A pass
 // runs its attempts as the sequence in a per-pass priority order would (each
 // seeing the records every earlier one left): attempts that share no cell run
-// at once, the others in rounds, in priority order (k_cpm_pass).  So a pass is
+// at once, the others in rounds, in priority order (k_cpm_sweep).  So a pass is
 // deterministic whatever the thread schedule, and keeps the sequential
 // sweep's volume statistics.  The colours are swept in an order shuffled anew
 // every step.
@@ -70,7 +70,7 @@ struct Tables {
 
 __device__ __forceinline__ int32_t kind_of(const int32_t *type_h, int64_t cap, int32_t id) {
     if (id < 0 || id >= cap) return 0;  // the obstacle reads as the medium (cpm.rs:908-917)
-    return type_h[id];
+    return __ldg(type_h + id);
 }
 
 // von_neumann, cpm.rs:922-944: y-1, y+1, x-1, x+1, z-1, z+1, clipped; as a
@@ -126,20 +126,37 @@ __device__ __forceinline__ Vn vn_of(int4 dm, int x, int y, int z) {
 }
 
 // contact_delta_h (cpm.rs:851-876) on history grid `g`; *num before the division.
-__device__ __forceinline__ double contact_delta(const int32_t *__restrict__ g, int4 dm, int x, int y, int z, int32_t src,
+__device__ __forceinline__ double contact_delta(const int32_t *g, int4 dm, int x, int y, int z, int32_t src,
                                 int32_t dst, const int32_t *type_h, int64_t cap, const double *sJ, int K,
                                 const int8_t *reach, int nreach, double across, int64_t i, Vn vn, double *num) {
     int32_t ks = kind_of(type_h, cap, src), kd = kind_of(type_h, cap, dst);
     double dh = 0.0;
     if (nreach > 0) {
-        for (int k = 0; k < nreach; ++k) {
-            int a = x + reach[3 * k], b = y + reach[3 * k + 1], c = z + reach[3 * k + 2];
-            if (a < 0 || b < 0 || c < 0 || a >= dm.x || b >= dm.y || c >= dm.z) continue;
-            int32_t nb = g[((int64_t)c * dm.y + b) * dm.x + a];
-            int32_t kn = kind_of(type_h, cap, nb);
-            double ed = dst == nb ? 0.0 : sJ[kd * K + kn];
-            double es = src == nb ? 0.0 : sJ[ks * K + kn];
-            dh += ed - es;
+        // a batch of neighbours' ids, then their kinds, in flight at once (one at
+        // a time each waits for two reads); added in the reach's order
+        constexpr int NB = 13;
+        for (int k0 = 0; k0 < nreach; k0 += NB) {
+            int32_t nb[NB], kn[NB];
+            unsigned in = 0;
+#pragma unroll
+            for (int q = 0; q < NB; ++q) {
+                const int k = k0 + q;
+                nb[q] = 0;
+                if (k >= nreach) continue;
+                const int a = x + reach[3 * k], b = y + reach[3 * k + 1], c = z + reach[3 * k + 2];
+                if (a < 0 || b < 0 || c < 0 || a >= dm.x || b >= dm.y || c >= dm.z) continue;
+                in |= 1u << q;
+                nb[q] = g[((int64_t)c * dm.y + b) * dm.x + a];
+            }
+#pragma unroll
+            for (int q = 0; q < NB; ++q) kn[q] = kind_of(type_h, cap, nb[q]);
+#pragma unroll
+            for (int q = 0; q < NB; ++q) {
+                if (!((in >> q) & 1u)) continue;
+                const double ed = dst == nb[q] ? 0.0 : sJ[kd * K + kn[q]];
+                const double es = src == nb[q] ? 0.0 : sJ[ks * K + kn[q]];
+                dh += ed - es;
+            }
         }
         *num = dh;
         return dh / across;
@@ -157,21 +174,31 @@ __device__ __forceinline__ double contact_delta(const int32_t *__restrict__ g, i
     return dh;
 }
 
-// volume_delta_h, cpm.rs:879-894, on the volumes given (c0: the history's first cell).
-__device__ __forceinline__ double volume_delta(const int32_t *vol, const int32_t *target, const double *lambda,
-                                               int64_t c0, int32_t src, int32_t dst) {
+// volume_delta_h, cpm.rs:879-894: each cell's change of lambda (V - V_target)^2
+// on losing (source) or gaining (copied) a pixel, added in that order.
+__device__ __forceinline__ double volume_terms(bool has_src, int32_t vs, int32_t ts, double ls, bool has_dst, int32_t vd,
+                                               int32_t td, double ld) {
     double dh = 0.0;
-    if (src != 0) {
-        double v = (double)vol[c0 + src], vt = (double)target[c0 + src];
-        double a = v - 1.0 - vt, b = v - vt;
-        dh += lambda[c0 + src] * (a * a - b * b);
+    if (has_src) {
+        const double v = (double)vs, vt = (double)ts;
+        const double a = v - 1.0 - vt, b = v - vt;
+        dh += ls * (a * a - b * b);
     }
-    if (dst != 0) {
-        double v = (double)vol[c0 + dst], vt = (double)target[c0 + dst];
-        double a = v + 1.0 - vt, b = v - vt;
-        dh += lambda[c0 + dst] * (a * a - b * b);
+    if (has_dst) {
+        const double v = (double)vd, vt = (double)td;
+        const double a = v + 1.0 - vt, b = v - vt;
+        dh += ld * (a * a - b * b);
     }
     return dh;
+}
+// The same on the volumes given (c0: the history's first cell).
+__device__ __forceinline__ double volume_delta(const int32_t *vol, const int32_t *target, const double *lambda,
+                                               int64_t c0, int32_t src, int32_t dst) {
+    int32_t vs = 0, ts = 0, vd = 0, td = 0;
+    double ls = 0.0, ld = 0.0;
+    if (src != 0) { vs = vol[c0 + src]; ts = target[c0 + src]; ls = lambda[c0 + src]; }
+    if (dst != 0) { vd = vol[c0 + dst]; td = target[c0 + dst]; ld = lambda[c0 + dst]; }
+    return volume_terms(src != 0, vs, ts, ls, dst != 0, vd, td, ld);
 }
 
 __device__ __forceinline__ void surface_change(const int32_t *g, int64_t i, Vn vn, int32_t src, int32_t dst,
@@ -189,30 +216,40 @@ __device__ __forceinline__ void surface_change(const int32_t *g, int64_t i, Vn v
     ddst = (nvn - eq_d) - eq_d;
 }
 
-__device__ __forceinline__ double surface_delta(const int32_t *surf, const int32_t *tsurf, const double *lsurf,
-                                                int64_t c0, int32_t src, int32_t dst, int32_t dsrc, int32_t ddst) {
+__device__ __forceinline__ double surface_terms(bool has_src, int32_t ss, int32_t tss, double lss, int32_t dsrc,
+                                                bool has_dst, int32_t sd, int32_t tsd, double lsd, int32_t ddst) {
     double dh = 0.0;
-    if (src > 0) {
-        double s = (double)surf[c0 + src], st = (double)tsurf[c0 + src];
-        double a = s + (double)dsrc - st, b = s - st;
-        dh += lsurf[c0 + src] * (a * a - b * b);
+    if (has_src) {
+        const double s = (double)ss, st = (double)tss;
+        const double a = s + (double)dsrc - st, b = s - st;
+        dh += lss * (a * a - b * b);
     }
-    if (dst > 0) {
-        double s = (double)surf[c0 + dst], st = (double)tsurf[c0 + dst];
-        double a = s + (double)ddst - st, b = s - st;
-        dh += lsurf[c0 + dst] * (a * a - b * b);
+    if (has_dst) {
+        const double s = (double)sd, st = (double)tsd;
+        const double a = s + (double)ddst - st, b = s - st;
+        dh += lsd * (a * a - b * b);
     }
     return dh;
+}
+__device__ __forceinline__ double surface_delta(const int32_t *surf, const int32_t *tsurf, const double *lsurf,
+                                                int64_t c0, int32_t src, int32_t dst, int32_t dsrc, int32_t ddst) {
+    int32_t ss = 0, tss = 0, sd = 0, tsd = 0;
+    double lss = 0.0, lsd = 0.0;
+    if (src > 0) { ss = surf[c0 + src]; tss = tsurf[c0 + src]; lss = lsurf[c0 + src]; }
+    if (dst > 0) { sd = surf[c0 + dst]; tsd = tsurf[c0 + dst]; lsd = lsurf[c0 + dst]; }
+    return surface_terms(src > 0, ss, tss, lss, dsrc, dst > 0, sd, tsd, lsd, ddst);
 }
 
 // The colour order of the current step for every history: a Fisher-Yates
 // shuffle driven by Philox(all-ones, step, 1, i); with `pass_keys`, each
 // pass's priority key, word 0 of Philox(all-ones - 1, step, 2, colour);
-// advances the step counter.
+// advances the step counter, and clears the sweep's barrier words and counts
+// (the eight 32-bit words at `words`).
 __global__ void k_colour_order(const uint2 *keys, int nh, int ncol, uint32_t *mcs_ctr, uint32_t *mcs_cur,
-                               int32_t *perm, uint32_t *pass_keys) {
+                               int32_t *perm, uint32_t *pass_keys, uint32_t *words) {
     // one block: every thread reads the counter before thread 0 advances it
     uint32_t m = *mcs_ctr;
+    if (threadIdx.x < 8) words[threadIdx.x] = 0u;
     for (int h = threadIdx.x; h < nh; h += blockDim.x) {
         int32_t p[27];
         for (int i = 0; i < ncol; ++i) p[i] = i;
@@ -234,23 +271,24 @@ __global__ void k_colour_order(const uint2 *keys, int nh, int ncol, uint32_t *mc
     }
 }
 
-// The pixel with index k among the pixels of colour `colour` inside the box
-// b = (x0, y0, z0, x1, y1, z1) (inclusive) of a history; false past the end.
+// The rows (y, z) that hold pixels of colour `colour` inside the box b = (x0,
+// y0, z0, x1, y1, z1) (inclusive) of a history: row `row` of them, its first
+// such pixel fx, their spacing `step` and count nx; false past the last row.
 // Colour classes: the chessboard (x + y + z) mod 2 for period 0, else the
 // residues of x, y, z modulo the period.  (32-bit index arithmetic: a
 // history holds fewer than 2^31 pixels.)
-__device__ __forceinline__ bool colour_site_box(const int (&b)[6], int period, int colour, uint32_t k, int &x, int &y,
-                                                int &z) {
+__device__ __forceinline__ bool colour_row(const int (&b)[6], int period, int colour, uint32_t row, int &y, int &z,
+                                           int &fx, int &step, int &nx) {
     if (b[3] < b[0] || b[4] < b[1] || b[5] < b[2]) return false;
     if (period == 0) {
-        const uint32_t hw = ((uint32_t)(b[3] - b[0]) + 2u) >> 1;
         const uint32_t wy = (uint32_t)(b[4] - b[1] + 1);
-        const uint32_t row = k / hw;
         if (row >= wy * (uint32_t)(b[5] - b[2] + 1)) return false;
         y = b[1] + (int)(row % wy);
         z = b[2] + (int)(row / wy);
-        x = b[0] + ((colour - b[0] - y - z) & 1) + 2 * (int)(k - row * hw);
-        return x <= b[3];
+        fx = b[0] + ((colour - b[0] - y - z) & 1);
+        step = 2;
+        nx = fx <= b[3] ? (b[3] - fx) / 2 + 1 : 0;
+        return true;
     }
     const int c[3] = {colour % period, (colour / period) % period, colour / (period * period)};
     int f[3];
@@ -260,20 +298,25 @@ __device__ __forceinline__ bool colour_site_box(const int (&b)[6], int period, i
         f[a] = b[a] + ((c[a] - b[a] % period + period) % period);
         n[a] = f[a] <= b[3 + a] ? (uint32_t)((b[3 + a] - f[a]) / period + 1) : 0u;
     }
-    if (n[0] == 0 || n[1] == 0 || n[2] == 0 || k >= n[0] * n[1] * n[2]) return false;
-    const uint32_t r = k / n[0];
-    x = f[0] + period * (int)(k - r * n[0]);
-    y = f[1] + period * (int)(r % n[1]);
-    z = f[2] + period * (int)(r / n[1]);
+    if (n[0] == 0 || n[1] == 0 || n[2] == 0 || row >= n[1] * n[2]) return false;
+    y = f[1] + period * (int)(row % n[1]);
+    z = f[2] + period * (int)(row / n[1]);
+    fx = f[0];
+    step = period;
+    nx = (int)n[0];
     return true;
 }
 
-// The most pixels one colour holds in a box of sides (wx, wy, wz): the plan
-// of a pass gives each history that many sites.
-__host__ __device__ __forceinline__ int64_t colour_sites_max(int64_t wx, int64_t wy, int64_t wz, int period) {
+// Segments of 32 `useg` pixels of one colour that a row of a box of side wx
+// takes at most, and a box's items (rows times segments).
+__host__ __device__ __forceinline__ int64_t colour_segments(int64_t wx, int period, int useg) {
+    const int64_t n = period == 0 ? (wx + 1) / 2 : (wx + period - 1) / period;
+    return (n + 32 * useg - 1) / (32 * useg);
+}
+__host__ __device__ __forceinline__ int64_t colour_items(int64_t wx, int64_t wy, int64_t wz, int period, int useg) {
     if (wx <= 0 || wy <= 0 || wz <= 0) return 0;
-    if (period == 0) return ((wx + 1) / 2) * wy * wz;
-    return ((wx + period - 1) / period) * ((wy + period - 1) / period) * ((wz + period - 1) / period);
+    const int64_t rows = period == 0 ? wy * wz : ((wy + period - 1) / period) * ((wz + period - 1) / period);
+    return rows * colour_segments(wx, period, useg);
 }
 
 // MurmurHash3's 32-bit finaliser (Appleby): a bijection of 32-bit words, so
@@ -287,28 +330,78 @@ __device__ __forceinline__ uint32_t fmix32(uint32_t h) {
     return h;
 }
 
+constexpr uint32_t NONE = 0xFFFFFFFFu;
+
 // One copy attempt of a pass, with everything about it that the pass cannot
 // change: the pixels of a colour lie outside one another's reach, so the
 // contact term, the surface counts' changes and the draws are fixed when the
-// pass starts; only the volume and surface records move.
-struct __align__(16) Attempt {
-    int64_t c0;        // the history's first cell record
-    int32_t src, dst;  // source and copied ids
-    uint32_t prio;     // the pass priority
-    int32_t dsurf;     // surface changes of source and copied cell (int16 each)
-    uint32_t u0, u1;   // the acceptance draw's words
-    int64_t gi;        // the pixel in the batch's flat order
-    union {
-        double contact;  // contact Delta-H (cpm.rs:851-876)
-        uint2 where;     // until the contact is taken: history | z << 16, x | y << 16
-    };
+// pass starts; only the volume and surface records move.  One line of memory.
+struct __align__(128) Attempt {
+    double contact;            // contact Delta-H (cpm.rs:851-876)
+    double limit;              // Delta-H below it is accepted, above it rejected (decide)
+    double ls, ld;             // lambda of the source and of the copied cell
+    int32_t ts, td;            // their target volumes
+    uint32_t cs, cd;           // their records (NONE: the medium)
+    uint32_t next_s, next_d;   // the attempt after this one on each (link; NONE: the last)
+    int32_t dst;               // the copied id
+    int32_t dsurf;             // surface changes of source and copied cell (int16 each)
+    int64_t gi;                // the pixel in the batch's flat order
+    uint32_t u0, u1;           // the acceptance draw's words
+    double lss, lsd;           // with a surface constraint: the surface lambdas
+    int32_t tss, tsd;          // and target surfaces
+    uint32_t prio;             // the pass priority
+    int32_t src;               // the source id
+    uint2 where;               // history | z << 16, x | y << 16
+    uint32_t pad[2];
 };
-static_assert(sizeof(Attempt) == 48, "an attempt is three 16-byte words");
+static_assert(sizeof(Attempt) == 128, "an attempt is one line");
 
-constexpr int PT = 1024;           // threads of a pass block; one block per SM
-constexpr int PEND_SMEM = 4096;    // pending attempts a block lists in shared memory (else in its global segment)
+// What running an attempt takes, read by words of 16 bytes (a copy of the
+// struct goes through local memory).
+struct Terms {
+    double contact, limit, ls, ld, lss, lsd;
+    int64_t gi;
+    int32_t ts, td, tss, tsd, dst, dsurf;
+    uint32_t cs, cd, next_s, next_d, u0, u1;
+    __device__ __forceinline__ void read(const Attempt *a, bool surface) {
+        const double2 *d = (const double2 *)a;
+        const int4 *w = (const int4 *)a;
+        const double2 d0 = d[0], d1 = d[1];
+        const int4 w2 = w[2], w3 = w[3], w4 = w[4];
+        contact = d0.x;
+        limit = d0.y;
+        ls = d1.x;
+        ld = d1.y;
+        ts = w2.x;
+        td = w2.y;
+        cs = (uint32_t)w2.z;
+        cd = (uint32_t)w2.w;
+        next_s = (uint32_t)w3.x;
+        next_d = (uint32_t)w3.y;
+        dst = w3.z;
+        dsurf = w3.w;
+        gi = (int64_t)(((uint64_t)(uint32_t)w4.y << 32) | (uint32_t)w4.x);
+        u0 = (uint32_t)w4.z;
+        u1 = (uint32_t)w4.w;
+        lss = lsd = 0.0;
+        tss = tsd = 0;
+        if (surface) {
+            const double2 d5 = d[5];
+            const int4 w6 = w[6];
+            lss = d5.x;
+            lsd = d5.y;
+            tss = w6.x;
+            tsd = w6.y;
+        }
+    }
+};
+
+constexpr int PT = 512;            // threads of a pass block; one block per SM
+constexpr int PW = PT / 32;        // its warps, an item (a row's segment) each of a chunk
+constexpr int UMAX = 4;            // pixels of a row a lane reads at once at most
+constexpr int PEND = 3072;         // pending attempts a block lists in shared memory (rounds)
 constexpr int PLAN_SMEM = 1024;    // pass plans of up to 1023 histories sit in shared memory
-constexpr int ILP = 2;             // attempts a thread carries at once through a round
+constexpr int CHAIN = 64;          // attempts a cell's list holds
 constexpr int MAX_ROUNDS = 256;
 constexpr uint32_t ROUND_SPAN = MAX_ROUNDS + 2;  // claim tags one pass may use
 // passes before the claim tags would overflow 32 bits: the pass that reaches
@@ -316,76 +409,95 @@ constexpr uint32_t ROUND_SPAN = MAX_ROUNDS + 2;  // claim tags one pass may use
 constexpr uint32_t SEQ_LIMIT = 0xFFFFFFFFu / ROUND_SPAN - 1u;
 constexpr unsigned long long BARRIER_NS = 2000000000ull;
 
-// Scratch of the passes.  Claims: two words per cell (by round parity), each
+// Scratch of the passes.  Attempts: a segment of `seg` per block; beside them
+// a mailbox and two index words each.  A cell's list: its attempts' count and
+// CHAIN entries (priority << 32 | attempt << 2 | only cell << 1 | side), side 0
+// for the source.  Claims (rounds): two words per cell (by round parity), each
 // (tag << 32 | priority) with the tag (pass sequence x ROUND_SPAN + round)
 // rising from pass to pass, so that old claims lose to new ones and nothing
-// needs clearing.  Attempts: a segment of `seg` per block.  Pending lists:
-// indices into the block's segment, in shared memory or, for a block with
-// more than PEND_SMEM attempts, in two segments of `seg` in `idx`.
+// needs clearing.
 struct PassScratch {
     unsigned long long *claim[2];  // ncells each
     Attempt *list;
-    uint32_t *idx;
+    ulonglong2 *mail;              // per attempt
+    uint32_t *idx, *link;          // per attempt: the blocks' lists (ready; pending, even rounds) and the lanes'
+                                   // stacks (pending, odd rounds)
+    uint32_t *count;               // per cell: the attempts listed (zero between passes)
+    unsigned long long *chain;     // per cell: CHAIN entries; null: every pass by rounds
     uint32_t seg;
+    int32_t useg;                  // pixels a lane of an item reads (1 to UMAX)
     int64_t ncells;
     uint32_t *ctl;                 // CTL_* below, then the pass keys (history x colour)
-    const int32_t *vplan;          // nh + 1: each history's first chunk of PT sites; vplan[nh]: all chunks
+    const int32_t *vplan;          // nh + 1: each history's first chunk of PW items; vplan[nh]: all chunks
     unsigned long long barrier_ns; // a grid barrier's wait limit
     int32_t withhold;              // a block that never arrives at a barrier (failure tests; -1: none)
     int32_t max_rounds;            // rounds before a pass gives up (CW_ERR_SIMULATION)
 };
-// control words: list counts and the barrier's arrivals share a line (both
-// left at zero when a pass ends); the barrier's generation (only ever
-// compared with itself) another; the error, round and sequence records a
-// third; then the pass keys
-enum { CTL_COUNT = 0, CTL_BAR = 3, CTL_GEN = 32, CTL_ERR = 48, CTL_ROUNDS = 49, CTL_SEQ = 50, CTL_KEYS = 64 };
+// control words: the barrier's three 64-bit words (arrivals in the low 16 bits,
+// flags summed in the next 16, the blocks' pending attempts summed in the high
+// half; used in turn) and the passes' two counts of ready attempts, all cleared
+// before every sweep and as the sweep goes on; the error, round and sequence
+// records in a line of their own; then the pass keys
+enum { CTL_WORDS = 0, CTL_READY = 6, CTL_ERR = 48, CTL_ROUNDS = 49, CTL_SEQ = 50, CTL_KEYS = 64 };
 
-// A barrier over the whole (co-resident, cooperatively launched) grid whose
+// The n-th barrier of a sweep over the whole (co-resident, cooperatively
+// launched) grid; *left: the sum of every block's `pending`, *flags of every
+// block's `flag`.  The block's
+// writes are ordered before the arrival by the block barrier and the release,
+// the others' before what follows by the acquire and the block barrier.  The
 // wait gives up after S.barrier_ns; false then, on every thread of the block.
 // The block S.withhold (a failure test) never arrives and returns false.
-__device__ __forceinline__ bool grid_barrier(const PassScratch &S, int *s_ok) {
+// (Count and arrival in one word: the count apart cost another read of L2 each
+// round before any work.)
+__device__ __forceinline__ bool grid_barrier(const PassScratch &S, uint32_t n, uint32_t pending, uint32_t flag,
+                                             uint32_t *left, uint32_t *flags, uint32_t *s_word) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        int ok = 1;
+        uint32_t ok = 1, sum = 0, any = 0;
         if ((int)blockIdx.x == S.withhold) {
             ok = 0;
         } else {
-            uint32_t *ctl = S.ctl;
-            const uint32_t g0 = ld_acquire_gpu(ctl + CTL_GEN);
-            __threadfence();
-            if (atomicAdd(ctl + CTL_BAR, 1u) == gridDim.x - 1) {
-                ctl[CTL_BAR] = 0u;
-                __threadfence();
-                atomicAdd(ctl + CTL_GEN, 1u);
-            } else {
-                uint32_t spins = 0;
-                uint64_t t0 = 0;
-                while (ld_acquire_gpu(ctl + CTL_GEN) == g0) {
-                    if ((++spins & 255u) == 0) {  // the clock only now and then
-                        const uint64_t t = global_ns();
-                        if (t0 == 0) t0 = t;
-                        else if (t - t0 > S.barrier_ns) { ok = 0; break; }
-                    }
+            unsigned long long *w = (unsigned long long *)(S.ctl + CTL_WORDS);
+            const unsigned long long mine = 1ull | ((unsigned long long)flag << 16) | ((unsigned long long)pending << 32);
+            asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(w + n % 3), "l"(mine) : "memory");
+            uint32_t spins = 0;
+            uint64_t t0 = 0;
+            for (;;) {
+                unsigned long long v;
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w + n % 3) : "memory");
+                if (((uint32_t)v & 0xFFFFu) == gridDim.x) {
+                    sum = (uint32_t)(v >> 32);
+                    any = ((uint32_t)v >> 16) & 0xFFFFu;
+                    break;
+                }
+                if ((++spins & 255u) == 0) {  // the clock only now and then
+                    const uint64_t t = global_ns();
+                    if (t0 == 0) t0 = t;
+                    else if (t - t0 > S.barrier_ns) { ok = 0; break; }
                 }
             }
+            // every block has left the barrier before this one
+            if (blockIdx.x == 0) w[(n + 2) % 3] = 0ull;
         }
-        __threadfence();
-        *s_ok = ok;
+        s_word[0] = ok;
+        s_word[1] = sum;
+        s_word[2] = any;
     }
     __syncthreads();
-    return *s_ok != 0;
+    *left = s_word[1];
+    *flags = s_word[2];
+    return s_word[0] != 0;
 }
 
-// Append `v` (where `take`) to `list` at a slot counted by *s_n, one
-// shared-memory atomic per warp.
-template <typename V>
-__device__ __forceinline__ void warp_append(V *list, uint32_t *s_n, bool take, const V &v) {
+// This lane's slot (where `take`) in a list counted by *s_n, one shared-memory
+// atomic per warp.
+__device__ __forceinline__ uint32_t warp_slot(uint32_t *s_n, bool take) {
     const int lane = threadIdx.x & 31;
     const unsigned m = __ballot_sync(0xffffffffu, take);
     uint32_t base = 0;
     if (lane == 0 && m) base = atomicAdd(s_n, (uint32_t)__popc(m));
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (take) list[base + __popc(m & ((1u << lane) - 1u))] = v;
+    return base + __popc(m & ((1u << lane) - 1u));
 }
 
 // The history whose chunks hold chunk vb (plan: nh + 1 prefix of chunks).
@@ -457,18 +569,19 @@ __global__ void k_span_finish(int32_t *span, const int4 *dims, int nh) {
     }
 }
 
-// The pass plan of every volume history from its span: the chunks of PT sites
+// The pass plan of every volume history from its span: the chunks of PW items
 // the largest colour of the span holds, as a prefix over the histories
 // (vplan[nh] = all of them).  One block: each thread sums a run of
 // histories, the runs' totals are scanned, then each run is written.
-__global__ void __launch_bounds__(1024) k_pass_plan(const int32_t *span, int nh, int period, int32_t *vplan) {
+__global__ void __launch_bounds__(1024) k_pass_plan(const int32_t *span, int nh, int period, int useg,
+                                                    int32_t *vplan) {
     __shared__ int32_t s_run[1024];
     const int per = (nh + blockDim.x - 1) / blockDim.x;
     const int h0 = threadIdx.x * per, h1 = min(h0 + per, nh);
     auto chunks = [&](int h) -> int32_t {
         const int32_t *s = span + 6 * h;
-        const int64_t n = colour_sites_max(s[3] - s[0] + 1, s[4] - s[1] + 1, s[5] - s[2] + 1, period);
-        return (int32_t)((n + PT - 1) / PT);
+        const int64_t n = colour_items(s[3] - s[0] + 1, s[4] - s[1] + 1, s[5] - s[2] + 1, period, useg);
+        return (int32_t)((n + PW - 1) / PW);
     };
     int32_t tot = 0;
     for (int h = h0; h < h1; ++h) tot += chunks(h);
@@ -491,257 +604,627 @@ __global__ void __launch_bounds__(1024) k_pass_plan(const int32_t *span, int nh,
     }
 }
 
-// One sublattice pass: one copy attempt at every pixel of this pass's colour
-// (the reference's try_flip, cpm.rs:797-838) inside each history's box (a
-// volume's occupied span, a plane's whole box), the attempts ordered by a
-// per-pass priority and run as that sequence would run them.  The pixels of
-// a colour lie outside one another's reach, so two attempts meet only
-// through the records of a cell they both involve (volume, surface).
+// The acceptance of an attempt: Delta-H <= 0, or u < exp(-Delta-H / T) with
+// own_exp.  Its limit, -T ln u taken once before the pass runs, decides all but
+// the Delta-H within 1e-10 of it (own_exp, the quotient and the limit are each
+// within 1e-14 relatively), which take the exponential: it is a third of an
+// attempt's time in the chain of attempts that bounds a pass.  A limit that is
+// not a number (u = 0, a temperature that is none) decides nothing.
+__device__ __forceinline__ double accept_limit(uint32_t u0, uint32_t u1, double T) {
+    const double u = u01(u0, u1);
+    return u > 0.0 && T > 0.0 ? -T * log(u) : (double)NAN;
+}
+__device__ __noinline__ bool accept_exactly(double delta, uint32_t u0, uint32_t u1, double T) {
+    return u01(u0, u1) < own_exp(-delta / T);
+}
+__device__ __forceinline__ bool decide(double delta, double limit, uint32_t u0, uint32_t u1, double T) {
+    if (delta <= 0.0) return true;
+    const double margin = 1e-10 * (T + limit);
+    if (delta < limit - margin) return true;
+    if (delta > limit + margin) return false;
+    return accept_exactly(delta, u0, u1, T);
+}
+
+// A cell's records on their way from one of its attempts to the next: bit 63
+// set, the sending attempt's depth (10 bits), the surface (25, signed) and the
+// volume (28, signed).  Cells past these ranges take the rounds.
+__device__ __forceinline__ unsigned long long pack_records(int32_t vol, int32_t surf, uint32_t depth) {
+    return (1ull << 63) | ((unsigned long long)min(depth, 1023u) << 53) | ((unsigned long long)((uint32_t)surf & 0x1FFFFFFu) << 28) |
+           (unsigned long long)((uint32_t)vol & 0xFFFFFFFu);
+}
+__device__ __forceinline__ bool records_fit(int32_t vol, int32_t surf) {
+    // (a pass changes a volume by CHAIN at most, a surface by 6 CHAIN)
+    return vol > -(1 << 27) + 1024 && vol < (1 << 27) - 1024 && surf > -(1 << 24) + 1024 && surf < (1 << 24) - 1024;
+}
+
+struct PassShared {
+    double J[64];
+    int8_t reach[3 * 124];
+    uint32_t word[3], n, pending[2], ready, odd;
+    int32_t plan[PLAN_SMEM];
+    uint4 edge[PW][64];        // proposals: pixels beside another id, gathered by each warp (x, y: where; z: id);
+                               // links: its ready attempts
+    uint32_t pend[2][PEND];    // rounds: the pending attempts
+};
+
+// One sweep of every colour: a sublattice pass each, one copy attempt at every
+// pixel of the pass's colour (the reference's try_flip, cpm.rs:797-838) inside
+// each history's box (a volume's occupied span, a plane's whole box), the
+// attempts ordered by a per-pass priority and run as that sequence would run
+// them.  The pixels of a colour lie outside one another's reach, so two
+// attempts meet only through the records of a cell they both involve (volume,
+// surface).
 //
-// Propose: every attempt that copies (source and copied ids differ, neither
-// the obstacle) claims its cells other than the medium with its priority and
-// is packed into its block's segment; then the terms the pass cannot change
-// (contact, surface counts) are taken over the packed attempts.  Rounds: an
-// attempt holding the claim on all its cells runs against the live records;
-// the others claim again for the next round.  An attempt runs only after
-// every higher-priority attempt sharing a cell with it, which is the
-// sequence in decreasing priority, whatever the thread schedule.  The blocks
-// meet at a grid barrier between rounds and count what is left in one word;
-// each block lists its pending attempts by index, in shared memory when they
-// fit.
-__global__ void __launch_bounds__(PT, 1) k_cpm_pass(LatView L, Tables tabs, int nh, const int32_t *perm, int pass,
-                                                    const uint32_t *mcs_cur, PassScratch S) {
-    // a pass queued after one that gave up does nothing: the barrier's count
-    // and the claims that one left behind are cleared by the host first
+// Propose: each warp takes rows' segments of the colour, a lane up to UMAX
+// pixels at once, and gathers the pixels that border another id; 32 of those
+// at a time draw their attempt.  An attempt that copies (source and copied ids
+// differ, neither the obstacle) is packed into its block's segment and listed
+// with its cells (not the medium).
+//
+// Link: every attempt finds in its cells' lists the one that follows it (the
+// next lower priority) and whether any goes before; the terms the pass cannot
+// change are taken.
+//
+// Run: an attempt that no other goes before on any of its cells runs, and hands
+// each cell's records to the attempt that follows there, in that one's mailbox;
+// of the two that meet in a mailbox the second finds the first's records and
+// runs the attempt.  The last attempt on a cell writes its records.  So every
+// attempt runs after all of higher priority that share a cell with it, which
+// is the sequence in decreasing priority, whatever the thread schedule, and
+// nothing waits: the blocks meet three times a pass.
+//
+// Rounds: a pass with a cell of more than CHAIN attempts (or records past
+// pack_records' ranges), or without room for the lists, runs by claims: every
+// attempt claims its cells with its priority, one that holds all its claims
+// runs against the live records, the others claim again, a meeting of the
+// blocks between rounds.  The same sequence.
+//
+// What bounds a pass is its longest chain of attempts that share cells (11 to 36
+// of them where cells have 50 to 125 pixels).  A round of claims costs 2 us of
+// meeting and two or three reads of L2 in turn, 4-6 us in all; an attempt of a
+// chain costs one exchange in L2 with its terms read behind it, about 1 us.
+// Large lattices are bound by the attempts' lines, 128 bytes each, in the
+// proposals and the terms.  Measured against a launch a pass of rounds only, a
+// Monte Carlo step: a 96^3 ball of 125-voxel cells with surfaces (8 passes, 36
+// attempts deep) 1,750 -> 650 us, the 256^3 spheroid 1,830 -> 667, a 300 x 300
+// tissue (4 sub-sweeps of 2 passes) 840 -> 322, 256 x 256 265 -> 109, the 2048 x
+// 2048 cord 757 -> 426, the campaign's 22.3 M pixels 1,490 -> 1,360.
+__global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int nh, const int32_t *perm,
+                                                     const uint32_t *mcs_cur, PassScratch S) {
+    // a sweep queued after one that gave up does nothing: the barrier's words,
+    // the lists and the claims that one left behind are cleared by the host first
     if (__ldcg(S.ctl + CTL_ERR) != 0u) return;
-    __shared__ double sJ[64];
-    __shared__ int8_t sreach[3 * 124];
-    __shared__ int s_ok;
-    __shared__ uint32_t s_n[2];
-    __shared__ int32_t s_plan[PLAN_SMEM];
-    __shared__ uint32_t s_pend[2][PEND_SMEM];
-    for (int i = threadIdx.x; i < L.K * L.K; i += blockDim.x) sJ[i] = tabs.J[i];
-    for (int i = threadIdx.x; i < 3 * L.nreach; i += blockDim.x) sreach[i] = tabs.reach[i];
+    __shared__ PassShared P;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < L.K * L.K; i += PT) P.J[i] = tabs.J[i];
+    for (int i = threadIdx.x; i < 3 * L.nreach; i += PT) P.reach[i] = tabs.reach[i];
     const bool plan_shared = nh + 1 <= PLAN_SMEM;
     if (plan_shared)
-        for (int i = threadIdx.x; i <= nh; i += blockDim.x) s_plan[i] = S.vplan[i];
-    if (threadIdx.x == 0) s_n[0] = s_n[1] = 0u;
+        for (int i = threadIdx.x; i <= nh; i += PT) P.plan[i] = S.vplan[i];
     __syncthreads();
-    const int32_t *plan = plan_shared ? s_plan : S.vplan;
+    const int32_t *plan = plan_shared ? P.plan : S.vplan;
     const int nvb = plan[nh];
     const uint32_t mcs = *mcs_cur;
-    const uint32_t seq = S.ctl[CTL_SEQ];
-    const uint32_t tag0 = seq * ROUND_SPAN;  // round r claims with tag tag0 + r
     const uint32_t *pass_key = S.ctl + CTL_KEYS;
-    Attempt *mine = S.list + (size_t)blockIdx.x * S.seg;
-    // ---- propose and claim (round 1's claims); a block's chunks come in
-    // increasing order, so its history only moves forward
-    int h = blockIdx.x < nvb ? plan_find(plan, nh, blockIdx.x) : 0;
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-        while (h + 1 < nh && plan[h + 1] <= vb) ++h;
-        const int4 dm = L.dims[h];
-        int box[6] = {0, 0, 0, dm.x - 1, dm.y - 1, dm.z - 1};
-        if (L.span && dm.z > 1)
-#pragma unroll
-            for (int a = 0; a < 6; ++a) box[a] = L.span[6 * h + a];
-        const int colour = perm[h * L.ncol + pass];
-        const uint32_t k = (uint32_t)(vb - plan[h]) * PT + threadIdx.x;
-        const int32_t *g = L.grid + L.off[h];
-        int x = 0, y = 0, z = 0;
-        bool copies = false;
-        Attempt a;
-        if (colour_site_box(box, L.period, colour, k, x, y, z)) {
+    const uint32_t id0 = blockIdx.x * S.seg;  // this block's first attempt
+    Attempt *const mine = S.list + id0;
+    const int h0 = blockIdx.x < nvb ? plan_find(plan, nh, blockIdx.x) : 0;
+    uint32_t seq = S.ctl[CTL_SEQ], bar = 0, left = 0, most = 0;
+    const bool surf_on = L.surface_on != 0;
+    auto gave_up = [&]() {
+        if (threadIdx.x == 0) atomicExch(S.ctl + CTL_ERR, 1u);
+    };
+    for (int pass = 0; pass < L.ncol; ++pass) {
+        if (threadIdx.x == 0) P.n = P.ready = P.odd = 0u;
+        __syncthreads();
+        // ---- propose
+        // 32 gathered pixels (those of the lanes with `live`): their attempts
+        auto draw = [&](uint4 px, bool live) {
+            if (!live) px = make_uint4(0u, 0u, 0u, 0u);
+            const int h = (int)(px.x & 0xFFFFu);
+            const int x = (int)(px.y & 0xFFFFu), y = (int)(px.y >> 16), z = (int)(px.x >> 16);
+            const int4 dm = __ldg(L.dims + h);
+            const int64_t off = __ldg(L.off + h);
             const int64_t i = ((int64_t)z * dm.y + y) * dm.x + x;
-            const int32_t src = __ldg(g + i);
-            // a pixel whose copy neighbours all hold its own id cannot copy: no draw needed
-            bool edge = false;
-            int nvn = 0;
-            Vn vn;
-            Moore mo;
-            // every neighbour read at once (no read waits on another's test)
-            if (!L.copy_moore) {
-                vn = vn_of(dm, x, y, z);
-                nvn = vn.count();
-                int32_t nb[6];
-#pragma unroll
-                for (int q = 0; q < 6; ++q) nb[q] = vn.has(q) ? __ldg(g + i + vn.step(q)) : src;
-#pragma unroll
-                for (int q = 0; q < 6; ++q) edge |= nb[q] != src;
-            } else {
-                mo = moore_of(dm, x, y, z);
-                nvn = mo.count();
-                int32_t nb[27];
-#pragma unroll
-                for (int q = 0; q < 27; ++q)
-                    nb[q] = q != 13 && ((mo.mask >> q) & 1u) ? __ldg(g + i + mo.step(q)) : src;
-#pragma unroll
-                for (int q = 0; q < 27; ++q) edge |= nb[q] != src;
-            }
+            const int32_t *g = L.grid + off;
+            const uint2 key = __ldg(L.keys + h);
+            const uint32_t pkey = __ldcg(pass_key + h * L.ncol + pass);
+            // (a batch holds fewer than 2^32 records: their claims alone take 16 bytes each)
+            const uint32_t c0 = (uint32_t)__ldg(L.cell_off + h);
+            bool copies = live;
+            const int32_t src = (int32_t)px.z;
+            int32_t dst = 0;
+            uint4 r = make_uint4(0, 0, 0, 0);
             // with sub-sweeps, a pixel attempts in this one with probability
             // 1 / subsweeps (its own draw), so that over the Monte Carlo step
             // its attempts are Binomial(subsweeps, 1 / subsweeps), near the
             // Poisson(1) of random pixels
-            if (edge && src != OBST && L.take_below &&
-                philox((uint32_t)i, mcs, 4u, 0u, L.keys[h].x, L.keys[h].y).x >= L.take_below)
-                edge = false;
-            if (edge && src != OBST) {
-                const uint2 key = L.keys[h];
-                const uint4 r = philox((uint32_t)i, mcs, 0u, 0u, key.x, key.y);
-                const int j = (int)(((uint64_t)r.x * (uint64_t)nvn) >> 32);
-                const int32_t dst = __ldg(g + i + (L.copy_moore ? mo.nth(j) : vn.nth(j)));
-                if (src != dst && dst != OBST) {
-                    copies = true;
-                    const uint32_t prio = fmix32((uint32_t)i ^ pass_key[h * L.ncol + pass]);
-                    const int64_t c0 = L.cell_off[h];
-                    const unsigned long long claim = ((unsigned long long)(tag0 + 1u) << 32) | prio;
-                    if (src > 0) atomicMax(S.claim[1] + c0 + src, claim);
-                    if (dst > 0) atomicMax(S.claim[1] + c0 + dst, claim);
-                    a.c0 = c0;
-                    a.src = src;
-                    a.dst = dst;
-                    a.prio = prio;
-                    a.dsurf = 0;
-                    a.u0 = r.y;
-                    a.u1 = r.z;
-                    a.gi = L.off[h] + i;
-                    a.where = make_uint2((uint32_t)h | ((uint32_t)z << 16), (uint32_t)x | ((uint32_t)y << 16));
+            if (copies && L.take_below && philox((uint32_t)i, mcs, 4u, 0u, key.x, key.y).x >= L.take_below)
+                copies = false;
+            if (copies) {
+                r = philox((uint32_t)i, mcs, 0u, 0u, key.x, key.y);
+                int64_t step;
+                if (!L.copy_moore) {
+                    const Vn vn = vn_of(dm, x, y, z);
+                    step = vn.nth((int)(((uint64_t)r.x * (uint64_t)vn.count()) >> 32));
+                } else {
+                    const Moore mo = moore_of(dm, x, y, z);
+                    step = mo.nth((int)(((uint64_t)r.x * (uint64_t)mo.count()) >> 32));
                 }
+                dst = g[i + step];
+                copies = src != dst && dst != OBST;
             }
-        }
-        warp_append(mine, &s_n[0], copies, a);
-    }
-    __syncthreads();
-    const uint32_t n = s_n[0];
-    // ---- what the pass cannot change, over the block's attempts packed
-    // together (a contact term reads no pixel of the colour, which only the
-    // rounds write)
-    for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
-        Attempt &a = mine[e];
-        const uint2 wh = a.where;
-        const int hh = (int)(wh.x & 0xFFFFu);
-        const int x = (int)(wh.y & 0xFFFFu), y = (int)(wh.y >> 16), z = (int)(wh.x >> 16);
-        const int4 dm = L.dims[hh];
-        const int64_t cap = L.cell_off[hh + 1] - a.c0;
-        const int64_t i = ((int64_t)z * dm.y + y) * dm.x + x;
-        const int32_t *g = L.grid + L.off[hh];
-        const Vn vn = vn_of(dm, x, y, z);
-        double num;
-        const double contact = contact_delta(g, dm, x, y, z, a.src, a.dst, L.type + a.c0, cap, sJ, L.K, sreach,
-                                             L.nreach, L.across, i, vn, &num);
-        int32_t ds = 0, dd = 0;
-        if (L.surface_on) surface_change(g, i, vn, a.src, a.dst, ds, dd);
-        a.contact = contact;
-        a.dsurf = (int32_t)((uint32_t)(uint16_t)(int16_t)ds | ((uint32_t)(uint16_t)(int16_t)dd << 16));
-    }
-    if (threadIdx.x == 0 && n) atomicAdd(S.ctl + CTL_COUNT + 0, n);
-    uint32_t *pend[2] = {s_pend[0], s_pend[1]};
-    if (n > PEND_SMEM) {
-        pend[0] = S.idx + (size_t)blockIdx.x * 2 * S.seg;
-        pend[1] = pend[0] + S.seg;
-    }
-    if (!grid_barrier(S, &s_ok)) {
-        if (threadIdx.x == 0) atomicExch(S.ctl + CTL_ERR, 1u);
-        return;
-    }
-    // ---- rounds
-    uint32_t npend = n;  // this block's attempts entering the round
-    for (int r = 1;; ++r) {
-        const uint32_t left = __ldcg(S.ctl + CTL_COUNT + (r - 1) % 3);
-        if (left == 0) break;
-        if (r > S.max_rounds) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(S.ctl + CTL_ERR, 2u);
-            break;
-        }
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            S.ctl[CTL_COUNT + (r + 1) % 3] = 0u;  // round r + 1's count; last read as round r - 1's
-            atomicMax(S.ctl + CTL_ROUNDS, (uint32_t)r);
-        }
-        if (threadIdx.x == 0) s_n[r & 1] = 0u;
-        __syncthreads();
-        const unsigned long long *cl = S.claim[r & 1];
-        unsigned long long *next = S.claim[(r + 1) & 1];
-        const uint32_t *pin = pend[(r - 1) & 1];
-        uint32_t *pout = pend[r & 1];
-        const unsigned long long key_tag = (unsigned long long)(tag0 + (uint32_t)r) << 32;
-        const unsigned long long next_tag = (unsigned long long)(tag0 + (uint32_t)r + 1u) << 32;
-        for (uint32_t e0 = 0; e0 < npend; e0 += ILP * PT) {
-            uint32_t id[ILP];
-            bool has[ILP], win[ILP];
-            Attempt a[ILP];
-            unsigned long long cs[ILP], cd[ILP];
-#pragma unroll
-            for (int j = 0; j < ILP; ++j) {
-                const uint32_t e = e0 + (uint32_t)j * PT + threadIdx.x;
-                has[j] = e < npend;
-                id[j] = has[j] ? (r == 1 ? e : pin[e]) : 0u;
+            const uint32_t e = warp_slot(&P.n, copies);
+            if (!copies) return;
+            const uint32_t prio = fmix32((uint32_t)i ^ pkey);
+            const uint32_t cs = src > 0 ? c0 + (uint32_t)src : NONE, cd = dst > 0 ? c0 + (uint32_t)dst : NONE;
+            if (S.chain) {
+                // both places taken at once
+                uint32_t ks = 0, kd = 0;
+                if (cs != NONE) ks = atomicAdd(S.count + cs, 1u);
+                if (cd != NONE) kd = atomicAdd(S.count + cd, 1u);
+                const bool only = cs == NONE || cd == NONE;
+                const unsigned long long entry = ((unsigned long long)prio << 32) | ((id0 + e) << 2) | (only ? 2u : 0u);
+                if (cs != NONE && ks < CHAIN) S.chain[(size_t)cs * CHAIN + ks] = entry;
+                if (cd != NONE && kd < CHAIN) S.chain[(size_t)cd * CHAIN + kd] = entry | 1u;
+                if (max(ks, kd) >= CHAIN) P.odd = 1u;
+                S.mail[id0 + e] = make_ulonglong2(0ull, 0ull);
             }
+            int4 *const w = (int4 *)(mine + e);
+            const int64_t gi = off + i;
+            w[2] = make_int4(0, 0, (int)cs, (int)cd);
+            w[3] = make_int4((int)NONE, (int)NONE, dst, 0);
+            w[4] = make_int4((int)(uint32_t)gi, (int)(gi >> 32), (int)r.y, (int)r.z);
+            w[6] = make_int4(0, 0, (int)prio, src);
+            w[7] = make_int4((int)px.x, (int)px.y, 0, 0);
+        };
+        {
+            uint4 *const gathered = P.edge[warp];
+            int have = 0;  // pixels gathered, the same in every lane
+            int h = h0;    // a block's chunks come in increasing order: its history only moves forward
+            for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+                while (h + 1 < nh && plan[h + 1] <= vb) ++h;
+                const int4 dm = __ldg(L.dims + h);
+                int box[6] = {0, 0, 0, dm.x - 1, dm.y - 1, dm.z - 1};
+                if (L.span && dm.z > 1)
 #pragma unroll
-            for (int j = 0; j < ILP; ++j)
-                if (has[j]) a[j] = mine[id[j]];
+                    for (int a = 0; a < 6; ++a) box[a] = __ldg(L.span + 6 * h + a);
+                const uint32_t item = (uint32_t)(vb - plan[h]) * PW + (uint32_t)warp;
+                const uint32_t segs = (uint32_t)colour_segments(box[3] - box[0] + 1, L.period, S.useg);
+                const uint32_t row = segs ? item / segs : 0u;
+                int y = 0, z = 0, fx = 0, step = 0, nx = 0;
+                if (segs == 0 || !colour_row(box, L.period, __ldg(perm + h * L.ncol + pass), row, y, z, fx, step, nx)) continue;
+                const int j0 = (int)(item - row * segs) * 32 * S.useg + lane;
+                const int32_t *g = L.grid + __ldg(L.off + h) + ((int64_t)z * dm.y + y) * dm.x;
+                const int64_t w = dm.x, slice = (int64_t)dm.x * dm.y;
+                const bool up = y > 0, down = y + 1 < dm.y, in = z > 0, out = z + 1 < dm.z;
+                // every pixel's neighbours read at once (no read waits on another's
+                // test); a pixel whose copy neighbours all hold its own id cannot copy
+                bool edge[UMAX];
+                int xs[UMAX];
+                int32_t src[UMAX];
+                if (!L.copy_moore) {
+                    int32_t nb[UMAX][6];
+                    unsigned there[UMAX];
 #pragma unroll
-            for (int j = 0; j < ILP; ++j) {
-                cs[j] = cd[j] = 0ull;
-                if (has[j]) {
-                    if (a[j].src > 0) cs[j] = __ldcg(cl + a[j].c0 + a[j].src);
-                    if (a[j].dst > 0) cd[j] = __ldcg(cl + a[j].c0 + a[j].dst);
-                }
-            }
+                    for (int u = 0; u < UMAX; ++u) {
+                        const int j = j0 + 32 * u;
+                        const bool live = u < S.useg && j < nx;
+                        const int x = xs[u] = fx + step * j;
+                        src[u] = OBST;
+                        if (live) src[u] = g[x];
+                        // (not `: src[u]`: taking the pixel's own id where there is no
+                        // neighbour holds every later read until that id has come)
+                        const bool has[6] = {live && up, live && down, live && x > 0, live && x + 1 < dm.x, live && in,
+                                             live && out};
+                        const int64_t to[6] = {-w, w, -1, 1, -slice, slice};
+                        there[u] = 0u;
 #pragma unroll
-            for (int j = 0; j < ILP; ++j) {
-                win[j] = false;
-                if (has[j]) {
-                    const unsigned long long key = key_tag | a[j].prio;
-                    win[j] = (a[j].src <= 0 || cs[j] == key) && (a[j].dst <= 0 || cd[j] == key);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < ILP; ++j) {
-                bool again = false;
-                if (win[j]) {
-                    const Attempt &t = a[j];
-                    const int32_t ds = (int32_t)(int16_t)(t.dsurf & 0xFFFF), dd = (int32_t)(int16_t)(t.dsurf >> 16);
-                    double delta = t.contact + volume_delta(L.volume, L.target, L.lambda, t.c0, t.src, t.dst);
-                    if (L.surface_on) delta += surface_delta(L.surface, L.tsurf, L.lsurf, t.c0, t.src, t.dst, ds, dd);
-                    bool accept = delta <= 0.0;
-                    if (!accept) accept = u01(t.u0, t.u1) < own_exp(-delta / L.temperature);
-                    if (accept) {
-                        L.grid[t.gi] = t.dst;
-                        // the records: its cells are its own this round
-                        if (t.src != 0) L.volume[t.c0 + t.src] -= 1;
-                        if (t.dst != 0) L.volume[t.c0 + t.dst] += 1;
-                        if (L.surface_on) {
-                            if (t.src > 0) L.surface[t.c0 + t.src] += ds;
-                            if (t.dst > 0) L.surface[t.c0 + t.dst] += dd;
+                        for (int q = 0; q < 6; ++q) {
+                            nb[u][q] = 0;
+                            if (has[q]) {
+                                nb[u][q] = g[x + to[q]];
+                                there[u] |= 1u << q;
+                            }
                         }
                     }
-                } else if (has[j]) {
-                    const unsigned long long claim = next_tag | a[j].prio;
-                    if (a[j].src > 0) atomicMax(next + a[j].c0 + a[j].src, claim);
-                    if (a[j].dst > 0) atomicMax(next + a[j].c0 + a[j].dst, claim);
-                    again = true;
+#pragma unroll
+                    for (int u = 0; u < UMAX; ++u) {
+                        edge[u] = false;
+#pragma unroll
+                        for (int q = 0; q < 6; ++q) edge[u] |= ((there[u] >> q) & 1u) && nb[u][q] != src[u];
+                        edge[u] = edge[u] && src[u] != OBST;
+                    }
+                } else {
+#pragma unroll 1
+                    for (int u = 0; u < UMAX; ++u) {
+                        const int j = j0 + 32 * u;
+                        const int x = fx + step * j;
+                        bool e = false;
+                        int32_t own = OBST;
+                        if (u < S.useg && j < nx) {
+                            own = g[x];
+                            const Moore mo = moore_of(dm, x, y, z);
+                            if (own != OBST)
+                                for (int q = 0; q < 27; ++q)
+                                    if ((mo.mask >> q) & 1u) e |= g[x + mo.step(q)] != own;
+                        }
+#pragma unroll
+                        for (int v = 0; v < UMAX; ++v)
+                            if (v == u) { edge[v] = e; xs[v] = x; src[v] = own; }
+                    }
                 }
-                warp_append(pout, &s_n[r & 1], again, id[j]);
+#pragma unroll
+                for (int u = 0; u < UMAX; ++u) {
+                    const unsigned m = __ballot_sync(0xffffffffu, edge[u]);
+                    if (edge[u])
+                        gathered[have + __popc(m & ((1u << lane) - 1u))] =
+                            make_uint4((uint32_t)h | ((uint32_t)z << 16), (uint32_t)xs[u] | ((uint32_t)y << 16),
+                                       (uint32_t)src[u], 0u);
+                    have += __popc(m);
+                    if (have >= 32) {
+                        __syncwarp();
+                        const uint4 px = gathered[lane], rest = gathered[32 + lane];
+                        __syncwarp();
+                        gathered[lane] = rest;
+                        have -= 32;
+                        draw(px, true);
+                        __syncwarp();
+                    }
+                }
+            }
+            __syncwarp();
+            if (have > 0) draw(gathered[lane], lane < have);
+        }
+        __syncthreads();
+        const uint32_t n = P.n;
+        uint32_t flags = 0;
+        if (!grid_barrier(S, bar++, n, P.odd, &left, &flags, P.word)) { gave_up(); return; }
+        // (the next pass's count: last used by the pass before, which is over)
+        if (blockIdx.x == 0 && threadIdx.x == 0) S.ctl[CTL_READY + ((pass + 1) & 1)] = 0u;
+        if (left == 0) continue;
+        bool linked = S.chain != nullptr && flags == 0u;
+        const uint32_t tag0 = seq * ROUND_SPAN;  // round r claims with tag tag0 + r
+        // round 1's claims
+        auto claim_first = [&](const Attempt &a) {
+            const unsigned long long claim = ((unsigned long long)(tag0 + 1u) << 32) | a.prio;
+            if (a.cs != NONE) atomicMax(S.claim[1] + a.cs, claim);
+            if (a.cd != NONE) atomicMax(S.claim[1] + a.cd, claim);
+            if (S.chain) {
+                if (a.cs != NONE) S.count[a.cs] = 0u;
+                if (a.cd != NONE) S.count[a.cd] = 0u;
+            }
+        };
+        // ---- link: a warp takes a cell's whole list, an entry or two a lane; each
+        // entry's follower into its attempt, and the cell's records to the first
+        if (linked) {
+            uint32_t *const found = (uint32_t *)P.edge[warp];
+            uint32_t have = 0;  // ready attempts found and not yet in the list, the same in every lane
+            auto flush = [&](uint32_t m) {
+                __syncwarp();
+                uint32_t at = 0;
+                if (lane == 0) {
+                    at = atomicAdd(S.ctl + CTL_READY + (pass & 1), m);
+                    atomicAdd(&P.ready, m);
+                }
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (lane < m) S.idx[at + lane] = found[lane];
+                __syncwarp();
+            };
+            // (a warp's cells lie a stride apart: those with attempts are often the
+            // first of the records)
+            const int64_t stride = (int64_t)gridDim.x * PW;
+            for (int64_t c0 = blockIdx.x * PW + warp; c0 < S.ncells; c0 += 32 * stride) {
+                const uint32_t cnt = c0 + lane * stride < S.ncells ? __ldcg(S.count + c0 + lane * stride) : 0u;
+                for (unsigned live = __ballot_sync(0xffffffffu, cnt != 0u); live; live &= live - 1u) {
+                    const int q = __ffs(live) - 1;
+                    const uint32_t k = __shfl_sync(0xffffffffu, cnt, q);
+                    const size_t c = (size_t)(c0 + q * stride);
+                    const unsigned long long *list = S.chain + c * CHAIN;
+                    const int32_t vol = __ldcg(L.volume + c), surf = surf_on ? __ldcg(L.surface + c) : 0;
+                    unsigned long long mine2[2] = {lane < k ? __ldcg(list + lane) : 0ull,
+                                                   lane + 32 < k ? __ldcg(list + 32 + lane) : 0ull};
+                    if (!records_fit(vol, surf)) P.odd = 1u;
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        if (half && k <= 32) break;
+                        const unsigned long long own = mine2[half];
+                        const uint32_t prio = (uint32_t)(own >> 32);
+                        unsigned long long below = 0ull;
+                        bool followed = false, first = lane + 32u * half < k;
+                        for (uint32_t j = 0; j < k; ++j) {
+                            // (a cell's attempts have distinct priorities)
+                            const unsigned long long x = __shfl_sync(0xffffffffu, j < 32 ? mine2[0] : mine2[1], j & 31);
+                            const uint32_t xp = (uint32_t)(x >> 32);
+                            if (xp > prio) first = false;
+                            if (xp < prio && (!followed || x > below)) {
+                                below = x;
+                                followed = true;
+                            }
+                        }
+                        bool ready = false;
+                        const uint32_t id = ((uint32_t)own >> 2);
+                        if (lane + 32u * half < k) {
+                            if (followed) (own & 1ull ? S.list[id].next_d : S.list[id].next_s) = (uint32_t)below;
+                            if (first) {
+                                const unsigned long long box = pack_records(vol, surf, 0u);
+                                unsigned long long met = 0ull;
+                                ready = (own & 2ull) != 0ull || (met = atomicExch(&S.mail[id].x, box)) != 0ull;
+                                if (ready) S.mail[id] = (own & 1ull) ? make_ulonglong2(met, box) : make_ulonglong2(box, met);
+                            }
+                        }
+                        // (at most one a list)
+                        if (__any_sync(0xffffffffu, ready)) {
+                            if (ready) found[have] = id;
+                            if (++have == 32) {
+                                flush(32);
+                                have = 0;
+                            }
+                        }
+                    }
+                }
+            }
+            if (have) flush(have);
+        }
+        // ---- the terms the pass cannot change, over the block's attempts packed
+        // together (a contact term reads no pixel of the colour).  Everything is
+        // read before anything is written: a write between two reads that it might
+        // change holds the second until the first has come.
+        for (uint32_t e = threadIdx.x; e < n; e += PT) {
+            Attempt *const a = mine + e;
+            if (!linked) claim_first(*a);
+            const int4 w2 = ((const int4 *)a)[2], w3 = ((const int4 *)a)[3], w4 = ((const int4 *)a)[4], w6 = ((const int4 *)a)[6],
+                       w7 = ((const int4 *)a)[7];
+            const uint32_t cs = (uint32_t)w2.z, cd = (uint32_t)w2.w;
+            const int32_t dst = w3.z, src = w6.w;
+            const int hh = w7.x & 0xFFFF;
+            const int x = w7.y & 0xFFFF, y = (int)((uint32_t)w7.y >> 16), z = (int)((uint32_t)w7.x >> 16);
+            const int4 dm = __ldg(L.dims + hh);
+            const int64_t c0 = __ldg(L.cell_off + hh), cap = __ldg(L.cell_off + hh + 1) - c0;
+            const int64_t i = ((int64_t)z * dm.y + y) * dm.x + x;
+            const int32_t *g = L.grid + __ldg(L.off + hh);
+            const Vn vn = vn_of(dm, x, y, z);
+            int32_t ts = 0, td = 0, tss = 0, tsd = 0;
+            double ls = 0.0, ld = 0.0, lss = 0.0, lsd = 0.0;
+            if (cs != NONE) {
+                ts = __ldg(L.target + cs);
+                ls = __ldg(L.lambda + cs);
+                if (surf_on) { tss = __ldg(L.tsurf + cs); lss = __ldg(L.lsurf + cs); }
+            }
+            if (cd != NONE) {
+                td = __ldg(L.target + cd);
+                ld = __ldg(L.lambda + cd);
+                if (surf_on) { tsd = __ldg(L.tsurf + cd); lsd = __ldg(L.lsurf + cd); }
+            }
+            int32_t ds = 0, dd = 0;
+            if (surf_on) surface_change(g, i, vn, src, dst, ds, dd);
+            double num;
+            const double contact = contact_delta(g, dm, x, y, z, src, dst, L.type + c0, cap, P.J, L.K, P.reach, L.nreach,
+                                                 L.across, i, vn, &num);
+            const double limit = accept_limit((uint32_t)w4.z, (uint32_t)w4.w, L.temperature);
+            ((double2 *)a)[0] = make_double2(contact, limit);
+            ((double2 *)a)[1] = make_double2(ls, ld);
+            *(int2 *)&a->ts = make_int2(ts, td);
+            a->dsurf = (int32_t)((uint32_t)(uint16_t)(int16_t)ds | ((uint32_t)(uint16_t)(int16_t)dd << 16));
+            if (surf_on) {
+                ((double2 *)a)[5] = make_double2(lss, lsd);
+                *(int2 *)&a->tss = make_int2(tss, tsd);
             }
         }
         __syncthreads();
-        npend = s_n[r & 1];
-        if (threadIdx.x == 0 && npend) atomicAdd(S.ctl + CTL_COUNT + r % 3, npend);
-        if (!grid_barrier(S, &s_ok)) {
-            if (threadIdx.x == 0) atomicExch(S.ctl + CTL_ERR, 1u);
-            return;
+        if (!grid_barrier(S, bar++, linked ? P.ready : n, P.odd, &left, &flags, P.word)) { gave_up(); return; }
+        if (linked && flags != 0u) {
+            // a cell's records past the mailboxes' ranges: by rounds
+            linked = false;
+            for (uint32_t e = threadIdx.x; e < n; e += PT) claim_first(mine[e]);
+            if (!grid_barrier(S, bar++, n, 0u, &left, &flags, P.word)) { gave_up(); return; }
+        }
+        // an attempt on the records given: accepted or not, and its writes
+        auto attempt = [&](const Terms &a, int32_t &vs, int32_t &ss, int32_t &vd, int32_t &sd) {
+            const bool has_s = a.cs != NONE, has_d = a.cd != NONE;
+            const int32_t ds = (int32_t)(int16_t)(a.dsurf & 0xFFFF), dd = (int32_t)(int16_t)(a.dsurf >> 16);
+            double delta = a.contact + volume_terms(has_s, vs, a.ts, a.ls, has_d, vd, a.td, a.ld);
+            if (surf_on) delta += surface_terms(has_s, ss, a.tss, a.lss, ds, has_d, sd, a.tsd, a.lsd, dd);
+            if (!decide(delta, a.limit, a.u0, a.u1, L.temperature)) return false;
+            L.grid[a.gi] = a.dst;
+            vs -= 1;
+            vd += 1;
+            ss += ds;
+            sd += dd;
+            return true;
+        };
+        if (linked) {
+            // ---- run the chains: a lane takes what it made ready, else its spare or
+            // its stack, else its next of the list, else another lane's spare
+            // (dealt one to a warp, then a second to each: the chains of a warp
+            // wait for one another's reads, and its idle lanes take their branches)
+            const uint32_t warps = gridDim.x * PW, stride = 32u * warps;
+            uint32_t at = blockIdx.x * PW + warp + lane * warps;
+            uint32_t id = NONE, spare = NONE, top = NONE, listed = at < left ? __ldcg(S.idx + at) : NONE;
+            // the records that the current attempt and the spare were handed
+            unsigned long long box_s = 0ull, box_d = 0ull, spare_s = 0ull, spare_d = 0ull;
+            for (;;) {
+                if (id == NONE) {
+                    if (spare != NONE) {
+                        id = spare;
+                        box_s = spare_s;
+                        box_d = spare_d;
+                        spare = NONE;
+                    } else if (top != NONE || listed != NONE) {
+                        if (top != NONE) {
+                            id = top;
+                            top = S.link[id];
+                        } else {
+                            id = listed;
+                            at += stride;
+                            listed = at < left ? __ldcg(S.idx + at) : NONE;
+                        }
+                        const ulonglong2 b = __ldcg(S.mail + id);
+                        box_s = b.x;
+                        box_d = b.y;
+                    }
+                }
+                const unsigned idle = __ballot_sync(0xffffffffu, id == NONE);
+                if (idle) {
+                    const unsigned rich = __ballot_sync(0xffffffffu, spare != NONE), below = (1u << lane) - 1u;
+                    if (rich) {
+                        const int m = min(__popc(idle), __popc(rich)), ri = __popc(idle & below), rr = __popc(rich & below);
+                        const bool takes = ((idle >> lane) & 1u) && ri < m, gives = ((rich >> lane) & 1u) && rr < m;
+                        const int from = takes ? (int)__fns(rich, 0, ri + 1) : lane;
+                        const uint32_t got = __shfl_sync(0xffffffffu, spare, from);
+                        const unsigned long long gs = __shfl_sync(0xffffffffu, spare_s, from),
+                                                 gd = __shfl_sync(0xffffffffu, spare_d, from);
+                        if (gives) spare = NONE;
+                        if (takes) {
+                            id = got;
+                            box_s = gs;
+                            box_d = gd;
+                        }
+                    } else if (idle == 0xffffffffu) {
+                        break;
+                    }
+                }
+                if (id != NONE) {
+                    Terms a;
+                    a.read(S.list + id, surf_on);
+                    const uint32_t cs = a.cs, cd = a.cd;
+                    uint32_t depth = 0;
+                    int32_t vs = 0, ss = 0, vd = 0, sd = 0;
+                    auto open = [&](unsigned long long b, uint32_t c, int32_t &vol, int32_t &surf) {
+                        if (c == NONE) return;
+                        vol = (int32_t)((uint32_t)b << 4) >> 4;
+                        surf = (int32_t)((uint32_t)(b >> 28) << 7) >> 7;
+                        depth = max(depth, (uint32_t)(b >> 53) & 1023u);
+                    };
+                    open(box_s, cs, vs, ss);
+                    open(box_d, cd, vd, sd);
+                    attempt(a, vs, ss, vd, sd);
+                    depth += 1;
+                    most = max(most, depth);
+                    const uint32_t next[2] = {cs == NONE ? NONE : a.next_s, cd == NONE ? NONE : a.next_d};
+                    const unsigned long long send[2] = {pack_records(vs, ss, depth), pack_records(vd, sd, depth)};
+                    unsigned long long met[2] = {0ull, 0ull};
+#pragma unroll
+                    for (int side = 0; side < 2; ++side)
+                        if (next[side] != NONE) {
+                            const uint32_t to = next[side] >> 2;
+                            // its terms into L1 while the exchange is on its way
+                            const char *line = (const char *)(S.list + to);
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                uint32_t t;
+                                if (q < 3 || surf_on) asm volatile("ld.global.u32 %0, [%1];" : "=r"(t) : "l"(line + 32 * q) : "memory");
+                            }
+                            if (!(next[side] & 2u)) met[side] = atomicExch(&S.mail[to].x, send[side]);
+                        }
+                    // the last attempt on a cell writes its records
+                    if (cs != NONE && next[0] == NONE) {
+                        L.volume[cs] = vs;
+                        if (surf_on) L.surface[cs] = ss;
+                        S.count[cs] = 0u;
+                    }
+                    if (cd != NONE && next[1] == NONE) {
+                        L.volume[cd] = vd;
+                        if (surf_on) L.surface[cd] = sd;
+                        S.count[cd] = 0u;
+                    }
+                    id = NONE;
+#pragma unroll
+                    for (int side = 0; side < 2; ++side) {
+                        if (next[side] == NONE || !((next[side] & 2u) || met[side])) continue;
+                        const uint32_t to = next[side] >> 2;
+                        const unsigned long long bs = (next[side] & 1u) ? met[side] : send[side],
+                                                 bd = (next[side] & 1u) ? send[side] : met[side];
+                        if (id == NONE) {
+                            id = to;
+                            box_s = bs;
+                            box_d = bd;
+                        } else {
+                            if (spare != NONE) {
+                                S.mail[spare] = make_ulonglong2(spare_s, spare_d);
+                                S.link[spare] = top;
+                                top = spare;
+                            }
+                            spare = to;
+                            spare_s = bs;
+                            spare_d = bd;
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            if (!grid_barrier(S, bar++, 0u, 0u, &left, &flags, P.word)) { gave_up(); return; }
+            continue;
+        }
+        // ---- rounds
+        const bool listed = n <= PEND;
+        uint32_t *const gpend[2] = {S.idx + id0, S.link + id0};
+        uint32_t npend = n;  // this block's attempts entering the round
+        for (uint32_t r = 1; left != 0; ++r) {
+            if ((int)r > S.max_rounds) {
+                if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(S.ctl + CTL_ERR, 2u);
+                return;
+            }
+            most = max(most, r);
+            if (threadIdx.x == 0) P.pending[r & 1] = 0u;
+            __syncthreads();
+            const unsigned long long *cl = S.claim[r & 1];
+            unsigned long long *next = S.claim[(r + 1) & 1];
+            const uint32_t *pin = listed ? P.pend[(r - 1) & 1] : gpend[(r - 1) & 1];
+            uint32_t *pout = listed ? P.pend[r & 1] : gpend[r & 1];
+            for (uint32_t e0 = 0; e0 < npend; e0 += PT) {
+                const uint32_t e = e0 + threadIdx.x;
+                const bool has = e < npend;
+                const uint32_t k = has ? (r == 1 ? e : pin[e]) : 0u;
+                bool again = false;
+                if (has) {
+                    const Attempt &a = mine[k];
+                    const unsigned long long key = ((unsigned long long)(tag0 + r) << 32) | a.prio;
+                    unsigned long long ks = key, kd = key;
+                    if (a.cs != NONE) ks = __ldcg(cl + a.cs);
+                    if (a.cd != NONE) kd = __ldcg(cl + a.cd);
+                    if (ks == key && kd == key) {
+                        int32_t vs = 0, ss = 0, vd = 0, sd = 0;
+                        if (a.cs != NONE) { vs = L.volume[a.cs]; if (surf_on) ss = L.surface[a.cs]; }
+                        if (a.cd != NONE) { vd = L.volume[a.cd]; if (surf_on) sd = L.surface[a.cd]; }
+                        Terms t;
+                        t.read(&a, surf_on);
+                        if (attempt(t, vs, ss, vd, sd)) {
+                            // the records: its cells are its own this round
+                            if (a.cs != NONE) { L.volume[a.cs] = vs; if (surf_on) L.surface[a.cs] = ss; }
+                            if (a.cd != NONE) { L.volume[a.cd] = vd; if (surf_on) L.surface[a.cd] = sd; }
+                        }
+                    } else {
+                        const unsigned long long claim = ((unsigned long long)(tag0 + r + 1u) << 32) | a.prio;
+                        if (a.cs != NONE) atomicMax(next + a.cs, claim);
+                        if (a.cd != NONE) atomicMax(next + a.cd, claim);
+                        again = true;
+                    }
+                }
+                const uint32_t slot = warp_slot(&P.pending[r & 1], again);
+                if (again) pout[slot] = k;
+            }
+            __syncthreads();
+            npend = P.pending[r & 1];
+            if (!grid_barrier(S, bar++, npend, 0u, &left, &flags, P.word)) { gave_up(); return; }
+        }
+        // the pass is over on every block: the sequence advances; at its limit
+        // the claims are cleared and it starts again
+        seq += 1u;
+        if (seq >= SEQ_LIMIT) {
+            for (int64_t c = (int64_t)blockIdx.x * PT + threadIdx.x; c < S.ncells; c += (int64_t)gridDim.x * PT)
+                S.claim[0][c] = S.claim[1][c] = 0ull;
+            seq = 0u;
+            if (!grid_barrier(S, bar++, 0u, 0u, &left, &flags, P.word)) { gave_up(); return; }
         }
     }
-    // ---- the pass is over on every block: the counts go back to zero for the
-    // next pass (no block reads them again), the sequence advances; at the
-    // sequence's limit the claims are cleared and it starts again
-    if (seq + 1u >= SEQ_LIMIT) {
-        for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < S.ncells;
-             c += (int64_t)gridDim.x * blockDim.x)
-            S.claim[0][c] = S.claim[1][c] = 0ull;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        S.ctl[CTL_COUNT + 0] = S.ctl[CTL_COUNT + 1] = S.ctl[CTL_COUNT + 2] = 0u;
-        S.ctl[CTL_SEQ] = seq + 1u >= SEQ_LIMIT ? 0u : seq + 1u;
+    // the others read the sequence as they started: all have met since
+    if (blockIdx.x == 0 && threadIdx.x == 0) S.ctl[CTL_SEQ] = seq;
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0 && most) {
+        atomicMax(S.ctl + CTL_ROUNDS, most);
+        // (past the limit the sequence has still run whole)
+        if ((int)most > S.max_rounds) atomicExch(S.ctl + CTL_ERR, 2u);
     }
 }
 
@@ -870,47 +1353,76 @@ int cw_lattice_s::build_plans() {
         period = r + 1;
         ncol = volume ? period * period * period : period * period;
     }
-    // the pass plan: chunks of PT sites, as many as the largest colour of each
-    // history's box holds (a plane's plan; in a volume a bound of the plan the
-    // device takes from the occupied span every Monte Carlo step)
-    std::vector<int32_t> vp(g.nh + 1, 0);
-    for (uint32_t k = 0; k < g.nh; ++k) {
-        const int64_t sites = colour_sites_max(g.w[k], g.h[k], g.d[k], period);
-        vp[k + 1] = vp[k] + (int32_t)((sites + PT - 1) / PT);
-    }
     int rc;
     if (pass_grid == 0) {
         int per_sm = 0, dev = 0, nsm = 0;
-        CW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_cpm_pass, PT, 0));
+        CW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_cpm_sweep, PT, 0));
         CW_CUDA(cudaGetDevice(&dev));
         CW_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        pass_grid = std::max(1, per_sm * nsm);
+        pass_grid = std::max(1, per_sm > 0 ? nsm : 0);
     }
-    // the pass scratch: a block's segment holds every site of the chunks it
-    // visits, (chunks / blocks launched, rounded up) x PT
+    // the pass plan: chunks of PW items, as many as the largest colour of each
+    // history's box holds (a plane's plan; in a volume a bound of the plan the
+    // device takes from the occupied span every Monte Carlo step).  A lane of an
+    // item reads as many pixels (4, 2 or 1) as still give every block four chunks.
+    std::vector<int32_t> vp(g.nh + 1, 0);
+    for (useg = UMAX; useg >= 1; useg /= 2) {
+        for (uint32_t k = 0; k < g.nh; ++k) {
+            const int64_t items = colour_items(g.w[k], g.h[k], g.d[k], period, useg);
+            vp[k + 1] = vp[k] + (int32_t)((items + PW - 1) / PW);
+        }
+        if (useg == 1 || vp[g.nh] >= 4 * pass_grid) break;
+    }
+    // the pass scratch: a block's segment holds every pixel of the chunks it
+    // visits, (chunks / blocks launched, rounded up) items of 32 useg
     const int32_t nvb = vp[g.nh];
     pass_blocks = std::max(1, std::min(nvb, pass_grid));
-    pass_seg = (int64_t)((nvb + pass_blocks - 1) / pass_blocks) * PT;
-    const int64_t need = (int64_t)pass_blocks * pass_seg;
-    if (need > plist_cap) {
-        dfree(plist);
-        dfree(pidx);
-        plist_cap = 0;
-        if ((rc = dalloc(&plist, 3 * (size_t)need)) != CW_OK) return rc;  // an attempt is 3 uint4
-        if ((rc = dalloc(&pidx, 2 * (size_t)need)) != CW_OK) return rc;   // two pending lists
-        plist_cap = need;
-    }
+    pass_seg = (int64_t)((nvb + pass_blocks - 1) / pass_blocks) * PW * 32 * useg;
     if (!d_vplan && (rc = dalloc(&d_vplan, (size_t)g.nh + 1)) != CW_OK) return rc;
     CW_CUDA(cudaMemcpyAsync(d_vplan, vp.data(), sizeof(int32_t) * (g.nh + 1), cudaMemcpyHostToDevice, stream()));
-    if (!claim) {
-        if ((rc = dalloc(&claim, 2 * (size_t)ncells)) != CW_OK) return rc;
-        CW_CUDA(cudaMemsetAsync(claim, 0, sizeof(unsigned long long) * 2 * (size_t)ncells, stream()));
-    }
     if (!pctl) {
         if ((rc = dalloc(&pctl, CTL_KEYS + 27 * (size_t)g.nh)) != CW_OK) return rc;
         CW_CUDA(cudaMemsetAsync(pctl, 0, sizeof(uint32_t) * (CTL_KEYS + 27 * (size_t)g.nh), stream()));
     }
     CW_CUDA(cudaStreamSynchronize(stream()));
+    return CW_OK;
+}
+
+// The passes' scratch, taken by the first sweep (a lattice is made with the
+// chessboard's plan, twice the pixels of a colour that the contact set on it
+// usually has).
+int cw_lattice_s::ensure_scratch() {
+    int rc;
+    const int64_t need = (int64_t)pass_blocks * pass_seg;
+    if (need > plist_cap) {
+        dfree(plist);
+        dfree(pidx);
+        dfree(pmail);
+        plist_cap = 0;
+        if ((rc = dalloc(&plist, sizeof(Attempt) / sizeof(uint4) * (size_t)need)) != CW_OK) return rc;
+        if ((rc = dalloc(&pidx, 2 * (size_t)need)) != CW_OK) return rc;
+        if ((rc = dalloc(&pmail, (size_t)need)) != CW_OK) return rc;
+        plist_cap = need;
+    }
+    if (!claim) {
+        if ((rc = dalloc(&claim, 2 * (size_t)ncells)) != CW_OK) return rc;
+        CW_CUDA(cudaMemsetAsync(claim, 0, sizeof(unsigned long long) * 2 * (size_t)ncells, stream()));
+    }
+    // the cells' lists, 512 bytes a record: a batch of so many records that they
+    // would take more than 1 GiB, or a device without the room, runs its passes
+    // by rounds (so does one of more than 2^30 attempts, which a list's entry
+    // does not number)
+    if (!chain_tried && ncells * (int64_t)(CHAIN * sizeof(unsigned long long)) <= (1ll << 30)) {
+        chain_tried = true;
+        if (cudaMalloc((void **)&pcount, sizeof(uint32_t) * (size_t)ncells) != cudaSuccess ||
+            cudaMalloc((void **)&pchain, sizeof(unsigned long long) * CHAIN * (size_t)ncells) != cudaSuccess) {
+            (void)cudaGetLastError();
+            dfree(pcount);
+            pchain = nullptr;
+        } else {
+            CW_CUDA(cudaMemsetAsync(pcount, 0, sizeof(uint32_t) * (size_t)ncells, stream()));
+        }
+    }
     return CW_OK;
 }
 
@@ -986,8 +1498,8 @@ int lattice_recount(cw_lattice_s *l, int32_t *vol_out, int32_t *surf_out) {
 }
 
 // One Monte Carlo step of every history (no host synchronisation): the
-// colour order, then one cooperative launch per colour (its rounds meet at a
-// grid barrier), the claims and control words cleared before each.
+// colour order, then one cooperative launch of every colour's pass (their
+// rounds meet at a grid barrier).
 int lattice_span_enqueue(cw_lattice_s *l) {
     if (!l->d_span) return CW_OK;
     Plan &p = l->site_plan;
@@ -1004,7 +1516,7 @@ int lattice_span_enqueue(cw_lattice_s *l) {
     CW_LAUNCHED();
     k_span_finish<<<(nh + 127) / 128, 128, 0, stream()>>>(l->d_span, l->g.d_dims, nh);
     CW_LAUNCHED();
-    k_pass_plan<<<1, 1024, 0, stream()>>>(l->d_span, nh, l->period, l->d_vplan);
+    k_pass_plan<<<1, 1024, 0, stream()>>>(l->d_span, nh, l->period, l->useg, l->d_vplan);
     CW_LAUNCHED();
     return CW_OK;
 }
@@ -1023,9 +1535,11 @@ int lattice_sweep(cw_lattice_s *l) {
 // One sweep of every colour (a whole Monte Carlo step with one sub-sweep);
 // the device's step counter advances by one per sub-sweep.
 int lattice_subsweep(cw_lattice_s *l) {
+    const int rc = l->ensure_scratch();
+    if (rc != CW_OK) return rc;
     LatDevice d = dev_of(l);
     k_colour_order<<<1, 128, 0, stream()>>>(l->d_keys, l->g.nh, l->ncol, d.mcs, d.mcs + 1, d.perm,
-                                            l->pctl + CTL_KEYS);
+                                            l->pctl + CTL_KEYS, l->pctl + CTL_WORDS);
     CW_LAUNCHED();
     LatView v = lat_view(l);
     Tables t = lat_tables(l);
@@ -1033,7 +1547,12 @@ int lattice_subsweep(cw_lattice_s *l) {
     S.claim[0] = l->claim;
     S.claim[1] = l->claim + l->ncells;
     S.list = (Attempt *)l->plist;
+    S.mail = l->pmail;
     S.idx = l->pidx;
+    S.link = l->pidx + l->plist_cap;
+    S.count = l->pcount;
+    S.chain = l->plist_cap < (1ll << 30) ? l->pchain : nullptr;
+    S.useg = l->useg;
     S.seg = (uint32_t)l->pass_seg;
     S.ncells = l->ncells;
     S.ctl = l->pctl;
@@ -1044,21 +1563,19 @@ int lattice_subsweep(cw_lattice_s *l) {
     S.max_rounds = tf.max_rounds > 0 ? tf.max_rounds : MAX_ROUNDS;
     int nh = (int)l->g.nh;
     const uint32_t *cur = d.mcs + 1;
-    for (int q = 0; q < l->ncol; ++q) {
-        void *args[] = {&v, &t, &nh, &d.perm, &q, (void *)&cur, &S};
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.gridDim = dim3((unsigned)l->pass_blocks);
-        cfg.blockDim = dim3(PT);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = stream();
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        CW_CUDA(cudaLaunchKernelExC(&cfg, (const void *)k_cpm_pass, args));
-        count_launch(1);
-    }
+    void *args[] = {&v, &t, &nh, &d.perm, (void *)&cur, &S};
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.gridDim = dim3((unsigned)l->pass_blocks);
+    cfg.blockDim = dim3(PT);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = stream();
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CW_CUDA(cudaLaunchKernelExC(&cfg, (const void *)k_cpm_sweep, args));
+    count_launch(1);
     return CW_OK;
 }
 
@@ -1068,10 +1585,11 @@ int lattice_pass_error(cw_lattice_s *l) {
     uint32_t e = 0;
     CW_CUDA(cudaMemcpy(&e, l->pctl + CTL_ERR, sizeof e, cudaMemcpyDeviceToHost));
     if (!e) return CW_OK;
-    // a pass that gave up left its counts, the barrier's arrivals and its
-    // claims behind: all start again from zero
+    // a pass that gave up left the barrier's words, its claims and its cells'
+    // lists behind: all start again from zero
     CW_CUDA(cudaMemset(l->pctl, 0, sizeof(uint32_t) * CTL_KEYS));
-    CW_CUDA(cudaMemset(l->claim, 0, sizeof(unsigned long long) * 2 * (size_t)l->ncells));
+    if (l->claim) CW_CUDA(cudaMemset(l->claim, 0, sizeof(unsigned long long) * 2 * (size_t)l->ncells));
+    if (l->pcount) CW_CUDA(cudaMemset(l->pcount, 0, sizeof(uint32_t) * (size_t)l->ncells));
     return e == 1 ? fail(CW_ERR_TIMEOUT, "a sublattice pass waited too long at a grid barrier")
                   : fail(CW_ERR_SIMULATION, "a sublattice pass needed more rounds than allowed");
 }
@@ -1137,7 +1655,8 @@ int cw_lattice_destroy(cw_lattice l) {
     CW_SCOPE(l);
     dfree(l->grid); dfree(l->type); dfree(l->volume); dfree(l->target); dfree(l->lambda); dfree(l->vsnap);
     dfree(l->surface); dfree(l->ssnap); dfree(l->tsurf); dfree(l->lsurf); dfree(l->d_cell_off); dfree(l->d_keys);
-    dfree(l->d_flag); dfree(l->claim); dfree(l->plist); dfree(l->pidx); dfree(l->d_vplan); dfree(l->pctl); dfree(l->d_used);
+    dfree(l->d_flag); dfree(l->claim); dfree(l->plist); dfree(l->pidx);
+    dfree(l->pmail); dfree(l->pcount); dfree(l->pchain); dfree(l->d_vplan); dfree(l->pctl); dfree(l->d_used);
     dfree(l->bath_label); dfree(l->bath_mark); dfree(l->stage); dfree(l->d_bad); dfree(l->d_span);
     l->div.release();
     l->site_plan.release();
