@@ -89,6 +89,34 @@ const TestFaults &test_faults();
         if (e_ != cudaSuccess) return ::cw::cuda_fail(e_, "kernel launch"); \
     } while (0)
 
+// ------------------------------------------------------------------ launches that overlap their beginnings
+// Programmatic dependent launch: a kernel launched with `overlap` begins as
+// soon as every block of the one before it in the stream has passed
+// let_next_begin, and sets itself up beside that one's last blocks; what the
+// one before wrote it reads after await_previous, which waits until that one
+// is over.  Every block passes await_previous before let_next_begin, so no more
+// than two launches are ever under way and all before them have ended.
+// Overlap only behind a kernel of the same kind: what the beginning reads must
+// have been written before that kernel's own launch.
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_after(bool overlap, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                         A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ------------------------------------------------------------------ device memory
 template <class T>
 int dalloc(T **p, size_t n) {

@@ -17,13 +17,26 @@
 // that border.  The correction crosses HBM once per DEPTH half-sweeps.
 //
 // The wide kernel (rows 16-byte aligned in every history, the campaign's
-// case): 128 x 64 windows, a warp per 8 rows, a lane per 4 consecutive
+// case): 128 x 64 windows, a warp per 16 rows, a lane per 4 consecutive
 // columns held as float4 registers (two pixels of each colour per row, one
-// warp shuffle per two updates).  Blocks are persistent, two per SM; while a
-// block sweeps one window in registers, the TMA engine brings the next
-// window's correction and coefficients into shared memory (one mbarrier,
-// 96 KB), so the HBM reads overlap the sweeps.  Windows start at x = k (128 -
-// 2 DEPTH), a multiple of 4 floats as TMA needs, and at y = k (64 - 2 DEPTH).
+// warp shuffle per two updates; 244 registers a thread, no spills).  Blocks
+// are persistent, two per SM; while a block sweeps one window in registers,
+// the TMA engine brings the next window's correction and coefficients into
+// shared memory (one mbarrier, 96 KB), so the HBM reads overlap the sweeps.
+// Windows start at x = k (128 - 2 DEPTH), a multiple of 4 floats as TMA needs,
+// and at y = k (64 - 2 DEPTH).
+//
+// What bounds it: at depth 8 the four sweeps' own instructions, not HBM (54 us
+// of traffic a launch on 64 histories of up to 1024^2, 64.6 Mpx), and next to
+// them what a window costs besides: the published rows, the barriers, the
+// look-up.  Sixteen rows a warp instead of eight halve the published rows and
+// the warps at a barrier per update and let two half-sweeps run unrolled;
+// listing 32 windows at a time takes three dependent reads off every window;
+// launches that overlap their beginnings take the empty tail of one and the
+// set-up of the next off the line.  Together, depth 8, a launch: 92.3 -> 66.4 us
+// on that field (62.7 in 128 x 128 windows), 22.9 -> 16.2 on one 2048^2 plane,
+// 10.5 -> 7.6 on 1024^2.  Tried and slower: waiting for the neighbours' rows a
+// half-sweep later by an mbarrier of arrivals (76.3 against 70.3 without it).
 //
 // The narrow kernel (any width): 64 x 64 windows, a lane per column pair,
 // plain loads, one window per block.
@@ -147,59 +160,60 @@ __global__ void __launch_bounds__(32 * WARPS) k_sor32_tb(const float *__restrict
 // ------------------------------------------------------------------ wide windows (TMA)
 
 constexpr int WX = 128;              // window columns
-constexpr int WROWS = 8;             // rows per warp; a window has 8 rows per warp of its block
-// Two shapes: 8 warps (128 x 64 windows, two blocks per SM) or 16 warps
-// (128 x 128 windows, one block per SM: a smaller share of the window is
-// halo, 1.31 pixels swept per interior pixel at depth 8 against 1.52).
+constexpr int WROWS = 16;            // rows per warp; a window has WROWS rows per warp of its block
+// Two shapes: 128 x 64 windows, two blocks per SM, or 128 x 128 windows, one
+// block per SM: a smaller share of the window is halo, 1.31 pixels swept per
+// interior pixel at depth 8 against 1.52.
 constexpr size_t wide_smem(int warps) {
-    return (size_t)3 * WX * WROWS * warps * sizeof(float) + (size_t)2 * warps * 2 * (WX / 4) * sizeof(float4);
+    return (size_t)3 * WX * WROWS * warps * sizeof(float) + (size_t)2 * (warps + 2) * 2 * (WX / 4) * sizeof(float4);
 }
 __device__ int g_wide_wait_failed;
 
-// The first window at or after `t`, in steps of `step`, whose history is not settled.
-__device__ __forceinline__ int next_live(int t, int ntiles, int step, const int4 *tiles, const int32_t *done,
-                                         int stride) {
-    while (t < ntiles && done[(int64_t)tiles[t].x * stride]) t += step;
-    return t;
-}
-
-// One half-sweep of colour C over rows J0..J1-1 of a lane's 8 rows x 4
-// columns.  Column c of row j has colour (c + j) mod 2 (windows start at even
-// x and y): colour C takes columns 0 and 2 of the rows with C + j even, 1 and
-// 3 of the others.  Every update reads only pixels of the other colour, which
-// this half-sweep does not change.
-template <int C, int J0, int J1>
+// One half-sweep of colour C over a lane's WROWS rows x 4 columns.  Column c
+// of row j has colour (c + j) mod 2 (windows start at even x and y): colour C
+// takes columns 0 and 2 of the rows with C + j even, 1 and 3 of the others.
+// Every update reads only pixels of the other colour, which this half-sweep
+// does not change.
+template <int C>
 __device__ __forceinline__ void rows4(float4 (&d)[WROWS], const float4 (&a)[WROWS], const float4 (&b)[WROWS],
                                       const float4 ab, const float4 be, float lm, float rm, float omc) {
-    // the across-lane neighbours first: they are of the other colour, which
-    // this half-sweep does not change, and their latency then overlaps
-    float nb[WROWS];
 #pragma unroll
-    for (int j = J0; j < J1; ++j)
-        nb[j] = ((C + j) & 1) == 0 ? __shfl_up_sync(0xffffffffu, d[j].w, 1) : __shfl_down_sync(0xffffffffu, d[j].x, 1);
+    for (int j0 = 0; j0 < WROWS; j0 += 8) {
+        // eight rows' across-lane neighbours first: they are of the other
+        // colour, and their latency then overlaps
+        float nb[8];
 #pragma unroll
-    for (int j = J0; j < J1; ++j) {
-        const float4 up = j > 0 ? d[j - 1] : ab, dn = j < WROWS - 1 ? d[j + 1] : be;
-        if (((C + j) & 1) == 0) {
-            const float left = nb[j];
-            const float s0 = fmaf(lm, left, d[j].y) + (up.x + dn.x);
-            const float s2 = (d[j].y + d[j].w) + (up.z + dn.z);
-            d[j].x = fmaf(a[j].x, s0, fmaf(omc, d[j].x, b[j].x));
-            d[j].z = fmaf(a[j].z, s2, fmaf(omc, d[j].z, b[j].z));
-        } else {
-            const float right = nb[j];
-            const float s1 = (d[j].x + d[j].z) + (up.y + dn.y);
-            const float s3 = fmaf(rm, right, d[j].z) + (up.w + dn.w);
-            d[j].y = fmaf(a[j].y, s1, fmaf(omc, d[j].y, b[j].y));
-            d[j].w = fmaf(a[j].w, s3, fmaf(omc, d[j].w, b[j].w));
+        for (int q = 0; q < 8; ++q) {
+            const int j = j0 + q;
+            nb[q] = ((C + j) & 1) == 0 ? __shfl_up_sync(0xffffffffu, d[j].w, 1)
+                                       : __shfl_down_sync(0xffffffffu, d[j].x, 1);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int j = j0 + q;
+            const float4 up = j > 0 ? d[j > 0 ? j - 1 : 0] : ab, dn = j < WROWS - 1 ? d[j < WROWS - 1 ? j + 1 : j] : be;
+            if (((C + j) & 1) == 0) {
+                const float s0 = fmaf(lm, nb[q], d[j].y) + (up.x + dn.x);
+                const float s2 = (d[j].y + d[j].w) + (up.z + dn.z);
+                d[j].x = fmaf(a[j].x, s0, fmaf(omc, d[j].x, b[j].x));
+                d[j].z = fmaf(a[j].z, s2, fmaf(omc, d[j].z, b[j].z));
+            } else {
+                const float s1 = (d[j].x + d[j].z) + (up.y + dn.y);
+                const float s3 = fmaf(rm, nb[q], d[j].z) + (up.w + dn.w);
+                d[j].y = fmaf(a[j].y, s1, fmaf(omc, d[j].y, b[j].y));
+                d[j].w = fmaf(a[j].w, s3, fmaf(omc, d[j].w, b[j].w));
+            }
         }
     }
 }
 
-// What a block needs of a window, staged in shared memory by thread 0 one
-// window ahead, so that no thread waits on a global load at a window's start.
+// What a block needs of a window.  A block's next 32 are looked up at once, a
+// lane each, and the live ones listed in shared memory: looking up one at each
+// window's turn (its record, whether its history has settled, then the
+// history's scalars: three reads in turn by one thread, the block waiting) took
+// a fifth of a window's time.
 struct WideTile {
-    int4 tl;      // (history, x0, y0, 0); history < 0: no window left
+    int4 tl;      // (history, x0, y0, 0)
     int4 dm;      // the history's dimensions
     int64_t off;  // its first pixel
     float omc;    // 1 - omega
@@ -211,70 +225,96 @@ struct WideTile {
 // it is not read.  apply_c: the last launch of a solve adds its correction to
 // the FP64 field (floored at zero when `floor`) instead of writing it to dst.
 template <int DEPTH, int WWARPS>
-__global__ void __launch_bounds__(32 * WWARPS, WWARPS == 8 ? 2 : 1)
+__global__ void __launch_bounds__(32 * WWARPS, WWARPS * WROWS == 64 ? 2 : 1)
     k_sor32_wide(const CUtensorMap *__restrict__ maps, int src_map, float *__restrict__ dst,
                  const int4 *__restrict__ tiles, int ntiles, const int4 *__restrict__ dims,
                  const int64_t *__restrict__ off, const float *__restrict__ omega, const int32_t *done,
-                 int done_stride, int nhalf, int start_colour, int zero_start, double *__restrict__ apply_c,
+                 int done_stride, int nhalf, int zero_start, double *__restrict__ apply_c,
                  int floor, unsigned long long wait_ns, int skip_copies, unsigned long long *corr, int corr_stride) {
     constexpr int WY = WROWS * WWARPS;  // window rows
     constexpr int STAGE = WX * WY;      // floats per array of the staged window
     extern __shared__ __align__(128) float smem[];
     const float4 *sd = (const float4 *)smem, *sb = (const float4 *)(smem + STAGE),
                  *sa = (const float4 *)(smem + 2 * STAGE);
-    float4 *edge = (float4 *)(smem + 3 * STAGE);  // [buffer][warp][0 top, 1 bottom][lane]
+    // [buffer][warp + 1][0 top, 1 bottom][lane], a warp of zeros at either end
+    float4 *edge = (float4 *)(smem + 3 * STAGE);
+    constexpr int EBUF_ALL = (WWARPS + 2) * 64;
     __shared__ __align__(8) uint64_t bar_word;
-    __shared__ WideTile s_info[2];
-    __shared__ int s_fail;
+    __shared__ WideTile s_tile[32];
+    __shared__ int s_tiles, s_from, s_fail;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t bar = sh_addr(&bar_word);
     const uint32_t boxes = zero_start ? 2u : 3u;
-    // thread 0: find the next live window at or after t, stage its scalars
-    // in s_info[slot] and start its copies
-    auto stage_next = [&](int t, int slot) {
-        t = next_live(t, ntiles, gridDim.x, tiles, done, done_stride);
-        WideTile w;
-        w.tl = make_int4(-1, 0, 0, 0);
-        if (t < ntiles) {
-            w.tl = tiles[t];
-            w.tl.w = t;
-            w.dm = dims[w.tl.x];
-            w.off = off[w.tl.x];
-            w.omc = 1.f - omega[w.tl.x];
-            const CUtensorMap *m = maps + 4 * w.tl.x;
-            mbar_expect_tx(bar, (uint32_t)(boxes * STAGE * sizeof(float)));
-            // skip_copies (a failure test): the bytes announced never come,
-            // and the wait below runs out
-            if (!skip_copies) {
-                if (!zero_start) tma_load_2d(smem, m + src_map, bar, w.tl.y, w.tl.z);
-                tma_load_2d(smem + STAGE, m + 2, bar, w.tl.y, w.tl.z);
-                tma_load_2d(smem + 2 * STAGE, m + 3, bar, w.tl.y, w.tl.z);
+    // warp 0: the live ones of this block's windows from `from` on, until there
+    // is one or no window is left
+    auto look_up = [&](int from) {
+        unsigned live = 0;
+        for (; live == 0u && from < ntiles; from += 32 * gridDim.x) {
+            const int t = from + lane * gridDim.x;
+            int4 tl = make_int4(0, 0, 0, 0);
+            bool on = t < ntiles;
+            if (on) {
+                tl = tiles[t];
+                on = !done[(int64_t)tl.x * done_stride];
+            }
+            live = __ballot_sync(0xffffffffu, on);
+            if (on) {
+                WideTile &w = s_tile[__popc(live & ((1u << lane) - 1u))];
+                w.tl = tl;
+                w.dm = dims[tl.x];
+                w.off = off[tl.x];
+                w.omc = 1.f - omega[tl.x];
             }
         }
-        s_info[slot] = w;
+        if (lane == 0) {
+            s_tiles = __popc(live);
+            s_from = from;
+        }
+        __syncwarp();
     };
+    // thread 0: start the copies of a listed window
+    auto copy = [&](const int4 tl) {
+        const CUtensorMap *m = maps + 4 * tl.x;
+        mbar_expect_tx(bar, (uint32_t)(boxes * STAGE * sizeof(float)));
+        // skip_copies (a failure test): the bytes announced never come,
+        // and the wait below runs out
+        if (!skip_copies) {
+            if (!zero_start) tma_load_2d(smem, m + src_map, bar, tl.y, tl.z);
+            tma_load_2d(smem + STAGE, m + 2, bar, tl.y, tl.z);
+            tma_load_2d(smem + 2 * STAGE, m + 3, bar, tl.y, tl.z);
+        }
+    };
+    for (int i = threadIdx.x; i < 2 * EBUF_ALL; i += 32 * WWARPS) edge[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         mbar_init_fence();
         s_fail = 0;
-        stage_next(blockIdx.x, 0);
     }
+    // (a launch that overlaps another follows a sweep, which does not write
+    // what the look-up reads; the buffers wait for that sweep's end)
+    if (warp == 0) look_up(blockIdx.x);
+    await_previous();
+    let_next_begin();
+    if (threadIdx.x == 0 && s_tiles > 0) copy(s_tile[0].tl);
     __syncthreads();
     uint32_t parity = 0;
     const float lm = lane == 0 ? 0.f : 1.f, rm = lane == 31 ? 0.f : 1.f;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto ed = [&](int buf, int w, int side) -> float4 & { return edge[((buf * WWARPS + w) * 2 + side) * 32 + lane]; };
-    for (int slot = 0;; slot ^= 1) {
-        const WideTile info = s_info[slot];
-        if (info.tl.x < 0) break;
+    // this lane's published top row in either buffer; the bottom row 32 behind,
+    // the warps above and below 64 before and behind
+    constexpr int EBUF = EBUF_ALL;
+    float4 *const my_edge = edge + (warp + 1) * 64 + lane;
+    for (int k = 0; k < s_tiles;) {
+        const WideTile info = s_tile[k];
+        const bool relist = k + 1 == s_tiles;  // read before warp 0 lists anew
         if (!mbar_wait_bounded(bar, parity, wait_ns)) s_fail = 1;
         float4 d[WROWS], a[WROWS], b[WROWS];
 #pragma unroll
         for (int j = 0; j < WROWS; ++j) {
-            const int k = (warp * WROWS + j) * 32 + lane;
-            d[j] = zero_start ? z4 : sd[k];
-            b[j] = sb[k];
-            a[j] = sa[k];
+            const int q = (warp * WROWS + j) * 32 + lane;
+            d[j] = zero_start ? z4 : sd[q];
+            b[j] = sb[q];
+            a[j] = sa[q];
         }
         __syncthreads();  // the stage is read: free for the next window
         if (s_fail) {
@@ -286,27 +326,31 @@ __global__ void __launch_bounds__(32 * WWARPS, WWARPS == 8 ? 2 : 1)
             return;
         }
         parity ^= 1u;
-        if (threadIdx.x == 0) {
-            // the generic-proxy reads of the stage before the async-proxy writes
-            fence_proxy_async_shared();
-            stage_next(info.tl.w + gridDim.x, slot ^ 1);
+        // the next window, from the list or a new one
+        k = relist ? 0 : k + 1;
+        if (warp == 0) {
+            if (relist) look_up(s_from);
+            if (lane == 0 && s_tiles > 0) {
+                // the generic-proxy reads of the stage before the async-proxy writes
+                fence_proxy_async_shared();
+                copy(s_tile[k].tl);
+            }
         }
         const float omc = info.omc;
-        ed(0, warp, 0) = d[0];
-        ed(0, warp, 1) = d[WROWS - 1];
+        my_edge[0] = d[0];
+        my_edge[32] = d[WROWS - 1];
         __syncthreads();
-        for (int s = 0; s < nhalf; ++s) {
-            const int buf = s & 1;
-            const float4 ab = warp > 0 ? ed(buf, warp - 1, 1) : z4;
-            const float4 be = warp < WWARPS - 1 ? ed(buf, warp + 1, 0) : z4;
-            if (((start_colour + s) & 1) == 0)
-                rows4<0, 0, WROWS>(d, a, b, ab, be, lm, rm, omc);
-            else
-                rows4<1, 0, WROWS>(d, a, b, ab, be, lm, rm, omc);
-            if (s + 1 < nhalf) {
-                // the other buffer was last read before the previous barrier
-                ed(buf ^ 1, warp, 0) = d[0];
-                ed(buf ^ 1, warp, 1) = d[WROWS - 1];
+        // (a launch's half-sweeps are even in number and begin with the red: two a turn)
+        for (int s = 0; s < nhalf; s += 2) {
+            rows4<0>(d, a, b, my_edge[-32], my_edge[64], lm, rm, omc);
+            // the other buffer was last read before the previous barrier
+            my_edge[EBUF] = d[0];
+            my_edge[EBUF + 32] = d[WROWS - 1];
+            __syncthreads();
+            rows4<1>(d, a, b, my_edge[EBUF - 32], my_edge[EBUF + 64], lm, rm, omc);
+            if (s + 2 < nhalf) {
+                my_edge[0] = d[0];
+                my_edge[32] = d[WROWS - 1];
                 __syncthreads();
             }
         }
@@ -369,6 +413,21 @@ __global__ void __launch_bounds__(32 * WWARPS, WWARPS == 8 ? 2 : 1)
                     unsigned long long *mine = corr + (int64_t)info.tl.x * corr_stride;
                     if (most > 0.f) atomicMax(mine, (unsigned long long)__double_as_longlong((double)most));
                     if (top > 0.0) atomicMax(mine + 1, (unsigned long long)__double_as_longlong(top));
+                }
+            }
+        } else if (j0 <= 0 && j1 >= WROWS) {
+            // every row of the warp (most warps)
+            float *row = dst + first;
+            if (full) {
+#pragma unroll
+                for (int j = 0; j < WROWS; ++j, row += dm.x) *(float4 *)row = d[j];
+            } else if (part) {
+#pragma unroll
+                for (int j = 0; j < WROWS; ++j, row += dm.x) {
+                    if (gx >= ix0 && gx < ix1) row[0] = d[j].x;
+                    if (gx + 1 >= ix0 && gx + 1 < ix1) row[1] = d[j].y;
+                    if (gx + 2 >= ix0 && gx + 2 < ix1) row[2] = d[j].z;
+                    if (gx + 3 >= ix0 && gx + 3 < ix1) row[3] = d[j].w;
                 }
             }
         } else {
@@ -652,7 +711,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
 typedef void (*TbKernel)(const float *, float *, const float *, const float *, const int4 *, const int64_t *,
                          const int32_t *, int, const float *, const int32_t *, int, int, int);
 typedef void (*WideKernel)(const CUtensorMap *, int, float *, const int4 *, int, const int4 *, const int64_t *,
-                           const float *, const int32_t *, int, int, int, int, double *, int, unsigned long long,
+                           const float *, const int32_t *, int, int, int, double *, int, unsigned long long,
                            int, unsigned long long *, int);
 
 TbKernel tb_kernel(int depth) {
@@ -687,7 +746,9 @@ VolKernel vol_kernel(int vy, int align, bool full) {
                     : (full ? vol_kernel_of<16, true>(align) : vol_kernel_of<16, false>(align));
 }
 
-WideKernel wide_kernel(int depth, int warps) { return warps == 16 ? wide_kernel_of<16>(depth) : wide_kernel_of<8>(depth); }
+WideKernel wide_kernel(int depth, int warps) {
+    return warps * WROWS == 128 ? wide_kernel_of<128 / WROWS>(depth) : wide_kernel_of<64 / WROWS>(depth);
+}
 
 // Window starts along one axis of n pixels for windows of `win` with a halo
 // of `depth`: the first at 0, then every win - 2 depth until one reaches n.
@@ -837,7 +898,7 @@ int Sor32::init(cw_field_s *f, int d, const std::vector<double> &om, int window)
     if (blocked) {
         wide = false;
         if ((window == CW_WINDOW_AUTO || window == CW_WINDOW_TALL) &&
-            (rc = wide_init(*this, f, window == CW_WINDOW_TALL ? 16 : 8)) != CW_OK)
+            (rc = wide_init(*this, f, window == CW_WINDOW_TALL ? 128 / WROWS : 64 / WROWS)) != CW_OK)
             return rc;
         if (!wide) {
             const int in = WIN - 2 * depth;
@@ -909,11 +970,12 @@ int Sor32::sweeps(cw_field_s *f, int n, const int32_t *done, int done_stride, fl
             // the first launch starts from zero without reading it; with
             // `apply` the last adds its correction to the field
             const bool last = remaining == dd;
-            wide_kernel(depth, wwarps)<<<wgrid, 32 * wwarps, wide_smem(wwarps), stream()>>>(
-                (const CUtensorMap *)maps, a == f->d32a ? 0 : 1, b, wtiles, nwtiles, f->g.d_dims, f->g.d_off, omega,
-                done, done_stride, dd, done_half & 1, done_half == 0 ? 1 : 0, apply && last ? f->c : nullptr,
-                f->floor ? 1 : 0, test_faults().wait_ns ? test_faults().wait_ns : TMA_WAIT_NS, test_faults().skip_tma,
-                apply && last ? corr : nullptr, corr_stride);
+            CW_CUDA(launch_after(done_half > 0, wide_kernel(depth, wwarps), wgrid, 32 * wwarps, wide_smem(wwarps),
+                                 stream(), (const CUtensorMap *)maps, a == f->d32a ? 0 : 1, b, wtiles, nwtiles, f->g.d_dims,
+                                 f->g.d_off, omega, done, done_stride, dd, done_half == 0 ? 1 : 0,
+                                 apply && last ? f->c : nullptr, f->floor ? 1 : 0,
+                                 test_faults().wait_ns ? test_faults().wait_ns : TMA_WAIT_NS, test_faults().skip_tma,
+                                 apply && last ? corr : nullptr, corr_stride));
         } else {
             tb_kernel(depth)<<<tiles.nblocks, 32 * WARPS, 0, stream()>>>(a, b, f->r32, f->inv32, f->g.d_dims,
                                                                          f->g.d_off, tiles.d_blk, f->g.nh, omega,

@@ -1024,9 +1024,12 @@ static int tune_depth(cw_sim_s *s) {
     // volumes march tiles along z at four half-sweeps a launch (two take twice
     // the time a sweep at every size)
     const bool volume = s->d[0] > 1;
-    for (int w : {CW_WINDOW_AUTO, CW_WINDOW_64})
+    // the tall windows pay on many large planes (62.7 us a launch against 66.4
+    // on 64.6 Mpx) and only at the full depth, where the halo is widest
+    for (int w : {CW_WINDOW_AUTO, CW_WINDOW_TALL, CW_WINDOW_64})
         for (int d : {4, 6, 8}) {
             if (volume && d != 4) continue;
+            if (w == CW_WINDOW_TALL && (volume || d != 8)) continue;
             float ms = 0.f;
             int64_t launches = 0;
             int rc = cw_field_time_inner(s->o2, 8, d, w, 1.9, &ms, &launches);
