@@ -39,7 +39,8 @@
 // half-sweep later by an mbarrier of arrivals (76.3 against 70.3 without it).
 //
 // The narrow kernel (any width): 64 x 64 windows, a lane per column pair,
-// plain loads, one window per block.
+// plain loads, one window per block.  Its launches, and the volumes', overlap
+// too: 2.56 -> 2.23 ms the relax of a 1023 x 769 sheet.
 //
 // Between warps, each warp publishes its top and bottom rows in shared memory
 // after every half-sweep (double-buffered, so one barrier per half-sweep).
@@ -98,7 +99,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_sor32_tb(const float *__restrict
     if (threadIdx.x == 0) s_h = plan_history(blk, nh, blockIdx.x);
     __syncthreads();
     const int h = s_h;
-    if (done[(int64_t)h * done_stride]) return;
+    const bool idle = done[(int64_t)h * done_stride];
+    await_previous();
+    let_next_begin();
+    if (idle) return;
     const int4 dm = dims[h];
     const int ntx = (dm.x + IN - 1) / IN;
     const int t = blockIdx.x - blk[h];
@@ -552,7 +556,10 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
     constexpr int EWARP = 64, ESTAGE = (NW + 2) * EWARP, EBUF = (D - 1) * ESTAGE;
     const int4 tl = tiles[blockIdx.x];
     const int h = tl.x;
-    if (done[(int64_t)h * done_stride]) return;
+    const bool idle = done[(int64_t)h * done_stride];
+    await_previous();
+    let_next_begin();
+    if (idle) return;
     const int4 dm = dims[h];
     const int x0 = tl.y, y0 = tl.z, z0 = tl.w;
     const int z1 = min(z0 + vz, dm.z);
@@ -937,9 +944,10 @@ int Sor32::sweeps(cw_field_s *f, int n, const int32_t *done, int done_stride, fl
             // with `apply` the last launch adds its correction to the field
             const bool last = remaining == dd;
             const bool full = dd == VD && done_half > 0 && !(apply && last);
-            vol_kernel(vy, valign, full)<<<nvtiles, 16 * vy, vol_smem(vy / 2), stream()>>>(
-                a, b, f->r32, f->inv32, f->g.d_dims, f->g.d_off, vtiles, vz, omega, done, done_stride, dd,
-                done_half == 0 ? 1 : 0, apply && last ? f->c : nullptr, f->floor ? 1 : 0);
+            CW_CUDA(launch_after(done_half > 0, vol_kernel(vy, valign, full), nvtiles, 16 * vy, vol_smem(vy / 2),
+                                 stream(), a, b, f->r32, f->inv32, f->g.d_dims, f->g.d_off, vtiles, vz, omega, done,
+                                 done_stride, dd, done_half == 0 ? 1 : 0, apply && last ? f->c : nullptr,
+                                 f->floor ? 1 : 0));
             CW_LAUNCHED();
             remaining -= dd;
             done_half += dd;
@@ -977,9 +985,9 @@ int Sor32::sweeps(cw_field_s *f, int n, const int32_t *done, int done_stride, fl
                                  test_faults().wait_ns ? test_faults().wait_ns : TMA_WAIT_NS, test_faults().skip_tma,
                                  apply && last ? corr : nullptr, corr_stride));
         } else {
-            tb_kernel(depth)<<<tiles.nblocks, 32 * WARPS, 0, stream()>>>(a, b, f->r32, f->inv32, f->g.d_dims,
-                                                                         f->g.d_off, tiles.d_blk, f->g.nh, omega,
-                                                                         done, done_stride, dd, done_half & 1);
+            CW_CUDA(launch_after(done_half > 0, tb_kernel(depth), tiles.nblocks, 32 * WARPS, 0, stream(), a, b,
+                                 f->r32, f->inv32, f->g.d_dims, f->g.d_off, tiles.d_blk, f->g.nh, omega, done,
+                                 done_stride, dd, done_half & 1));
         }
         CW_LAUNCHED();
         remaining -= dd;
