@@ -2,11 +2,8 @@
 //
 // Compilation (from_spec, network.rs:283-445) runs once on the host: names
 // are resolved to indices, terms laid out per node in file order.  The RK4
-// step (rk4, network.rs:777-799) runs one cell per thread when there are many
-// cells (k_rk4: every cell of a launch walks the same term list, so a warp
-// never diverges; state, midpoint, stage slope and accumulated slope in
-// shared memory laid out [node][thread]), and a lane per node when there are
-// few (k_rk4_lanes: 8, 16 or 32 lanes a cell, source nodes by shuffle).
+// step (rk4, network.rs:777-799) runs a lane per cell, a cell's nodes dealt to
+// the warps of its block (k_rk4).
 // Built without fused multiply-add: the sums round as the reference's do.
 #include <algorithm>
 #include <cmath>
@@ -25,160 +22,111 @@ const char *INPUTS[6] = {"oxygen", "egf", "crowding", "stress", "waste", "necrot
 
 constexpr int MAXS = 32;
 
-constexpr int RT = 64;  // cells per block of the one-cell-per-thread kernels
+// RK4 with a block per 32 cells (rk4, derivatives and term_rate,
+// network.rs:686-799): a lane per cell, the nodes dealt to the block's G warps.
+// Every lane of a warp is at the same node, so a warp never diverges by kind of
+// term, and a cell's evaluations run G nodes at a time.  A node's terms are
+// added in file order by one thread: the reference's operations in its order.
+// A stage's values live in shared memory, [node][lane], in two buffers turn by
+// turn, so a stage is one barrier; the six inputs stand clamped behind them.
+// nets null: every cell under N, its terms in shared memory; else cell c under
+// nets[clone[c]], its terms read from global memory (a network's tables are a
+// few KB: they stay in L1).
+// state: node i of cell c at state[i * node_stride + c * cell_stride], input q
+// at inputs[q * in_stride + c * in_cell]; alive (optional): cells whose entry is
+// zero are left as they are.
+//
+// What bounds it: with few cells the chain of a node's terms, each with a
+// division; with many the FP64 instructions themselves.  A thread per cell (and
+// for few cells a lane per node, whose warps diverged by kind of term) took, 10
+// steps of 8 nodes: 300 cells 111 -> 47 us, 1,260 cells 115 -> 51, 16,000 cells
+// 163 -> 70; 8 steps: 137,000 cells 452 -> 334, 40,000 cells of 16 nodes 693 ->
+// 366, of 32 nodes 5,959 -> 1,177.  Five blocks of 8 warps an SM (48 registers a
+// thread, a few of the power spilled; four blocks spill next to none and take
+// 445 us where five take 366).
+constexpr int RC = 32;  // cells per block
+enum { SQUARE = 2, POWER = 3 };  // a term's Hill flag in shared memory
 
-// One cell's `substeps` RK4 steps (rk4, network.rs:777-799) on its column of
-// the block's shared arrays (xs: state, ms: midpoint, ks: stage slope, as:
-// accumulated slope, each [node][RT]), under the terms at sterm/spar/sptr.
-__device__ __forceinline__ void rk4_cell(const NetDev &N, const int4 *sterm, const double4 *spar, const int32_t *sptr,
-                                         double *xs, double *ms, double *ks, double *as, const double *in, double dt,
-                                         int substeps) {
-    const int S = N.S;
-    for (int sub = 0; sub < substeps; ++sub) {
-        // k1 at x
-        derivatives(N, sterm, spar, sptr, xs, in, ks, RT);
-        for (int i = 0; i < S; ++i) {
-            double k1 = ks[i * RT];
-            as[i * RT] = k1;
-            ms[i * RT] = xs[i * RT] + 0.5 * dt * k1;
-        }
-        // k2 at x + dt/2 k1, k3 at x + dt/2 k2, k4 at x + dt k3
-        for (int stage = 1; stage < 4; ++stage) {
-            derivatives(N, sterm, spar, sptr, ms, in, ks, RT);
-            double step = stage < 2 ? 0.5 * dt : dt;
-            for (int i = 0; i < S; ++i) {
-                double kv = ks[i * RT];
-                if (stage < 3) {
-                    as[i * RT] = as[i * RT] + 2.0 * kv;
-                    ms[i * RT] = xs[i * RT] + step * kv;
-                } else {
-                    as[i * RT] = as[i * RT] + kv;
-                }
-            }
-        }
-        for (int i = 0; i < S; ++i) {
-            double delta = (dt / 6.0) * as[i * RT];
-            xs[i * RT] = fmin(fmax(xs[i * RT] + delta, 0.0), 1.0);
-        }
-    }
+size_t rk4_block(int S, int nterms) {
+    return sizeof(double) * (4 * S + 6) * RC + nterms * (sizeof(int4) + sizeof(double4)) + sizeof(int32_t) * (S + 1);
 }
 
-// state: [S][ncells] (node-major, coalesced); inputs: [6][ncells].
-// alive (optional): cells whose entry is zero are left as they are.
-__global__ void __launch_bounds__(RT) k_rk4(NetDev N, double *state, const double *inputs, int64_t ncells,
-                                            int64_t state_stride, int64_t input_stride, double dt, int substeps,
-                                            const uint8_t *alive) {
+template <int G, bool CLONES>
+__global__ void __launch_bounds__(32 * G, 40 / G)
+    k_rk4(NetDev N, const NetDev *nets, const int32_t *clone, int S, double *state, const double *inputs,
+          int64_t ncells, int64_t node_stride, int64_t cell_stride, int64_t in_stride, int64_t in_cell, double dt,
+          int substeps, const uint8_t *alive) {
     extern __shared__ double sm[];
-    const int S = N.S;
-    double *x = sm, *mid = sm + S * RT, *kk = sm + 2 * S * RT, *acc = sm + 3 * S * RT;
-    int4 *sterm = (int4 *)(sm + 4 * S * RT);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *const xs = sm + lane, *const as = xs + S * RC, *const m0 = as + S * RC, *const m1 = m0 + S * RC,
+                  *const in = m1 + S * RC;
+    int4 *sterm = (int4 *)(sm + (4 * S + 6) * RC);
     double4 *spar = (double4 *)(sterm + N.nterms);
     int32_t *sptr = (int32_t *)(spar + N.nterms);
-    for (int t = threadIdx.x; t < N.nterms; t += RT) { sterm[t] = N.term[t]; spar[t] = N.par[t]; }
-    for (int t = threadIdx.x; t <= S; t += RT) sptr[t] = N.node_ptr[t];
-    __syncthreads();
-    int64_t c = (int64_t)blockIdx.x * RT + threadIdx.x;
-    if (c >= ncells) return;
-    if (alive && !alive[c]) return;
-    const int tid = threadIdx.x;
-    double in[6];
-    for (int q = 0; q < 6; ++q) in[q] = inputs[q * input_stride + c];
-    double *xs = x + tid, *ms = mid + tid, *ks = kk + tid, *as = acc + tid;
-    for (int i = 0; i < S; ++i) xs[i * RT] = state[i * state_stride + c];
-    rk4_cell(N, sterm, spar, sptr, xs, ms, ks, as, in, dt, substeps);
-    for (int i = 0; i < S; ++i) state[i * state_stride + c] = xs[i * RT];
-}
-
-// The same for cells of many networks: cell c under nets[clone[c]], its
-// terms read from global memory (a network's tables are a few KB: they stay
-// in L1 across the block's cells of that network).
-// state: [S][state_stride], inputs: [6][input_stride]; alive (optional):
-// cells whose entry is zero are left as they are.
-__global__ void __launch_bounds__(RT) k_rk4_clones(const NetDev *nets, const int32_t *clone, int S, double *state,
-                                                   const double *inputs, int64_t ncells, int64_t state_stride,
-                                                   int64_t input_stride, double dt, int substeps,
-                                                   const uint8_t *alive) {
-    extern __shared__ double sm[];
-    double *x = sm, *mid = sm + S * RT, *kk = sm + 2 * S * RT, *acc = sm + 3 * S * RT;
-    int64_t c = (int64_t)blockIdx.x * RT + threadIdx.x;
-    if (c >= ncells) return;
-    if (alive && !alive[c]) return;
-    const NetDev N = nets[clone[c]];
-    const int tid = threadIdx.x;
-    double in[6];
-    for (int q = 0; q < 6; ++q) in[q] = inputs[q * input_stride + c];
-    double *xs = x + tid, *ms = mid + tid, *ks = kk + tid, *as = acc + tid;
-    for (int i = 0; i < S; ++i) xs[i * RT] = state[i * state_stride + c];
-    rk4_cell(N, N.term, N.par, N.node_ptr, xs, ms, ks, as, in, dt, substeps);
-    for (int i = 0; i < S; ++i) state[i * state_stride + c] = xs[i * RT];
-}
-
-// RK4 with a lane per node (derivatives and term_rate, network.rs:686-734;
-// rk4, 777-799): W lanes (W >= S, a power of two) hold one cell, lane i its
-// node i's state, midpoint and accumulated slope in registers; a node's
-// terms read their source nodes from the other lanes by shuffle.  A term
-// loop runs to the most terms any node of the warp has, every lane taking
-// part in each shuffle, and a lane adds its own node's terms in file order:
-// the same operations in the same order as one cell per thread, to the bit.
-// nets null: every cell under N; else cell c under nets[clone[c]].
-template <int W>
-__global__ void __launch_bounds__(128) k_rk4_lanes(NetDev N, const NetDev *nets, const int32_t *clone, double *state,
-                                                   const double *inputs, int64_t ncells, int64_t state_stride,
-                                                   int64_t input_stride, double dt, int substeps,
-                                                   const uint8_t *alive) {
-    const int lane = threadIdx.x & 31, node = lane % W, base = lane - node;
-    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / W;
-    const bool cell = c < ncells;
-    const NetDev M = (nets && cell) ? nets[clone[c]] : N;
-    const int S = M.S;
-    const bool live = cell && node < S && !(alive && !alive[c]);
-    int p0 = 0, cnt = 0;
-    if (cell && node < S) {
-        p0 = M.node_ptr[node];
-        cnt = M.node_ptr[node + 1] - p0;
+    const int64_t c = (int64_t)blockIdx.x * RC + lane;
+    const bool live = c < ncells && !(alive && !alive[c]);
+    const int4 *term = sterm;
+    const double4 *par = spar;
+    const int32_t *ptr = sptr;
+    if (CLONES) {
+        if (live) {
+            const NetDev M = nets[clone[c]];
+            term = M.term;
+            par = M.par;
+            ptr = M.node_ptr;
+        }
+    } else {
+        for (int t = threadIdx.x; t < N.nterms; t += 32 * G) {
+            int4 tm = N.term[t];
+            double4 p = N.par[t];
+            // what a Hill response takes from its term alone is worked out here
+            if (tm.z) {
+                tm.z = p.y == 2.0 ? SQUARE : POWER;
+                p.z = p.y == 2.0 ? p.z * p.z : pow(p.z, p.y);
+            }
+            sterm[t] = tm;
+            spar[t] = p;
+        }
+        for (int t = threadIdx.x; t <= S; t += 32 * G) sptr[t] = N.node_ptr[t];
     }
-    int tmax = cnt;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tmax = max(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-    double in[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) in[q] = cell ? inputs[q * input_stride + c] : 0.0;
-    double x = live ? state[node * state_stride + c] : 0.0;
-    // the rate of this lane's node at the cell's values v (one value a lane)
-    auto rate_of = [&](double own) -> double {
+    if (live) {
+        for (int i = warp; i < S; i += G) xs[i * RC] = state[i * node_stride + c * cell_stride];
+        // read, network.rs:670-680: oxygen and crowding in [0, 1], stress and
+        // the released not below zero
+        for (int q = warp; q < 6; q += G) {
+            double v = inputs[q * in_stride + c * in_cell];
+            if (q == 0 || q == 2) v = fmin(fmax(v, 0.0), 1.0);
+            else if (q >= 3) v = fmax(v, 0.0);
+            in[q * RC] = v;
+        }
+    }
+    __syncthreads();
+    // the rate of node i at the values v
+    auto rate_of = [&](const double *v, int i) -> double {
+        const double own = v[i * RC], rest = 1.0 - own;
         double rate = 0.0;
-        for (int t = 0; t < tmax; ++t) {
-            const bool has = t < cnt;
-            const int4 tm = has ? M.term[p0 + t] : make_int4(-1, -1, 0, 0);
-            const int from = (has && tm.y >= 0 && tm.y < S) ? base + tm.y : lane;
-            const double nodev = __shfl_sync(0xffffffffu, own, from);
-            if (!has) continue;
-            const double4 p = M.par[p0 + t];
-            // read, network.rs:670-680
-            double s = 0.0;
-            if (tm.y >= 0) s = nodev;
-            else switch (-1 - tm.y) {
-                case 0: s = fmin(fmax(in[0], 0.0), 1.0); break;
-                case 1: s = in[1]; break;
-                case 2: s = fmin(fmax(in[2], 0.0), 1.0); break;
-                case 3: s = fmax(in[3], 0.0); break;
-                case 4: s = fmax(in[4], 0.0); break;
-                default: s = fmax(in[5], 0.0); break;
-                }
+        const int end = ptr[i + 1];
+        for (int t = ptr[i]; t < end; ++t) {
+            const int4 tm = term[t];
+            const double4 p = par[t];
+            const double s = tm.y >= 0 ? v[tm.y * RC] : in[min(-1 - tm.y, 5) * RC];
             const double k = p.x;
             double r;
             switch (tm.x) {
-            case CW_ACTIVATED_BY: {
-                const double drv = tm.z ? hill(s, p.y, p.z) : s;
-                r = k * drv * (1.0 - own);
-                break;
-            }
+            case CW_ACTIVATED_BY:
             case CW_INHIBITED_BY: {
-                const double drv = tm.z ? hill(s, p.y, p.z) : s;
-                r = -k * drv * own;
+                double drv = s;
+                if (CLONES) {
+                    if (tm.z) drv = hill(s, p.y, p.z);
+                } else if (tm.z) {  // driver, network.rs:56-64, the half's power from the table
+                    const double sp = s > 0.0 ? s : 0.0;
+                    const double sn = tm.z == SQUARE ? sp * sp : pow(sp, p.y);
+                    drv = sn / (p.z + sn);
+                }
+                r = tm.x == CW_ACTIVATED_BY ? k * drv * rest : -k * drv * own;
                 break;
             }
-            case CW_ACTIVATED_BY_ABSENCE_OF: r = k * (1.0 - s) * (1.0 - own); break;
+            case CW_ACTIVATED_BY_ABSENCE_OF: r = k * (1.0 - s) * rest; break;
             case CW_PRODUCED_BY: r = k * s; break;
             case CW_DECAYS: r = -k * own; break;
             case CW_RELAXES_TO: r = -k * (own - p.w); break;
@@ -190,68 +138,69 @@ __global__ void __launch_bounds__(128) k_rk4_lanes(NetDev N, const NetDev *nets,
         return rate;
     };
     for (int sub = 0; sub < substeps; ++sub) {
-        // k1 at x
-        double k1 = rate_of(x);
-        double acc = k1;
-        double mid = x + 0.5 * dt * k1;
-        // k2 at x + dt/2 k1, k3 at x + dt/2 k2, k4 at x + dt k3
-        for (int stage = 1; stage < 4; ++stage) {
-            const double kv = rate_of(mid);
-            const double step = stage < 2 ? 0.5 * dt : dt;
-            if (stage < 3) {
-                acc = acc + 2.0 * kv;
-                mid = x + step * kv;
-            } else {
-                acc = acc + kv;
+        // k1 at x, k2 at x + dt/2 k1, k3 at x + dt/2 k2, k4 at x + dt k3
+        if (live)
+            for (int i = warp; i < S; i += G) {
+                const double k1 = rate_of(xs, i);
+                as[i * RC] = k1;
+                m0[i * RC] = xs[i * RC] + 0.5 * dt * k1;
             }
-        }
-        const double delta = (dt / 6.0) * acc;
-        x = fmin(fmax(x + delta, 0.0), 1.0);
+        __syncthreads();
+        if (live)
+            for (int i = warp; i < S; i += G) {
+                const double k2 = rate_of(m0, i);
+                as[i * RC] = as[i * RC] + 2.0 * k2;
+                m1[i * RC] = xs[i * RC] + 0.5 * dt * k2;
+            }
+        __syncthreads();
+        if (live)
+            for (int i = warp; i < S; i += G) {
+                const double k3 = rate_of(m1, i);
+                as[i * RC] = as[i * RC] + 2.0 * k3;
+                m0[i * RC] = xs[i * RC] + dt * k3;
+            }
+        __syncthreads();
+        if (live)
+            for (int i = warp; i < S; i += G) {
+                const double acc = as[i * RC] + rate_of(m0, i);
+                const double delta = (dt / 6.0) * acc;
+                xs[i * RC] = fmin(fmax(xs[i * RC] + delta, 0.0), 1.0);
+            }
+        __syncthreads();
     }
-    if (live) state[node * state_stride + c] = x;
+    if (live)
+        for (int i = warp; i < S; i += G) state[i * node_stride + c * cell_stride] = xs[i * RC];
 }
 
-// Cells above this many take one thread each (the warps walk one term list
-// together, no divergence); below it a lane per node puts more threads on
-// the few cells (measured: 2,144 cells of 12 nodes 384 -> 178 us; 136,384
-// cells of 8 nodes 521 -> 2,430 us with lanes, whose nodes diverge by term).
-constexpr int64_t LANES_BELOW = 16384;
-
-int rk4_lanes(const NetDev &N, const NetDev *nets, const int32_t *clone, int S, double *state, const double *inputs,
-              int64_t ncells, int64_t state_stride, int64_t input_stride, double dt, int substeps,
-              const uint8_t *alive, size_t cell_smem) {
-    if (ncells >= LANES_BELOW) {
-        const unsigned grid = (unsigned)((ncells + RT - 1) / RT);
-        if (nets) {
-            const size_t smem = sizeof(double) * 4 * S * RT;
-            if (smem > 48 * 1024)
-                CW_CUDA(cudaFuncSetAttribute(k_rk4_clones, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_rk4_clones<<<grid, RT, smem, stream()>>>(nets, clone, S, state, inputs, ncells, state_stride,
-                                                       input_stride, dt, substeps, alive);
-        } else {
-            k_rk4<<<grid, RT, cell_smem, stream()>>>(N, state, inputs, ncells, state_stride, input_stride, dt, substeps,
-                                                     alive);
-        }
-        CW_LAUNCHED();
-        return CW_OK;
-    }
-    const int W = S <= 8 ? 8 : S <= 16 ? 16 : 32;
-    const int64_t threads = ncells * W;
-    const unsigned grid = (unsigned)((threads + 127) / 128);
-    if (W == 8)
-        k_rk4_lanes<8><<<grid, 128, 0, stream()>>>(N, nets, clone, state, inputs, ncells, state_stride, input_stride,
-                                                   dt, substeps, alive);
-    else if (W == 16)
-        k_rk4_lanes<16><<<grid, 128, 0, stream()>>>(N, nets, clone, state, inputs, ncells, state_stride,
-                                                    input_stride, dt, substeps, alive);
-    else
-        k_rk4_lanes<32><<<grid, 128, 0, stream()>>>(N, nets, clone, state, inputs, ncells, state_stride,
-                                                    input_stride, dt, substeps, alive);
+template <int G, bool CLONES>
+int rk4_launch(const NetDev &N, const NetDev *nets, const int32_t *clone, int S, double *state, const double *inputs,
+               int64_t ncells, int64_t node_stride, int64_t cell_stride, int64_t in_stride, int64_t in_cell, double dt,
+               int substeps, const uint8_t *alive) {
+    k_rk4<G, CLONES><<<(unsigned)((ncells + RC - 1) / RC), 32 * G, rk4_block(S, CLONES ? 0 : N.nterms), stream()>>>(
+        N, nets, clone, S, state, inputs, ncells, node_stride, cell_stride, in_stride, in_cell, dt, substeps, alive);
     CW_LAUNCHED();
     return CW_OK;
 }
 
-// mechanics, network.rs:811-821.
+int rk4_cells(const NetDev &N, const NetDev *nets, const int32_t *clone, int S, double *state, const double *inputs,
+              int64_t ncells, int64_t node_stride, int64_t cell_stride, int64_t in_stride, int64_t in_cell, double dt,
+              int substeps, const uint8_t *alive) {
+    int dev = 0, nsm = 0;
+    CW_CUDA(cudaGetDevice(&dev));
+    CW_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t nblocks = (ncells + RC - 1) / RC;
+    // A warp per node up to 16 while the blocks are few, for the shortest chain
+    // (5,000 cells of 12 nodes 78 us against 120 with 8 warps); 8 warps where the
+    // blocks fill the device, which then holds more cells at a time (40,000 cells
+    // of 16 nodes 366 us against 425 with 16); 4 for many cells of few nodes, for
+    // fewer warps at a barrier (400,000 cells of 8 nodes 918 us against 971 with 8).
+    auto go = S > 8 && nblocks <= 2 * nsm     ? (nets ? rk4_launch<16, true> : rk4_launch<16, false>)
+              : S <= 8 && nblocks > 16 * nsm ? (nets ? rk4_launch<4, true> : rk4_launch<4, false>)
+                                             : (nets ? rk4_launch<8, true> : rk4_launch<8, false>);
+    return go(N, nets, clone, S, state, inputs, ncells, node_stride, cell_stride, in_stride, in_cell, dt, substeps,
+              alive);
+}
+
 __global__ void k_mechanics(const double *state, int64_t ncells, int64_t stride, int growth, double coefficient,
                             double max_target, int has_max, uint32_t reference_volume, uint32_t *target) {
     int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,8 +212,10 @@ __global__ void k_mechanics(const double *state, int64_t ncells, int64_t stride,
     target[c] = isnan(t) ? 0u : (t >= 4294967295.0 ? 4294967295u : (uint32_t)t);
 }
 
-size_t rk4_smem(const cw_network_s *n) {
-    return sizeof(double) * 4 * n->S * RT + n->nterms * (sizeof(int4) + sizeof(double4)) + sizeof(int32_t) * (n->S + 1);
+// The most terms a network may have: what a block's shared memory would hold
+// beside 64 cells' columns.
+size_t network_bytes(const cw_network_s *n) {
+    return sizeof(double) * 4 * n->S * 64 + n->nterms * (sizeof(int4) + sizeof(double4)) + sizeof(int32_t) * (n->S + 1);
 }
 
 // The device copies of a network's host tables (h_ptr, h_term, h_par).
@@ -279,10 +230,16 @@ int network_upload(cw_network_s *n) {
         CW_CUDA(cudaMemcpy(n->term, n->h_term.data(), sizeof(int4) * n->nterms, cudaMemcpyHostToDevice));
         CW_CUDA(cudaMemcpy(n->par, n->h_par.data(), sizeof(double4) * n->nterms, cudaMemcpyHostToDevice));
     }
-    size_t smem = rk4_smem(n);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_rk4, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    int dev = 0, most = 0;
+    CW_CUDA(cudaGetDevice(&dev));
+    CW_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    if (network_bytes(n) > (size_t)most)
         return fail(CW_ERR_CONFIG, "the network is too large for one block's shared memory");
+    // (to the most there is, not to this network's need: it is the kernel's, whichever network it runs)
+    if (rk4_block(n->S, n->nterms) > 48 * 1024) {
+        for (auto k : {k_rk4<4, false>, k_rk4<8, false>, k_rk4<16, false>})
+            CW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    }
     return CW_OK;
 }
 
@@ -335,8 +292,8 @@ NetDev net_dev(const cw_network_s *n) { return NetDev{n->node_ptr, n->term, n->p
 int network_step_device(const cw_network_s *n, double *state, const double *inputs, int64_t ncells,
                         int64_t state_stride, int64_t input_stride, double dt, int substeps, const uint8_t *alive) {
     if (ncells <= 0) return CW_OK;
-    return rk4_lanes(net_dev(n), nullptr, nullptr, n->S, state, inputs, ncells, state_stride, input_stride, dt,
-                     substeps, alive, rk4_smem(n));
+    return rk4_cells(net_dev(n), nullptr, nullptr, n->S, state, inputs, ncells, state_stride, 1, input_stride, 1, dt,
+                     substeps, alive);
 }
 
 // RK4 for cells of many networks on node-major state (the driver's evolving
@@ -347,7 +304,8 @@ int network_step_clones_device(const NetDev *nets, const int32_t *clone, int S, 
     if (ncells <= 0) return CW_OK;
     NetDev none{};
     none.S = S;
-    return rk4_lanes(none, nets, clone, S, state, inputs, ncells, state_stride, input_stride, dt, substeps, alive, 0);
+    return rk4_cells(none, nets, clone, S, state, inputs, ncells, state_stride, 1, input_stride, 1, dt, substeps,
+                     alive);
 }
 
 int network_mechanics_device(const cw_network_s *n, const double *state, int64_t ncells, int64_t stride,
@@ -648,8 +606,8 @@ int cw_network_step_clones(int32_t nnets, const cw_network *nets, int64_t ncells
     CW_CUDA(cudaMemcpy(d_clone, clone, sizeof(int32_t) * ncells, cudaMemcpyHostToDevice));
     NetDev none{};
     none.S = S;
-    if ((rc = rk4_lanes(none, d_nets, d_clone, S, d_state, d_in, ncells, ncells, ncells, dt, substeps, nullptr, 0)) !=
-        CW_OK)
+    if ((rc = rk4_cells(none, d_nets, d_clone, S, d_state, d_in, ncells, ncells, 1, ncells, 1, dt, substeps,
+                        nullptr)) != CW_OK)
         return rc;
     CW_CUDA(cudaGetLastError());
     CW_CUDA(cudaMemcpyAsync(t.data(), d_state, sizeof(double) * ncells * S, cudaMemcpyDeviceToHost, stream()));
