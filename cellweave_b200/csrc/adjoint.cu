@@ -131,142 +131,279 @@ __global__ void __launch_bounds__(RB) k_fit_forward(NetDev N, const double *x0, 
     for (int i = 0; i < S; ++i) xT[i * nc + c] = x[i * RB + t];
 }
 
-// Hill response and its slope in s (driver, network.rs:56-64).
-__device__ __forceinline__ void hill_d(double s, double n, double half, double &v, double &dv) {
-    if (s <= 0.0) { v = 0.0; dv = 0.0; return; }
-    double sn, hn, dsn;
-    if (n == 2.0) { sn = s * s; hn = half * half; dsn = 2.0 * s; }
-    else { sn = pow(s, n); hn = pow(half, n); dsn = n * pow(s, n - 1.0); }
-    double den = hn + sn;
-    v = sn / den;
-    dv = dsn * hn / (den * den);
-}
-
-// Vector-Jacobian product of the network's right-hand side at z with the
-// adjoint a: adds a . df/dz to gx, a . df/dtheta (the first ntheta rates) to
-// gth, and a . df/d(oxygen input) to *gin.  Columns have stride RB.
-__device__ void vjp_f(const NetDev &N, const int4 *sterm, const double4 *spar, const int32_t *sptr, const double *z,
-                      const double *in, const double *a, double *gx, double *gth, int ntheta, double &gin) {
-    const int S = N.S;
-    const double o2 = in[0];
-    const double o2_slope = (o2 > 0.0 && o2 < 1.0) ? 1.0 : 0.0;  // read clamps oxygen to [0, 1]
-    for (int i = 0; i < S; ++i) {
-        const double ai = a[i * RB];
+// Vector-Jacobian product of the network's right-hand side at the lane's values
+// z with the adjoint a, for one node: a . df/d(z_node), and of node S the
+// oxygen's (gin).  `list` holds what the node takes part in, in file order: its
+// own terms (2 t) and the terms that read it (2 t + 1), a term that reads its
+// own node as both.  The rates' gradients (the first ntheta terms) go to gth,
+// each written by its own node's warp.
+__device__ __forceinline__ double vjp_node(const int4 *sterm, const double4 *spar, const uint32_t *list, int from,
+                                           int end, const double *z, const double *in, const double *a, double *gth,
+                                           int ntheta) {
+    double g = 0.0;
+    for (int e = from; e < end; ++e) {
+        const int t = (int)(list[e] >> 1);
+        const int4 tm = sterm[t];  // w: the term's own node
+        const double ai = a[tm.w * RC];
         if (ai == 0.0) continue;
-        const double own = z[i * RB];
-        for (int t = sptr[i]; t < sptr[i + 1]; ++t) {
-            const int4 tm = sterm[t];
-            const double4 p = spar[t];
-            const double k = p.x;
-            double s = 0.0, ds = 0.0;  // the source and d(read)/d(its variable)
-            if (tm.x != CW_DECAYS && tm.x != CW_RELAXES_TO) {
-                s = read_source(tm.y, in, z, RB);
-                ds = tm.y >= 0 ? 1.0 : (tm.y == -1 ? o2_slope : 0.0);
-            }
-            double g_own = 0.0, g_s = 0.0, g_k = 0.0;
+        const double4 p = spar[t];
+        const double own = z[tm.w * RC], s = source_of(tm, z, in), k = p.x;
+        if (list[e] & 1u) {
+            double gs = 0.0;
             switch (tm.x) {
             case CW_ACTIVATED_BY:
             case CW_INHIBITED_BY: {
-                double drv = s, ddrv = 1.0;
-                if (tm.z) hill_d(s, p.y, p.z, drv, ddrv);
-                if (tm.x == CW_ACTIVATED_BY) { g_own = -k * drv; g_s = k * ddrv * (1.0 - own); g_k = drv * (1.0 - own); }
-                else { g_own = -k * drv; g_s = -k * ddrv * own; g_k = -drv * own; }
+                double ddrv = 1.0;
+                if (tm.z) {
+                    ddrv = 0.0;
+                    if (s > 0.0) {
+                        const double sn = tm.z == SQUARE ? s * s : pow(s, p.y);
+                        const double dsn = tm.z == SQUARE ? 2.0 * s : p.y * pow(s, p.y - 1.0);
+                        const double den = p.z + sn;
+                        ddrv = dsn * p.z / (den * den);
+                    }
+                }
+                gs = tm.x == CW_ACTIVATED_BY ? k * ddrv * (1.0 - own) : -k * ddrv * own;
                 break;
             }
-            case CW_ACTIVATED_BY_ABSENCE_OF: g_own = -k * (1.0 - s); g_s = -k * (1.0 - own); g_k = (1.0 - s) * (1.0 - own); break;
-            case CW_PRODUCED_BY: g_s = k; g_k = s; break;
+            case CW_ACTIVATED_BY_ABSENCE_OF: gs = -k * (1.0 - own); break;
+            case CW_PRODUCED_BY: gs = k; break;
+            case CW_DAMAGED_BELOW:
+                if ((p.w - s) / p.w > 0.0) gs = k / p.w;
+                break;
+            default:
+                if ((s - p.w) / p.w > 0.0) gs = -k / p.w;
+                break;
+            }
+            g += ai * gs;
+        } else {
+            double g_own = 0.0, g_k = 0.0;
+            switch (tm.x) {
+            case CW_ACTIVATED_BY:
+            case CW_INHIBITED_BY: {
+                double drv = s;
+                if (tm.z) {
+                    drv = 0.0;
+                    if (s > 0.0) {
+                        const double sn = tm.z == SQUARE ? s * s : pow(s, p.y);
+                        drv = sn / (p.z + sn);
+                    }
+                }
+                g_own = -k * drv;
+                g_k = tm.x == CW_ACTIVATED_BY ? drv * (1.0 - own) : -drv * own;
+                break;
+            }
+            case CW_ACTIVATED_BY_ABSENCE_OF: g_own = -k * (1.0 - s); g_k = (1.0 - s) * (1.0 - own); break;
+            case CW_PRODUCED_BY: g_k = s; break;
             case CW_DECAYS: g_own = -k; g_k = -own; break;
             case CW_RELAXES_TO: g_own = -k; g_k = -(own - p.w); break;
             case CW_DAMAGED_BELOW: {
-                double u = (p.w - s) / p.w;
-                if (u > 0.0) { g_s = k / p.w; g_k = -u; }
+                const double u = (p.w - s) / p.w;
+                if (u > 0.0) g_k = -u;
                 break;
             }
             default: {
-                double u = (s - p.w) / p.w;
-                if (u > 0.0) { g_s = -k / p.w; g_k = -u; }
+                const double u = (s - p.w) / p.w;
+                if (u > 0.0) g_k = -u;
                 break;
             }
             }
-            gx[i * RB] += ai * g_own;
-            if (tm.y >= 0 && tm.x != CW_DECAYS && tm.x != CW_RELAXES_TO) gx[tm.y * RB] += ai * g_s * ds;
-            else if (tm.y == -1 && tm.x != CW_DECAYS && tm.x != CW_RELAXES_TO) gin += ai * g_s * ds;
-            if (t < ntheta) gth[t * RB] += ai * g_k;
+            g += ai * g_own;
+            if (t < ntheta) gth[t * RC] += ai * g_k;
         }
+    }
+    return g;
+}
+
+// Shared bytes of a backward block.
+size_t backward_block(int S, int nterms, int ntheta) {
+    return sizeof(double) * (9 * S + 6 + ntheta) * RC + nterms * (sizeof(int4) + sizeof(double4)) +
+           sizeof(int32_t) * (S + 1) + sizeof(uint32_t) * (2 * nterms + S + 2);
+}
+
+// Reverse RK4 over one checkpointed segment of K steps, a lane per cell and a
+// cell's nodes over the block's G warps, as the forward step runs (k_rk4).
+// Each node gathers what it takes part in, so no two warps add to one number,
+// and in file order: a result does not depend on G.  lam holds dL/dx at the
+// segment's end on entry and at its start on return.  Node i of cell c: the
+// state at ckm[i * node_stride + c * cell_stride], lam alike; input q at
+// inputs[q * in_stride + c * in_cell]; seg: K S nc numbers of scratch.
+//
+// What bounds it: FP64 latency, a chain of K steps with eight evaluations each.
+// A thread per cell, every node's terms in turn, took 3.86 ms for 8,192 cells of
+// 8 nodes and 40 steps (128 blocks of two warps); dealt to 8 warps
+// 0.89; of 16 nodes to 16 warps 12.3 -> 2.0 ms; 137,000 cells of 8 nodes, 8 steps,
+// 3.99 -> 1.88 ms.
+template <int G>
+__global__ void __launch_bounds__(32 * G)
+    k_fit_backward(NetDev N, const double *ckm, const double *inputs, int64_t nc, int64_t node_stride,
+                   int64_t cell_stride, int64_t in_stride, int64_t in_cell, int K, double dt, double *seg, double *lam,
+                   double *gin_out, double *gth_out, int ntheta) {
+    extern __shared__ double sm[];
+    const int S = N.S, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *const X = sm + lane, *const M1 = X + S * RC, *const M2 = M1 + S * RC, *const M3 = M2 + S * RC,
+                  *const AC = M3 + S * RC, *const MU = AC + S * RC, *const LN = MU + S * RC, *const A0 = LN + S * RC,
+                  *const A1 = A0 + S * RC, *const in = A1 + S * RC, *const gth = in + 6 * RC;
+    int4 *sterm = (int4 *)(sm + (9 * S + 6 + ntheta) * RC);
+    double4 *spar = (double4 *)(sterm + N.nterms);
+    int32_t *sptr = (int32_t *)(spar + N.nterms);
+    uint32_t *lptr = (uint32_t *)(sptr + S + 1), *list = lptr + S + 2;
+    stage_terms(N, sterm, spar, sptr);
+    __syncthreads();
+    for (int i = threadIdx.x; i < S; i += 32 * G)
+        for (int t = sptr[i]; t < sptr[i + 1]; ++t) sterm[t].w = i;
+    for (int q = warp; q < ntheta; q += G) gth[q * RC] = 0.0;
+    __syncthreads();
+    // the nodes' lists (node S: the terms that read oxygen): counted, placed, filled
+    auto reads = [](const int4 &tm) { return tm.x != CW_DECAYS && tm.x != CW_RELAXES_TO; };
+    for (int i = threadIdx.x; i <= S; i += 32 * G) {
+        uint32_t n = 0;
+        for (int t = 0; t < N.nterms; ++t) {
+            const int4 tm = sterm[t];
+            n += (tm.w == i) + (reads(tm) && tm.y == (i < S ? i : -1));
+        }
+        lptr[i + 1] = n;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        lptr[0] = 0;
+        for (int i = 0; i <= S; ++i) lptr[i + 1] += lptr[i];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= S; i += 32 * G) {
+        uint32_t e = lptr[i];
+        for (int t = 0; t < N.nterms; ++t) {
+            const int4 tm = sterm[t];
+            if (tm.w == i) list[e++] = 2u * t;
+            if (reads(tm) && tm.y == (i < S ? i : -1)) list[e++] = 2u * t + 1u;
+        }
+    }
+    const int64_t c = (int64_t)blockIdx.x * RC + lane;
+    const bool live = c < nc;
+    double gin = 0.0, o2_slope = 0.0;
+    if (live) {
+        const double o2 = inputs[c * in_cell];
+        o2_slope = (o2 > 0.0 && o2 < 1.0) ? 1.0 : 0.0;  // read clamps oxygen to [0, 1]
+        for (int q = warp; q < 6; q += G) in[q * RC] = clamped_input(q, inputs[q * in_stride + c * in_cell]);
+        for (int i = warp; i < S; i += G) {
+            X[i * RC] = ckm[i * node_stride + c * cell_stride];
+            LN[i * RC] = lam[i * node_stride + c * cell_stride];
+            seg[(int64_t)i * nc + c] = X[i * RC];
+        }
+    }
+    __syncthreads();
+    // the stages' points M1, M2, M3 of a step from X, and X's slopes summed in AC
+    // (k1 + 2 k2 + 2 k3 + k4); ends with the last stage read by this warp alone
+    auto stages = [&]() {
+        if (live)
+            for (int i = warp; i < S; i += G) {
+                const double k = node_rate<false>(sterm, spar, sptr, X, in, i);
+                AC[i * RC] = k;
+                M1[i * RC] = X[i * RC] + 0.5 * dt * k;
+            }
+        __syncthreads();
+#pragma unroll 1
+        for (int stage = 2; stage < 4; ++stage) {
+            const double *const v = stage == 2 ? M1 : M2;
+            double *const m = stage == 2 ? M2 : M3;
+            const double step = stage == 2 ? 0.5 * dt : dt;
+            if (live)
+                for (int i = warp; i < S; i += G) {
+                    const double k = node_rate<false>(sterm, spar, sptr, v, in, i);
+                    AC[i * RC] = AC[i * RC] + 2.0 * k;
+                    m[i * RC] = X[i * RC] + step * k;
+                }
+            __syncthreads();
+        }
+        if (live)
+            for (int i = warp; i < S; i += G) AC[i * RC] = AC[i * RC] + node_rate<false>(sterm, spar, sptr, M3, in, i);
+    };
+    // the segment's states
+    for (int s = 1; s < K; ++s) {
+        stages();
+        if (live)
+            for (int i = warp; i < S; i += G) {
+                const double x = fmin(fmax(X[i * RC] + (dt / 6.0) * AC[i * RC], 0.0), 1.0);
+                X[i * RC] = x;
+                seg[((int64_t)s * S + i) * nc + c] = x;
+            }
+        __syncthreads();
+    }
+    for (int s = K - 1; s >= 0; --s) {
+        if (s < K - 1) {
+            if (live)
+                for (int i = warp; i < S; i += G) X[i * RC] = seg[((int64_t)s * S + i) * nc + c];
+            __syncthreads();
+        }
+        stages();
+        if (live)
+            for (int i = warp; i < S; i += G) {
+                const double y = X[i * RC] + (dt / 6.0) * AC[i * RC];
+                const double mu = (y > 0.0 && y < 1.0) ? LN[i * RC] : 0.0;  // the clamp to [0, 1]
+                MU[i * RC] = mu;
+                LN[i * RC] = mu;                // x_{t+1} = y: dy/dx = 1
+                A0[i * RC] = mu * (dt / 6.0);   // stage 4's adjoint
+            }
+        __syncthreads();
+        // stages 4 to 1, at m3 = x + dt k3, m2 = x + dt/2 k2, m1 = x + dt/2 k1 and x
+#pragma unroll 1
+        for (int stage = 4; stage > 0; --stage) {
+            const double *const z = stage == 4 ? M3 : stage == 3 ? M2 : stage == 2 ? M1 : X;
+            const double *const a = stage & 1 ? A1 : A0;
+            double *const next = stage & 1 ? A0 : A1;
+            const double share = stage > 2 ? dt / 3.0 : dt / 6.0, step = stage == 4 ? dt : 0.5 * dt;
+            if (live)
+                for (int i = warp; i <= S; i += G) {
+                    const double g = vjp_node(sterm, spar, list, (int)lptr[i], (int)lptr[i + 1], z, in, a, gth, ntheta);
+                    if (i == S) {
+                        gin += g * o2_slope;
+                        continue;
+                    }
+                    LN[i * RC] += g;
+                    if (stage > 1) next[i * RC] = MU[i * RC] * share + step * g;
+                }
+            __syncthreads();
+        }
+    }
+    if (live) {
+        for (int i = warp; i < S; i += G) lam[i * node_stride + c * cell_stride] = LN[i * RC];
+        if (warp == S % G) gin_out[c] += gin;
+    }
+    // FP64 reduction of the rate gradients over the block's cells
+    for (int q = warp; q < ntheta; q += G) {
+        const double v = warp_sum(gth[q * RC]);
+        if (lane == 0 && v != 0.0) atomicAdd(gth_out + q, v);
     }
 }
 
-// Reverse RK4 over one checkpointed segment of K steps.  lam holds
-// dL/dx at the segment's end on entry and at its start on return.
-__global__ void __launch_bounds__(RB) k_fit_backward(NetDev N, const double *ckm, const double *inputs, int64_t nc,
-                                                     int K, double dt, double *seg, double *lam, double *gin_out,
-                                                     double *gth_out, int ntheta) {
-    extern __shared__ double sm[];
-    const int S = N.S;
-    double *x = sm, *m = x + S * RB, *k1 = m + S * RB, *k2 = k1 + S * RB, *k3 = k2 + S * RB, *ln = k3 + S * RB;
-    double *mu = ln + S * RB, *a = mu + S * RB, *gx = a + S * RB, *gth = gx + S * RB, *acc = gth + MAXTH * RB;
-    int4 *sterm = (int4 *)(acc + S * RB);
-    double4 *spar = (double4 *)(sterm + N.nterms);
-    int32_t *sptr = (int32_t *)(spar + N.nterms);
-    load_net(N, sterm, spar, sptr);
-    const int t = threadIdx.x;
-    for (int q = 0; q < ntheta; ++q) gth[q * RB + t] = 0.0;
-    __syncthreads();
-    int64_t c = (int64_t)blockIdx.x * RB + t;
-    double gin = 0.0;
-    if (c < nc) {
-        double in[6];
-        for (int q = 0; q < 6; ++q) in[q] = inputs[q * nc + c];
-        double *X = x + t, *M = m + t, *K1 = k1 + t, *K2 = k2 + t, *K3 = k3 + t, *LN = ln + t, *MU = mu + t;
-        double *A = a + t, *GX = gx + t, *G = gth + t, *ACC = acc + t;
-        // recompute the segment's states
-        for (int i = 0; i < S; ++i) { X[i * RB] = ckm[i * nc + c]; seg[(int64_t)i * nc + c] = X[i * RB]; }
-        for (int s = 0; s < K; ++s) {
-            rk4_step(N, sterm, spar, sptr, X, M, K1, ACC, in, dt);
-            for (int i = 0; i < S; ++i) seg[((int64_t)(s + 1) * S + i) * nc + c] = X[i * RB];
-        }
-        for (int s = K - 1; s >= 0; --s) {
-            for (int i = 0; i < S; ++i) X[i * RB] = seg[((int64_t)s * S + i) * nc + c];
-            // forward stages of this step
-            derivatives(N, sterm, spar, sptr, X, in, K1, RB);
-            for (int i = 0; i < S; ++i) M[i * RB] = X[i * RB] + 0.5 * dt * K1[i * RB];
-            derivatives(N, sterm, spar, sptr, M, in, K2, RB);
-            for (int i = 0; i < S; ++i) M[i * RB] = X[i * RB] + 0.5 * dt * K2[i * RB];
-            derivatives(N, sterm, spar, sptr, M, in, K3, RB);
-            for (int i = 0; i < S; ++i) M[i * RB] = X[i * RB] + dt * K3[i * RB];
-            derivatives(N, sterm, spar, sptr, M, in, GX, RB);  // k4 in GX for the moment
-            for (int i = 0; i < S; ++i) {
-                double y = X[i * RB] + (dt / 6.0) * (K1[i * RB] + 2.0 * K2[i * RB] + 2.0 * K3[i * RB] + GX[i * RB]);
-                double l = lam[(int64_t)i * nc + c];
-                MU[i * RB] = (y > 0.0 && y < 1.0) ? l : 0.0;  // the clamp to [0, 1]
-                LN[i * RB] = MU[i * RB];                       // x_{t+1} = y: dy/dx = 1
-            }
-            // stage 4 at m3 = x + dt k3, adjoint mu dt/6
-            for (int i = 0; i < S; ++i) { A[i * RB] = MU[i * RB] * (dt / 6.0); GX[i * RB] = 0.0; }
-            vjp_f(N, sterm, spar, sptr, M, in, A, GX, G, ntheta, gin);
-            for (int i = 0; i < S; ++i) { LN[i * RB] += GX[i * RB]; A[i * RB] = MU[i * RB] * (dt / 3.0) + dt * GX[i * RB]; }
-            // stage 3 at m2 = x + dt/2 k2
-            for (int i = 0; i < S; ++i) { M[i * RB] = X[i * RB] + 0.5 * dt * K2[i * RB]; GX[i * RB] = 0.0; }
-            vjp_f(N, sterm, spar, sptr, M, in, A, GX, G, ntheta, gin);
-            for (int i = 0; i < S; ++i) { LN[i * RB] += GX[i * RB]; A[i * RB] = MU[i * RB] * (dt / 3.0) + 0.5 * dt * GX[i * RB]; }
-            // stage 2 at m1 = x + dt/2 k1
-            for (int i = 0; i < S; ++i) { M[i * RB] = X[i * RB] + 0.5 * dt * K1[i * RB]; GX[i * RB] = 0.0; }
-            vjp_f(N, sterm, spar, sptr, M, in, A, GX, G, ntheta, gin);
-            for (int i = 0; i < S; ++i) { LN[i * RB] += GX[i * RB]; A[i * RB] = MU[i * RB] * (dt / 6.0) + 0.5 * dt * GX[i * RB]; }
-            // stage 1 at x
-            for (int i = 0; i < S; ++i) GX[i * RB] = 0.0;
-            vjp_f(N, sterm, spar, sptr, X, in, A, GX, G, ntheta, gin);
-            for (int i = 0; i < S; ++i) lam[(int64_t)i * nc + c] = LN[i * RB] + GX[i * RB];
-        }
-        gin_out[c] += gin;
-    }
-    // FP64 reduction of the rate gradients over the block's cells
-    __syncthreads();
-    for (int q = 0; q < ntheta; ++q) {
-        double v = gth[q * RB + t];
-        v = warp_sum(v);
-        if ((t & 31) == 0 && v != 0.0) atomicAdd(gth_out + q, v);
-    }
+// Whether the device holds a network's backward step (beside 64 cells' columns), and the launch.
+int backward_fits(int S, int nterms) {
+    int dev = 0, most = 0;
+    CW_CUDA(cudaGetDevice(&dev));
+    CW_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    if (sizeof(double) * (10 * S + MAXTH) * RB + nterms * (sizeof(int4) + sizeof(double4)) + sizeof(int32_t) * (S + 1) >
+        (size_t)most)
+        return CW_ERR_CONFIG;
+    // (to the most there is: the attribute is the kernel's, whichever network it runs)
+    if (backward_block(S, nterms, MAXTH) > 48 * 1024)
+        for (auto k : {k_fit_backward<8>, k_fit_backward<16>})
+            CW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return CW_OK;
+}
+
+int backward_launch(const NetDev &N, const double *ckm, const double *inputs, int64_t nc, int64_t node_stride,
+                    int64_t cell_stride, int64_t in_stride, int64_t in_cell, int K, double dt, double *seg, double *lam,
+                    double *gin, double *gth, int ntheta) {
+    const unsigned grid = (unsigned)((nc + RC - 1) / RC);
+    const size_t smem = backward_block(N.S, N.nterms, ntheta);
+    if (N.S > 8)
+        k_fit_backward<16><<<grid, 512, smem, stream()>>>(N, ckm, inputs, nc, node_stride, cell_stride, in_stride,
+                                                          in_cell, K, dt, seg, lam, gin, gth, ntheta);
+    else
+        k_fit_backward<8><<<grid, 256, smem, stream()>>>(N, ckm, inputs, nc, node_stride, cell_stride, in_stride,
+                                                         in_cell, K, dt, seg, lam, gin, gth, ntheta);
+    CW_LAUNCHED();
+    return CW_OK;
 }
 
 // Every cell's mean of `v` over its pixels (mean_per_cell, coupling.rs:164-182),
@@ -395,11 +532,6 @@ size_t fwd_smem(const cw_fit_s *f) {
     return sizeof(double) * 4 * f->S * RB + f->net->nterms * (sizeof(int4) + sizeof(double4)) +
            sizeof(int32_t) * (f->S + 1);
 }
-size_t bwd_smem(const cw_fit_s *f) {
-    return sizeof(double) * (10 * f->S + MAXTH) * RB + f->net->nterms * (sizeof(int4) + sizeof(double4)) +
-           sizeof(int32_t) * (f->S + 1);
-}
-
 int fit_relax(cw_fit_s *f, cw_field_s *fld, double tol) {
     cw_relax_opts o{};
     o.omega = f->cfg.omega;
@@ -468,7 +600,7 @@ int cw_fit_create(cw_lattice lat, cw_network net, const cw_fit_config *cfg, cw_f
         (rc = dalloc(&f->mean2, nc)) || (rc = dalloc(&f->count, nc)) || (rc = dalloc(&f->count2, nc)) ||
         (rc = dalloc(&f->inputs, 6 * nc)) || (rc = dalloc(&f->x0, S)) || (rc = dalloc(&f->xT, S * nc)) ||
         (rc = dalloc(&f->lam, S * nc)) || (rc = dalloc(&f->gin, nc)) || (rc = dalloc(&f->ck, M * S * nc)) ||
-        (rc = dalloc(&f->seg, (cfg->checkpoint_every + 1) * S * nc)) || (rc = dalloc(&f->bins, 3 * cfg->nbins)) ||
+        (rc = dalloc(&f->seg, cfg->checkpoint_every * S * nc)) || (rc = dalloc(&f->bins, 3 * cfg->nbins)) ||
         (rc = dalloc(&f->coef, 2 * cfg->nbins)) || (rc = dalloc(&f->grad, 4 + MAXTH))) {
         cw_fit_destroy(f);
         return rc;
@@ -520,8 +652,8 @@ int cw_fit_create(cw_lattice lat, cw_network net, const cw_fit_config *cfg, cw_f
                                 stream()));
         CW_CUDA(cudaStreamSynchronize(stream()));
     }
-    size_t sb = bwd_smem(f), sf = fwd_smem(f);
-    if (sb > 48 * 1024 && cudaFuncSetAttribute(k_fit_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb))
+    size_t sf = fwd_smem(f);
+    if (backward_fits(f->S, f->net->nterms) != CW_OK)
         return fail(CW_ERR_CONFIG, "the network is too large for the adjoint's shared memory");
     if (sf > 48 * 1024 && cudaFuncSetAttribute(k_fit_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf))
         return fail(CW_ERR_CONFIG, "the network is too large for the forward's shared memory");
@@ -664,10 +796,9 @@ int cw_fit_gradient(cw_fit f, double *loss, double *grad) {
     NetDev N = fit_net(f);
     const int M = c.steps / c.checkpoint_every;
     for (int m = M - 1; m >= 0; --m) {
-        k_fit_backward<<<(unsigned)((f->nc + RB - 1) / RB), RB, bwd_smem(f), stream()>>>(
-            N, f->ck + (int64_t)m * f->S * f->nc, f->inputs, f->nc, c.checkpoint_every, c.dt, f->seg, f->lam, f->gin,
-            f->grad + 4, f->ntheta);
-        CW_LAUNCHED();
+        if ((rc = backward_launch(N, f->ck + (int64_t)m * f->S * f->nc, f->inputs, f->nc, f->nc, 1, f->nc, 1,
+                                  c.checkpoint_every, c.dt, f->seg, f->lam, f->gin, f->grad + 4, f->ntheta)) != CW_OK)
+            return rc;
     }
     // oxygen adjoint
     k_fit_gc<<<blocks(f->n), T, 0, stream()>>>(f->lat->grid, f->o2->c, W, f->n, f->nc, c.vessel_x, c.bin_width, nb,
@@ -716,7 +847,7 @@ extern "C" int cw_network_backward_batch(cw_network net, int64_t ncells, const d
     double *d_x = nullptr, *d_in = nullptr, *d_seg = nullptr, *d_lam = nullptr, *d_gin = nullptr, *d_gth = nullptr;
     auto release = [&]() { dfree(d_x); dfree(d_in); dfree(d_seg); dfree(d_lam); dfree(d_gin); dfree(d_gth); };
     int rc;
-    if ((rc = dalloc(&d_x, S * nc)) || (rc = dalloc(&d_in, 6 * nc)) || (rc = dalloc(&d_seg, (substeps + 1) * S * nc)) ||
+    if ((rc = dalloc(&d_x, S * nc)) || (rc = dalloc(&d_in, 6 * nc)) || (rc = dalloc(&d_seg, substeps * S * nc)) ||
         (rc = dalloc(&d_lam, S * nc)) || (rc = dalloc(&d_gin, nc)) || (rc = dalloc(&d_gth, MAXTH))) {
         release();
         return rc;
@@ -726,19 +857,16 @@ extern "C" int cw_network_backward_batch(cw_network net, int64_t ncells, const d
     CW_CUDA(cudaMemcpyAsync(d_lam, lam.data(), sizeof(double) * S * nc, cudaMemcpyHostToDevice, stream()));
     CW_CUDA(cudaMemsetAsync(d_gin, 0, sizeof(double) * nc, stream()));
     CW_CUDA(cudaMemsetAsync(d_gth, 0, sizeof(double) * MAXTH, stream()));
-    const size_t smem = sizeof(double) * (10 * S + MAXTH) * RB + net->nterms * (sizeof(int4) + sizeof(double4)) +
-                        sizeof(int32_t) * (S + 1);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_fit_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (backward_fits(net->S, net->nterms) != CW_OK) {
         release();
         return fail(CW_ERR_CONFIG, "the network is too large for the backward step's shared memory");
     }
     NetDev N{net->node_ptr, net->term, net->par, net->S, net->nterms};
-    k_fit_backward<<<(unsigned)((nc + RB - 1) / RB), RB, smem, stream()>>>(N, d_x, d_in, nc, substeps, dt, d_seg,
-                                                                          d_lam, d_gin, d_gth, nrates);
-    count_launch();
-    const cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess) { release(); return cuda_fail(le, "kernel launch"); }
+    if ((rc = backward_launch(N, d_x, d_in, nc, nc, 1, nc, 1, substeps, dt, d_seg, d_lam, d_gin, d_gth, nrates)) !=
+        CW_OK) {
+        release();
+        return rc;
+    }
     std::vector<double> gin(nc), gth(MAXTH);
     CW_CUDA(cudaMemcpyAsync(lam.data(), d_lam, sizeof(double) * S * nc, cudaMemcpyDeviceToHost, stream()));
     CW_CUDA(cudaMemcpyAsync(gin.data(), d_gin, sizeof(double) * nc, cudaMemcpyDeviceToHost, stream()));

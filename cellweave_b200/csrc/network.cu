@@ -39,18 +39,11 @@ constexpr int MAXS = 32;
 // What bounds it: with few cells the chain of a node's terms, each with a
 // division; with many the FP64 instructions themselves.  A thread per cell (and
 // for few cells a lane per node, whose warps diverged by kind of term) took, 10
-// steps of 8 nodes: 300 cells 111 -> 47 us, 1,260 cells 115 -> 51, 16,000 cells
-// 163 -> 70; 8 steps: 137,000 cells 452 -> 334, 40,000 cells of 16 nodes 693 ->
-// 366, of 32 nodes 5,959 -> 1,177.  Five blocks of 8 warps an SM (48 registers a
-// thread, a few of the power spilled; four blocks spill next to none and take
-// 445 us where five take 366).
-constexpr int RC = 32;  // cells per block
-enum { SQUARE = 2, POWER = 3 };  // a term's Hill flag in shared memory
-
-size_t rk4_block(int S, int nterms) {
-    return sizeof(double) * (4 * S + 6) * RC + nterms * (sizeof(int4) + sizeof(double4)) + sizeof(int32_t) * (S + 1);
-}
-
+// steps of 8 nodes: 300 cells 111 -> 49 us, 1,260 cells 115 -> 51, 16,000 cells
+// 163 -> 72; 8 steps: 137,000 cells 452 -> 346, 40,000 cells of 16 nodes 693 ->
+// 380, of 32 nodes 5,959 -> 1,204.  Five blocks of 8 warps an SM (48 registers a
+// thread, a few of the power's spilled; four blocks spill next to none and take
+// 445 us where five take 380).
 template <int G, bool CLONES>
 __global__ void __launch_bounds__(32 * G, 40 / G)
     k_rk4(NetDev N, const NetDev *nets, const int32_t *clone, int S, double *state, const double *inputs,
@@ -76,67 +69,14 @@ __global__ void __launch_bounds__(32 * G, 40 / G)
             ptr = M.node_ptr;
         }
     } else {
-        for (int t = threadIdx.x; t < N.nterms; t += 32 * G) {
-            int4 tm = N.term[t];
-            double4 p = N.par[t];
-            // what a Hill response takes from its term alone is worked out here
-            if (tm.z) {
-                tm.z = p.y == 2.0 ? SQUARE : POWER;
-                p.z = p.y == 2.0 ? p.z * p.z : pow(p.z, p.y);
-            }
-            sterm[t] = tm;
-            spar[t] = p;
-        }
-        for (int t = threadIdx.x; t <= S; t += 32 * G) sptr[t] = N.node_ptr[t];
+        stage_terms(N, sterm, spar, sptr);
     }
     if (live) {
         for (int i = warp; i < S; i += G) xs[i * RC] = state[i * node_stride + c * cell_stride];
-        // read, network.rs:670-680: oxygen and crowding in [0, 1], stress and
-        // the released not below zero
-        for (int q = warp; q < 6; q += G) {
-            double v = inputs[q * in_stride + c * in_cell];
-            if (q == 0 || q == 2) v = fmin(fmax(v, 0.0), 1.0);
-            else if (q >= 3) v = fmax(v, 0.0);
-            in[q * RC] = v;
-        }
+        for (int q = warp; q < 6; q += G) in[q * RC] = clamped_input(q, inputs[q * in_stride + c * in_cell]);
     }
     __syncthreads();
-    // the rate of node i at the values v
-    auto rate_of = [&](const double *v, int i) -> double {
-        const double own = v[i * RC], rest = 1.0 - own;
-        double rate = 0.0;
-        const int end = ptr[i + 1];
-        for (int t = ptr[i]; t < end; ++t) {
-            const int4 tm = term[t];
-            const double4 p = par[t];
-            const double s = tm.y >= 0 ? v[tm.y * RC] : in[min(-1 - tm.y, 5) * RC];
-            const double k = p.x;
-            double r;
-            switch (tm.x) {
-            case CW_ACTIVATED_BY:
-            case CW_INHIBITED_BY: {
-                double drv = s;
-                if (CLONES) {
-                    if (tm.z) drv = hill(s, p.y, p.z);
-                } else if (tm.z) {  // driver, network.rs:56-64, the half's power from the table
-                    const double sp = s > 0.0 ? s : 0.0;
-                    const double sn = tm.z == SQUARE ? sp * sp : pow(sp, p.y);
-                    drv = sn / (p.z + sn);
-                }
-                r = tm.x == CW_ACTIVATED_BY ? k * drv * rest : -k * drv * own;
-                break;
-            }
-            case CW_ACTIVATED_BY_ABSENCE_OF: r = k * (1.0 - s) * rest; break;
-            case CW_PRODUCED_BY: r = k * s; break;
-            case CW_DECAYS: r = -k * own; break;
-            case CW_RELAXES_TO: r = -k * (own - p.w); break;
-            case CW_DAMAGED_BELOW: r = -k * fmax((p.w - s) / p.w, 0.0); break;
-            default: r = -k * fmax((s - p.w) / p.w, 0.0); break;
-            }
-            rate += r;
-        }
-        return rate;
-    };
+    auto rate_of = [&](const double *v, int i) { return node_rate<CLONES>(term, par, ptr, v, in, i); };
     for (int sub = 0; sub < substeps; ++sub) {
         // k1 at x, k2 at x + dt/2 k1, k3 at x + dt/2 k2, k4 at x + dt k3
         if (live)

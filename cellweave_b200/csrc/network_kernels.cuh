@@ -104,4 +104,76 @@ __device__ __forceinline__ void derivatives(const NetDev &N, const int4 *sterm, 
     }
 }
 
+// ------------------------------------------------------------------ a lane per cell, a cell's nodes over warps
+constexpr int RC = 32;           // cells per block: the stride of a column
+enum { SQUARE = 2, POWER = 3 };  // a staged term's Hill flag
+
+// read, network.rs:670-680: oxygen and crowding in [0, 1], stress and the
+// released not below zero.
+__device__ __forceinline__ double clamped_input(int q, double v) {
+    return q == 0 || q == 2 ? fmin(fmax(v, 0.0), 1.0) : q >= 3 ? fmax(v, 0.0) : v;
+}
+
+// A network's terms into shared memory, what a Hill response takes from its
+// term alone worked out: the flag says how s is raised, par.z is the half's power.
+__device__ __forceinline__ void stage_terms(const NetDev &N, int4 *sterm, double4 *spar, int32_t *sptr) {
+    for (int t = threadIdx.x; t < N.nterms; t += blockDim.x) {
+        int4 tm = N.term[t];
+        double4 p = N.par[t];
+        if (tm.z) {
+            tm.z = p.y == 2.0 ? SQUARE : POWER;
+            p.z = p.y == 2.0 ? p.z * p.z : pow(p.z, p.y);
+        }
+        sterm[t] = tm;
+        spar[t] = p;
+    }
+    for (int t = threadIdx.x; t <= N.S; t += blockDim.x) sptr[t] = N.node_ptr[t];
+}
+
+// A term's source from the lane's columns: node values v, clamped inputs in.
+__device__ __forceinline__ double source_of(const int4 &tm, const double *v, const double *in) {
+    return tm.y >= 0 ? v[tm.y * RC] : in[min(-1 - tm.y, 5) * RC];
+}
+
+// The rate of node i at the lane's values v (derivatives and term_rate,
+// network.rs:686-734), its terms added in file order; RAW: tables as compiled,
+// else as stage_terms leaves them.
+template <bool RAW>
+__device__ __forceinline__ double node_rate(const int4 *term, const double4 *par, const int32_t *ptr, const double *v,
+                                            const double *in, int i) {
+    const double own = v[i * RC], rest = 1.0 - own;
+    double rate = 0.0;
+    const int end = ptr[i + 1];
+    for (int t = ptr[i]; t < end; ++t) {
+        const int4 tm = term[t];
+        const double4 p = par[t];
+        const double s = source_of(tm, v, in);
+        const double k = p.x;
+        double r;
+        switch (tm.x) {
+        case CW_ACTIVATED_BY:
+        case CW_INHIBITED_BY: {
+            double drv = s;
+            if (RAW) {
+                if (tm.z) drv = hill(s, p.y, p.z);
+            } else if (tm.z) {  // driver, network.rs:56-64
+                const double sp = s > 0.0 ? s : 0.0;
+                const double sn = tm.z == SQUARE ? sp * sp : pow(sp, p.y);
+                drv = sn / (p.z + sn);
+            }
+            r = tm.x == CW_ACTIVATED_BY ? k * drv * rest : -k * drv * own;
+            break;
+        }
+        case CW_ACTIVATED_BY_ABSENCE_OF: r = k * (1.0 - s) * rest; break;
+        case CW_PRODUCED_BY: r = k * s; break;
+        case CW_DECAYS: r = -k * own; break;
+        case CW_RELAXES_TO: r = -k * (own - p.w); break;
+        case CW_DAMAGED_BELOW: r = -k * fmax((p.w - s) / p.w, 0.0); break;
+        default: r = -k * fmax((s - p.w) / p.w, 0.0); break;
+        }
+        rate += r;
+    }
+    return rate;
+}
+
 }  // namespace cw

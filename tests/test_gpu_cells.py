@@ -59,3 +59,63 @@ def test_every_split_of_a_cells_nodes_gives_the_same_bits(S, most):
     O.network_step(ref, want, np.ascontiguousarray(ins[pick]), 0.05, 3)
     # CUDA's pow is within 2 ulp of libm's; three steps of four evaluations
     np.testing.assert_allclose(whole[pick], want, rtol=1e-12, atol=1e-14)
+
+
+def torch_steps(spec, x, ins, rates, dt, steps):
+    """rk4 of step_batch on torch float64 tensors, for autograd."""
+    import torch
+
+    read = {"oxygen": ins[:, 0].clamp(0, 1), "egf": ins[:, 1], "crowding": ins[:, 2].clamp(0, 1)}
+    read.update({s: ins[:, q].clamp(min=0) for q, s in enumerate(SOURCES) if q > 2})
+
+    def f(z):
+        out, t = [], 0
+        for i, node in enumerate(spec["nodes"]):
+            own, rate = z[:, i], torch.zeros_like(z[:, 0])
+            for term in node["terms"]:
+                k, kind, src = rates[t], term["kind"], term.get("source")
+                t += 1
+                s = None if src is None else read[src] if src in read else z[:, int(src[1:])]
+                if "hill" in term:
+                    n, half = term["hill"]["n"], term["hill"]["k"]
+                    sn = s.clamp(min=0) ** n
+                    s = sn / (half ** n + sn)
+                th = term.get("threshold", 1.0)
+                rate = rate + {"activated_by": lambda: k * s * (1 - own), "inhibited_by": lambda: -k * s * own,
+                               "activated_by_absence_of": lambda: k * (1 - s) * (1 - own),
+                               "produced_by": lambda: k * s, "decays": lambda: -k * own,
+                               "relaxes_to": lambda: -k * (own - term["value"]),
+                               "damaged_below": lambda: -k * ((th - s) / th).clamp(min=0),
+                               "damaged_above": lambda: -k * ((s - th) / th).clamp(min=0)}[kind]()
+            out.append(rate)
+        return torch.stack(out, 1)
+
+    for _ in range(steps):
+        k1 = f(x)
+        k2 = f(x + 0.5 * dt * k1)
+        k3 = f(x + 0.5 * dt * k2)
+        k4 = f(x + dt * k3)
+        x = (x + dt / 6 * (k1 + 2 * k2 + 2 * k3 + k4)).clamp(0, 1)
+    return x
+
+
+# one cell, a block and one more; a block's last warp without a node (7), the
+# oxygen's list on the first warp (8) and past the sixteenth (17)
+@pytest.mark.parametrize("S,n,steps", [(1, 1, 1), (7, 33, 3), (8, 32, 2), (9, 65, 3), (17, 40, 2), (32, 31, 2)])
+def test_the_backward_step_is_the_derivative_of_the_forward(S, n, steps):
+    import torch
+
+    spec = spec_of(S)
+    net = cw.Network.from_spec(spec, 64)
+    rng = np.random.default_rng(7)
+    st, (_, ins) = rng.uniform(0.2, 0.8, (n, S)), cells_of(n, S)
+    w = rng.normal(size=(n, S))
+    flat = [t["rate"] for nd in spec["nodes"] for t in nd["terms"]]
+    nr = min(len(flat), 32)
+    adj, d_o2, d_rates = net.backward_batch(st, ins, 0.02, steps, w, nrates=nr)
+    x, i, k = (torch.tensor(v, dtype=torch.float64, requires_grad=True) for v in (st, ins, flat))
+    (torch_steps(spec, x, i, k, 0.02, steps) * torch.tensor(w)).sum().backward()
+    # float64 throughout: a few hundred roundings of 1e-16 of numbers up to some tens
+    np.testing.assert_allclose(adj, x.grad.numpy(), rtol=1e-10, atol=1e-12)
+    np.testing.assert_allclose(d_o2, i.grad.numpy()[:, 0], rtol=1e-10, atol=1e-12)
+    np.testing.assert_allclose(d_rates, k.grad.numpy()[:nr], rtol=1e-10, atol=1e-12 * n)
