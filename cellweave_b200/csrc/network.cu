@@ -22,6 +22,11 @@ const char *INPUTS[6] = {"oxygen", "egf", "crowding", "stress", "waste", "necrot
 
 constexpr int MAXS = 32;
 
+// Shared bytes of a k_rk4 block.
+size_t rk4_block(int S, int nterms) {
+    return sizeof(double) * (4 * S + 6) * RC + nterms * (sizeof(int4) + sizeof(double4)) + sizeof(int32_t) * (S + 1);
+}
+
 // RK4 with a block per 32 cells (rk4, derivatives and term_rate,
 // network.rs:686-799): a lane per cell, the nodes dealt to the block's G warps.
 // Every lane of a warp is at the same node, so a warp never diverges by kind of
