@@ -834,49 +834,28 @@ extern "C" int cw_network_backward_batch(cw_network net, int64_t ncells, const d
         for (int32_t t = 0; t < nrates; ++t) d_rates[t] = 0.0;
         return CW_OK;
     }
-    const int64_t nc = ncells, S = net->S;
-    // cell-major host arrays to node-major device columns
-    std::vector<double> xs(S * nc), in(6 * nc), lam(S * nc);
-    for (int64_t c = 0; c < nc; ++c) {
-        for (int64_t i = 0; i < S; ++i) {
-            xs[i * nc + c] = state[c * S + i];
-            lam[i * nc + c] = adjoint[c * S + i];
-        }
-        for (int q = 0; q < 6; ++q) in[q * nc + c] = inputs[c * 6 + q];
-    }
-    double *d_x = nullptr, *d_in = nullptr, *d_seg = nullptr, *d_lam = nullptr, *d_gin = nullptr, *d_gth = nullptr;
-    auto release = [&]() { dfree(d_x); dfree(d_in); dfree(d_seg); dfree(d_lam); dfree(d_gin); dfree(d_gth); };
-    int rc;
-    if ((rc = dalloc(&d_x, S * nc)) || (rc = dalloc(&d_in, 6 * nc)) || (rc = dalloc(&d_seg, substeps * S * nc)) ||
-        (rc = dalloc(&d_lam, S * nc)) || (rc = dalloc(&d_gin, nc)) || (rc = dalloc(&d_gth, MAXTH))) {
-        release();
-        return rc;
-    }
-    CW_CUDA(cudaMemcpyAsync(d_x, xs.data(), sizeof(double) * S * nc, cudaMemcpyHostToDevice, stream()));
-    CW_CUDA(cudaMemcpyAsync(d_in, in.data(), sizeof(double) * 6 * nc, cudaMemcpyHostToDevice, stream()));
-    CW_CUDA(cudaMemcpyAsync(d_lam, lam.data(), sizeof(double) * S * nc, cudaMemcpyHostToDevice, stream()));
-    CW_CUDA(cudaMemsetAsync(d_gin, 0, sizeof(double) * nc, stream()));
-    CW_CUDA(cudaMemsetAsync(d_gth, 0, sizeof(double) * MAXTH, stream()));
-    if (backward_fits(net->S, net->nterms) != CW_OK) {
-        release();
+    if (backward_fits(net->S, net->nterms) != CW_OK)
         return fail(CW_ERR_CONFIG, "the network is too large for the backward step's shared memory");
-    }
+    // rows as the caller has them, [cell][node], in memory the network keeps
+    const int64_t nc = ncells, S = net->S;
+    CellLease mem(net->cells);
+    int rc;
+    if ((rc = mem.take((size_t)(nc * (2 * S + 7 + substeps * S) + MAXTH))) != CW_OK) return rc;
+    double *d_x = mem.p, *d_lam = d_x + S * nc, *d_in = d_lam + S * nc, *d_gin = d_in + 6 * nc, *d_gth = d_gin + nc,
+           *d_seg = d_gth + MAXTH;
+    CW_CUDA(cudaMemcpyAsync(d_x, state, sizeof(double) * S * nc, cudaMemcpyHostToDevice, stream()));
+    CW_CUDA(cudaMemcpyAsync(d_in, inputs, sizeof(double) * 6 * nc, cudaMemcpyHostToDevice, stream()));
+    CW_CUDA(cudaMemcpyAsync(d_lam, adjoint, sizeof(double) * S * nc, cudaMemcpyHostToDevice, stream()));
+    CW_CUDA(cudaMemsetAsync(d_gin, 0, sizeof(double) * (nc + MAXTH), stream()));
     NetDev N{net->node_ptr, net->term, net->par, net->S, net->nterms};
-    if ((rc = backward_launch(N, d_x, d_in, nc, nc, 1, nc, 1, substeps, dt, d_seg, d_lam, d_gin, d_gth, nrates)) !=
-        CW_OK) {
-        release();
+    if ((rc = backward_launch(N, d_x, d_in, nc, 1, S, 1, 6, substeps, dt, d_seg, d_lam, d_gin, d_gth, nrates)) != CW_OK)
         return rc;
-    }
-    std::vector<double> gin(nc), gth(MAXTH);
-    CW_CUDA(cudaMemcpyAsync(lam.data(), d_lam, sizeof(double) * S * nc, cudaMemcpyDeviceToHost, stream()));
-    CW_CUDA(cudaMemcpyAsync(gin.data(), d_gin, sizeof(double) * nc, cudaMemcpyDeviceToHost, stream()));
-    CW_CUDA(cudaMemcpyAsync(gth.data(), d_gth, sizeof(double) * MAXTH, cudaMemcpyDeviceToHost, stream()));
-    CW_CUDA(cudaStreamSynchronize(stream()));
-    release();
-    for (int64_t c = 0; c < nc; ++c)
-        for (int64_t i = 0; i < S; ++i) adjoint[c * S + i] = lam[i * nc + c];
+    double gth[MAXTH];
+    CW_CUDA(cudaMemcpyAsync(adjoint, d_lam, sizeof(double) * S * nc, cudaMemcpyDeviceToHost, stream()));
     if (d_oxygen)
-        for (int64_t c = 0; c < nc; ++c) d_oxygen[c] = gin[c];
+        CW_CUDA(cudaMemcpyAsync(d_oxygen, d_gin, sizeof(double) * nc, cudaMemcpyDeviceToHost, stream()));
+    CW_CUDA(cudaMemcpyAsync(gth, d_gth, sizeof(double) * MAXTH, cudaMemcpyDeviceToHost, stream()));
+    CW_CUDA(cudaStreamSynchronize(stream()));
     for (int32_t t = 0; t < nrates; ++t) d_rates[t] = gth[t];
     return CW_OK;
 }

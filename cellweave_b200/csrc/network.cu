@@ -382,7 +382,7 @@ int cw_network_compile(int32_t nnodes, const char *const *names, const double *i
 int cw_network_destroy(cw_network n) {
     if (!n) return CW_OK;
     CW_SCOPE(n);
-    dfree(n->node_ptr); dfree(n->term); dfree(n->par);
+    dfree(n->node_ptr); dfree(n->term); dfree(n->par); dfree(n->cells.p);
     n->hs.release();
     delete n;
     return CW_OK;
@@ -405,31 +405,26 @@ int cw_network_info(cw_network n, int32_t *nnodes, int32_t *roles7, double *init
     return CW_OK;
 }
 
+// The rows of a batch stay as the caller has them, [cell][node]: they are copied
+// as they are and the kernel reads them at that stride (the transposes on the
+// host and the allocations of each call took 3.3 of 4.0 ms for 40,000 cells of 16
+// nodes, the kernel 0.7).
 int cw_network_step_batch(cw_network n, int64_t ncells, double *state, const double *inputs, double dt,
                           int32_t substeps) {
     CW_SCOPE(n);
     if (ncells <= 0) return CW_OK;
     const int S = n->S;
-    double *d_state, *d_in;
+    CellLease mem(n->cells);
     int rc;
-    if ((rc = dalloc(&d_state, (size_t)ncells * S)) || (rc = dalloc(&d_in, (size_t)ncells * 6))) return rc;
-    // host rows are [cell][node]; the device works node-major
-    std::vector<double> t((size_t)ncells * (S > 6 ? S : 6));
-    for (int64_t c = 0; c < ncells; ++c)
-        for (int i = 0; i < S; ++i) t[(size_t)i * ncells + c] = state[c * S + i];
-    CW_CUDA(cudaMemcpyAsync(d_state, t.data(), sizeof(double) * ncells * S, cudaMemcpyHostToDevice, stream()));
-    CW_CUDA(cudaStreamSynchronize(stream()));
-    for (int64_t c = 0; c < ncells; ++c)
-        for (int q = 0; q < 6; ++q) t[(size_t)q * ncells + c] = inputs[c * 6 + q];
-    CW_CUDA(cudaMemcpyAsync(d_in, t.data(), sizeof(double) * ncells * 6, cudaMemcpyHostToDevice, stream()));
-    if ((rc = network_step_device(n, d_state, d_in, ncells, ncells, ncells, dt, substeps, nullptr)) != CW_OK)
+    if ((rc = mem.take((size_t)ncells * (S + 6))) != CW_OK) return rc;
+    double *d_state = mem.p, *d_in = d_state + ncells * S;
+    CW_CUDA(cudaMemcpyAsync(d_state, state, sizeof(double) * ncells * S, cudaMemcpyHostToDevice, stream()));
+    CW_CUDA(cudaMemcpyAsync(d_in, inputs, sizeof(double) * ncells * 6, cudaMemcpyHostToDevice, stream()));
+    if ((rc = rk4_cells(net_dev(n), nullptr, nullptr, S, d_state, d_in, ncells, 1, S, 1, 6, dt, substeps, nullptr)) !=
+        CW_OK)
         return rc;
-    CW_CUDA(cudaMemcpyAsync(t.data(), d_state, sizeof(double) * ncells * S, cudaMemcpyDeviceToHost, stream()));
+    CW_CUDA(cudaMemcpyAsync(state, d_state, sizeof(double) * ncells * S, cudaMemcpyDeviceToHost, stream()));
     CW_CUDA(cudaStreamSynchronize(stream()));
-    for (int64_t c = 0; c < ncells; ++c)
-        for (int i = 0; i < S; ++i) state[c * S + i] = t[(size_t)i * ncells + c];
-    dfree(d_state);
-    dfree(d_in);
     return CW_OK;
 }
 
@@ -533,36 +528,23 @@ int cw_network_step_clones(int32_t nnets, const cw_network *nets, int64_t ncells
         if (clone[c] < 0 || clone[c] >= nnets)
             return fail(CW_ERR_CONFIG, "cell " + std::to_string(c) + " names network " + std::to_string(clone[c]) +
                                            " of " + std::to_string(nnets));
-    NetDev *d_nets;
-    int32_t *d_clone;
-    double *d_state, *d_in;
+    CellLease mem(nets[0]->cells);
+    const size_t nets_at = (size_t)ncells * (S + 6), clone_at = nets_at + (sizeof(NetDev) * nnets + 7) / 8;
     int rc;
-    if ((rc = dalloc(&d_nets, (size_t)nnets)) || (rc = dalloc(&d_clone, (size_t)ncells)) ||
-        (rc = dalloc(&d_state, (size_t)ncells * S)) || (rc = dalloc(&d_in, (size_t)ncells * 6)))
-        return rc;
-    std::vector<double> t((size_t)ncells * (S > 6 ? S : 6));
-    for (int64_t c = 0; c < ncells; ++c)
-        for (int i = 0; i < S; ++i) t[(size_t)i * ncells + c] = state[c * S + i];
-    CW_CUDA(cudaMemcpy(d_state, t.data(), sizeof(double) * ncells * S, cudaMemcpyHostToDevice));
-    for (int64_t c = 0; c < ncells; ++c)
-        for (int q = 0; q < 6; ++q) t[(size_t)q * ncells + c] = inputs[c * 6 + q];
-    CW_CUDA(cudaMemcpy(d_in, t.data(), sizeof(double) * ncells * 6, cudaMemcpyHostToDevice));
-    CW_CUDA(cudaMemcpy(d_nets, dev.data(), sizeof(NetDev) * nnets, cudaMemcpyHostToDevice));
-    CW_CUDA(cudaMemcpy(d_clone, clone, sizeof(int32_t) * ncells, cudaMemcpyHostToDevice));
+    if ((rc = mem.take(clone_at + (size_t)(ncells + 1) / 2)) != CW_OK) return rc;
+    double *d_state = mem.p, *d_in = d_state + ncells * S;
+    NetDev *d_nets = (NetDev *)(mem.p + nets_at);
+    int32_t *d_clone = (int32_t *)(mem.p + clone_at);
+    CW_CUDA(cudaMemcpyAsync(d_state, state, sizeof(double) * ncells * S, cudaMemcpyHostToDevice, stream()));
+    CW_CUDA(cudaMemcpyAsync(d_in, inputs, sizeof(double) * ncells * 6, cudaMemcpyHostToDevice, stream()));
+    CW_CUDA(cudaMemcpyAsync(d_nets, dev.data(), sizeof(NetDev) * nnets, cudaMemcpyHostToDevice, stream()));
+    CW_CUDA(cudaMemcpyAsync(d_clone, clone, sizeof(int32_t) * ncells, cudaMemcpyHostToDevice, stream()));
     NetDev none{};
     none.S = S;
-    if ((rc = rk4_cells(none, d_nets, d_clone, S, d_state, d_in, ncells, ncells, 1, ncells, 1, dt, substeps,
-                        nullptr)) != CW_OK)
+    if ((rc = rk4_cells(none, d_nets, d_clone, S, d_state, d_in, ncells, 1, S, 1, 6, dt, substeps, nullptr)) != CW_OK)
         return rc;
-    CW_CUDA(cudaGetLastError());
-    CW_CUDA(cudaMemcpyAsync(t.data(), d_state, sizeof(double) * ncells * S, cudaMemcpyDeviceToHost, stream()));
+    CW_CUDA(cudaMemcpyAsync(state, d_state, sizeof(double) * ncells * S, cudaMemcpyDeviceToHost, stream()));
     CW_CUDA(cudaStreamSynchronize(stream()));
-    for (int64_t c = 0; c < ncells; ++c)
-        for (int i = 0; i < S; ++i) state[c * S + i] = t[(size_t)i * ncells + c];
-    dfree(d_nets);
-    dfree(d_clone);
-    dfree(d_state);
-    dfree(d_in);
     return CW_OK;
 }
 

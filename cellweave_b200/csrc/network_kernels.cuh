@@ -3,10 +3,59 @@
 #pragma once
 
 #include <cmath>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "cw_internal.cuh"
+
+namespace cw {
+
+// A network's device memory for the batches of cells that come from the host:
+// kept up to KEPT bytes, given back with the network.  One call at a time has it;
+// a call that finds it taken (another thread's on the same network), or that needs
+// more, allocates its own for its own time.
+struct CellSpace {
+    static constexpr size_t KEPT = (size_t)64 << 20;
+    std::mutex mu;
+    double *p = nullptr;
+    size_t bytes = 0;
+};
+class CellLease {
+  public:
+    explicit CellLease(CellSpace &s) : s_(s), lock_(s.mu, std::try_to_lock) {}
+    CellLease(const CellLease &) = delete;
+    CellLease &operator=(const CellLease &) = delete;
+    // what the call queued is over before the memory is another's
+    ~CellLease() {
+        if (p) cudaStreamSynchronize(stream());
+        dfree(own_);
+    }
+    int take(size_t numbers) {
+        const size_t bytes = numbers * sizeof(double);
+        int rc = CW_OK;
+        if (!lock_.owns_lock() || bytes > CellSpace::KEPT) {
+            if ((rc = dalloc(&own_, numbers)) == CW_OK) p = own_;
+            return rc;
+        }
+        if (bytes > s_.bytes) {
+            dfree(s_.p);
+            s_.bytes = 0;
+            if ((rc = dalloc(&s_.p, numbers)) != CW_OK) return rc;
+            s_.bytes = bytes;
+        }
+        p = s_.p;
+        return CW_OK;
+    }
+    double *p = nullptr;
+
+  private:
+    CellSpace &s_;
+    std::unique_lock<std::mutex> lock_;
+    double *own_ = nullptr;
+};
+
+}  // namespace cw
 
 struct cw_network_s {
     cw::HandleStream hs;  // its stream and last error
@@ -25,6 +74,7 @@ struct cw_network_s {
     int32_t *node_ptr = nullptr;  // S + 1
     int4 *term = nullptr;         // (kind, source, has_hill, 0)
     double4 *par = nullptr;       // (rate, hill_n, hill_k, param)
+    cw::CellSpace cells;
 };
 
 namespace cw {

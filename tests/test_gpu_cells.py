@@ -119,3 +119,34 @@ def test_the_backward_step_is_the_derivative_of_the_forward(S, n, steps):
     np.testing.assert_allclose(adj, x.grad.numpy(), rtol=1e-10, atol=1e-12)
     np.testing.assert_allclose(d_o2, i.grad.numpy()[:, 0], rtol=1e-10, atol=1e-12)
     np.testing.assert_allclose(d_rates, k.grad.numpy()[:nr], rtol=1e-10, atol=1e-12 * n)
+
+
+# the memory a network keeps: grown, shrunk into, past what is kept (64 MB), and
+# taken by two threads at a time
+def test_batches_of_any_size_share_a_networks_memory():
+    import threading
+
+    S = 8
+    net = cw.Network.from_spec(spec_of(S), 64)
+    st, ins = cells_of(650_000, S)
+
+    def step(n):
+        x = st[:n].copy()
+        return net.step_batch(x, ins[:n], 0.05, 1)
+
+    whole = step(650_000)
+    for n in (10, 40_000, 1, 650_000, 33):
+        np.testing.assert_array_equal(step(n).view(np.uint64), whole[:n].view(np.uint64))
+    out = {}
+
+    def many(k):
+        out[k] = [step(2_000 * (k + 1)) for _ in range(10)]
+
+    threads = [threading.Thread(target=many, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(4):
+        for x in out[k]:
+            np.testing.assert_array_equal(x.view(np.uint64), whole[:2_000 * (k + 1)].view(np.uint64))
