@@ -45,24 +45,9 @@ __global__ void k_span(const uint8_t *__restrict__ held, const int4 *dims, const
     bool ok = local < n && !held[off[h] + local];
     int x = 0, y = 0, z = 0;
     if (ok) locate(dims[h], local, x, y, z);
-    // warp-level reduction first, then one atomic per warp
-    int xmin = ok ? x : INT_MAX, xmax = ok ? x : -1, ymin = ok ? y : INT_MAX, ymax = ok ? y : -1;
-    int zmin = ok ? z : INT_MAX, zmax = ok ? z : -1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        xmin = min(xmin, __shfl_xor_sync(0xffffffffu, xmin, o));
-        xmax = max(xmax, __shfl_xor_sync(0xffffffffu, xmax, o));
-        ymin = min(ymin, __shfl_xor_sync(0xffffffffu, ymin, o));
-        ymax = max(ymax, __shfl_xor_sync(0xffffffffu, ymax, o));
-        zmin = min(zmin, __shfl_xor_sync(0xffffffffu, zmin, o));
-        zmax = max(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
-    }
-    if ((threadIdx.x & 31) == 0 && xmax >= 0) {
-        atomicMin(&span[h].x0, xmin); atomicMax(&span[h].x1, xmax);
-        atomicMin(&span[h].y0, ymin); atomicMax(&span[h].y1, ymax);
-        atomicMin(&span[h].z0, zmin); atomicMax(&span[h].z1, zmax);
-        span[h].found = 1;
-    }
+    int box[6] = {ok ? x : INT_MAX, ok ? x : -1, ok ? y : INT_MAX, ok ? y : -1, ok ? z : INT_MAX, ok ? z : -1};
+    span_into<true>(box, &span[h].x0);
+    if (__syncthreads_or(ok) && threadIdx.x == 0) span[h].found = 1;
 }
 
 __global__ void k_span_reset(Span *span, int nh) {

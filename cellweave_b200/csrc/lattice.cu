@@ -532,26 +532,17 @@ __global__ void k_span_occupied(const int32_t *grid, const int4 *dims, const int
     const int4 dm = dims[h];
     if (dm.z <= 1) return;  // the whole block: a plane visits its whole box
     const int64_t local = (int64_t)(blockIdx.x - blk[h]) * blockDim.x + threadIdx.x;
-    int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, mx[3] = {-1, -1, -1};
+    int box[6] = {0x7fffffff, -1, 0x7fffffff, -1, 0x7fffffff, -1};
     if (local < off[h + 1] - off[h] && grid[off[h] + local] != 0) {
         const int64_t slice = (int64_t)dm.x * dm.y;
         const int z = (int)(local / slice);
         const int64_t r = local - (int64_t)z * slice;
         const int y = (int)(r / dm.x), x = (int)(r - (int64_t)y * dm.x);
-        mn[0] = mx[0] = x;
-        mn[1] = mx[1] = y;
-        mn[2] = mx[2] = z;
+        box[0] = box[1] = x;
+        box[2] = box[3] = y;
+        box[4] = box[5] = z;
     }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
-        mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
-    }
-    if ((threadIdx.x & 31) == 0 && mx[0] >= 0)
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(span + 6 * h + a, mn[a]);
-            atomicMax(span + 6 * h + 3 + a, mx[a]);
-        }
+    span_into<false>(box, span + 6 * h);
 }
 __global__ void k_span_finish(int32_t *span, const int4 *dims, int nh) {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
