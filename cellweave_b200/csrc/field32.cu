@@ -537,10 +537,14 @@ __device__ __forceinline__ void copy_async(uint32_t to, const float *from, bool 
                      : "memory");
 }
 
-// FULL: VD half-sweeps, neither a first launch nor a last one (most of a
-// correction's launches: without the other cases' code the unrolled steps fit
-// the instruction cache; 89 -> 62 us a sweep of 256^3 before the ring).
-template <int NW, int ALIGN, bool FULL>
+// What a launch is, known at compile time: VD half-sweeps in the middle of a
+// correction, its first launch (from zero) or its last (the correction added to
+// the field); ANY: told at run time, for a launch of fewer half-sweeps.  Without
+// the other cases' code the unrolled steps fit the instruction cache (89 -> 62
+// us a sweep of 256^3 before the ring; the first and last launch of a
+// correction, both ANY before, 115 us on average, now 51 and 132).
+enum VolKind { VOL_ANY, VOL_MIDDLE, VOL_FIRST, VOL_LAST };
+template <int NW, int ALIGN, int KIND>
 __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
     k_sor32_vol(const float *__restrict__ src, float *__restrict__ dst, const float *__restrict__ rhs,
                 const float *__restrict__ inv, const int4 *__restrict__ dims, const int64_t *__restrict__ off,
@@ -564,11 +568,9 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
     const int x0 = tl.y, y0 = tl.z, z0 = tl.w;
     const int z1 = min(z0 + vz, dm.z);
     const int zlo = max(z0 - D, 0), zhi = min(z1 + D, dm.z);
-    const int S = FULL ? D : nhalf;
-    if (FULL) {
-        zero_start = 0;
-        apply_c = nullptr;
-    }
+    const int S = KIND != VOL_ANY ? D : nhalf;
+    if (KIND != VOL_ANY) zero_start = KIND == VOL_FIRST;
+    if (KIND == VOL_MIDDLE || KIND == VOL_FIRST) apply_c = nullptr;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gx = x0 + 2 * lane, gy = y0 + 2 * warp;
     // offsets inside the history in 32 bits (a history holds fewer than 2^31
@@ -577,7 +579,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
     const int64_t base = off[h];
     const float *const from[3] = {src + base, rhs + base, inv + base};
     float *hdst = dst + base;
-    double *hc = apply_c ? apply_c + base : nullptr;
+    double *hc = KIND == VOL_LAST || apply_c ? apply_c + base : nullptr;
     const float omc = 1.f - omega[h];
     const float lm = lane == 0 ? 0.f : 1.f, rm = lane == 31 ? 0.f : 1.f;
     // the output interior of the tile (a window edge on the history's border makes no error)
@@ -641,6 +643,12 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
             asm volatile("cp.async.wait_group %0;" ::"n"(NS - 3) : "memory");
             __syncthreads();
             fetch(t + NS - 1, (K + NS - 1) % NS);
+            // the field's slice that leaves D - 1 steps from now, into L2
+            if (KIND == VOL_LAST && t >= z0 && t < z1) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    if (out0[j]) asm volatile("prefetch.global.L2 [%0];" ::"l"(hc + t * plane + (gy + j) * dm.x + gx));
+            }
             take((K + 1) % NS, v[(K + 1) % NS], b[(K + 1) % NS], a[(K + 1) % NS]);
             // the pixels above and below as loaded, for the first stage
             float above0 = 0.f, below0 = 0.f;
@@ -689,10 +697,23 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
                     for (int j = 0; j < 2; ++j) {
                         const int i = pf * plane + (gy + j) * dm.x + gx;
                         const float2 q = v[p][j];
-                        if (hc) {
+                        if (KIND == VOL_LAST || hc) {
                             // the last launch of a correction: c += d on the free
                             // pixels (a held pixel has a = 0 and d = 0 throughout),
                             // floored as the reference's update is (pde.rs:395)
+                            if (ALIGN >= 8 && out0[j] && out1[j]) {
+                                double2 c = *(const double2 *)(hc + i);
+                                if (q.x != 0.f || a[p][j].x != 0.f) {
+                                    c.x = c.x + (double)q.x;
+                                    if (floor) c.x = fmax(c.x, 0.0);
+                                }
+                                if (q.y != 0.f || a[p][j].y != 0.f) {
+                                    c.y = c.y + (double)q.y;
+                                    if (floor) c.y = fmax(c.y, 0.0);
+                                }
+                                *(double2 *)(hc + i) = c;
+                                continue;
+                            }
                             if (out0[j] && (q.x != 0.f || a[p][j].x != 0.f)) {
                                 const double c = hc[i] + (double)q.x;
                                 hc[i] = floor ? fmax(c, 0.0) : c;
@@ -743,14 +764,19 @@ WideKernel wide_kernel_of(int depth) {
 typedef void (*VolKernel)(const float *, float *, const float *, const float *, const int4 *, const int64_t *,
                           const int4 *, int, const float *, const int32_t *, int, int, int, double *, int);
 
-template <int NW, bool FULL>
+template <int NW, int KIND>
 VolKernel vol_kernel_of(int align) {
-    return align == 16 ? k_sor32_vol<NW, 16, FULL> : align == 8 ? k_sor32_vol<NW, 8, FULL> : k_sor32_vol<NW, 4, FULL>;
+    return align == 16 ? k_sor32_vol<NW, 16, KIND> : align == 8 ? k_sor32_vol<NW, 8, KIND> : k_sor32_vol<NW, 4, KIND>;
 }
-
-VolKernel vol_kernel(int vy, int align, bool full) {
-    return vy == 16 ? (full ? vol_kernel_of<8, true>(align) : vol_kernel_of<8, false>(align))
-                    : (full ? vol_kernel_of<16, true>(align) : vol_kernel_of<16, false>(align));
+template <int NW>
+VolKernel vol_kernel_for(int align, int kind) {
+    return kind == VOL_MIDDLE  ? vol_kernel_of<NW, VOL_MIDDLE>(align)
+           : kind == VOL_FIRST ? vol_kernel_of<NW, VOL_FIRST>(align)
+           : kind == VOL_LAST  ? vol_kernel_of<NW, VOL_LAST>(align)
+                               : vol_kernel_of<NW, VOL_ANY>(align);
+}
+VolKernel vol_kernel(int vy, int align, int kind) {
+    return vy == 16 ? vol_kernel_for<8>(align, kind) : vol_kernel_for<16>(align, kind);
 }
 
 WideKernel wide_kernel(int depth, int warps) {
@@ -845,11 +871,11 @@ int vol_init(Sor32 &s, cw_field_s *f, int window) {
     s.vdepth = s.depth >= VD ? VD : 2;
     s.vy = window == CW_WINDOW_64 ? 16 : 32;
     const size_t smem = vol_smem(s.vy / 2);
-    for (bool full : {true, false})
-        CW_CUDA(cudaFuncSetAttribute((const void *)vol_kernel(s.vy, s.valign, full),
+    for (int kind : {VOL_ANY, VOL_MIDDLE, VOL_FIRST, VOL_LAST})
+        CW_CUDA(cudaFuncSetAttribute((const void *)vol_kernel(s.vy, s.valign, kind),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0, dev = 0, nsm = 0;
-    CW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)vol_kernel(s.vy, s.valign, true),
+    CW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)vol_kernel(s.vy, s.valign, VOL_MIDDLE),
                                                           16 * s.vy, smem));
     if (per_sm < 1) return CW_OK;  // one half-sweep per launch serves
     CW_CUDA(cudaGetDevice(&dev));
@@ -943,8 +969,12 @@ int Sor32::sweeps(cw_field_s *f, int n, const int32_t *done, int done_stride, fl
             const int dd = remaining < vdepth ? remaining : vdepth;
             // with `apply` the last launch adds its correction to the field
             const bool last = remaining == dd;
-            const bool full = dd == VD && done_half > 0 && !(apply && last);
-            CW_CUDA(launch_after(done_half > 0, vol_kernel(vy, valign, full), nvtiles, 16 * vy, vol_smem(vy / 2),
+            const bool adds = apply && last;
+            const int kind = dd != VD || (adds && done_half == 0) ? VOL_ANY
+                             : adds                              ? VOL_LAST
+                             : done_half == 0                    ? VOL_FIRST
+                                                                 : VOL_MIDDLE;
+            CW_CUDA(launch_after(done_half > 0, vol_kernel(vy, valign, kind), nvtiles, 16 * vy, vol_smem(vy / 2),
                                  stream(), a, b, f->r32, f->inv32, f->g.d_dims, f->g.d_off, vtiles, vz, omega, done,
                                  done_stride, dd, done_half == 0 ? 1 : 0, apply && last ? f->c : nullptr,
                                  f->floor ? 1 : 0));
