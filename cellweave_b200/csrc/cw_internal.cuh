@@ -89,38 +89,6 @@ const TestFaults &test_faults();
         if (e_ != cudaSuccess) return ::cw::cuda_fail(e_, "kernel launch"); \
     } while (0)
 
-// ------------------------------------------------------------------ boxes
-// A block's box (lowest and highest x, y and z of each thread's own) into a
-// history's: PAIRS, the bounds of each axis in turn, else the three lowest and
-// then the three highest.  The block's warps reduce theirs first, and
-// six threads then go to memory, with an atomic only where the box there is still
-// smaller: an atomic per warp and bound, all on one line, took 203 us on a 1024^2
-// plane and 103 us on a 256^3 volume, whose reads take 1 and 10.  Call it with
-// the whole block, of up to 1,024 threads.
-template <bool PAIRS>
-__device__ __forceinline__ void span_into(const int (&box)[6], int *span) {
-    __shared__ int s_box[32][6];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)blockDim.x >> 5;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const int v = q & 1 ? __reduce_max_sync(0xffffffffu, box[q]) : __reduce_min_sync(0xffffffffu, box[q]);
-        if (lane == 0) s_box[warp][q] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        const int q = threadIdx.x;
-        int v = s_box[0][q];
-        for (int w = 1; w < warps; ++w) v = q & 1 ? max(v, s_box[w][q]) : min(v, s_box[w][q]);
-        int *to = span + (PAIRS ? q : 3 * (q & 1) + (q >> 1));
-        const int have = __ldcg(to);
-        if (q & 1) {
-            if (v > have) atomicMax(to, v);
-        } else if (v < have) {
-            atomicMin(to, v);
-        }
-    }
-}
-
 // ------------------------------------------------------------------ launches that overlap their beginnings
 // Programmatic dependent launch: a kernel launched with `overlap` begins as
 // soon as every block of the one before it in the stream has passed
@@ -196,6 +164,80 @@ struct Plan {
 
 // The history of block b of a plan (Plan::build lays the table after the prefix).
 __device__ __forceinline__ int plan_history(const int32_t *blk, int nh, int b) { return __ldg(blk + nh + 1 + b); }
+
+// ------------------------------------------------------------------ boxes
+// The box around every history's live pixels, a block per SPAN_BLOCKS blocks of a
+// plan with a pixel a thread (blockDim.x pixels each).  A thread's pixels, then
+// the block's warps, are reduced before six threads go to memory, with an atomic
+// only where the box there is still smaller.  `span`, `stride` integers a
+// history: PAIRS, a Span (each axis' bounds in turn, then whether a pixel was
+// found), else the three lowest and then the three highest.
+// (A pixel a thread and six atomics a warp took 203 us on a plane of 1024^2, now
+// 16, and 58 on a volume of 96^3, now 11: the atomics, all on one line, and the
+// blocks of a few instructions each.)
+constexpr int SPAN_BLOCKS = 8;
+template <bool PAIRS, class Live>
+__device__ __forceinline__ void span_blocks(const int4 *dims, const int64_t *off, const int32_t *blk, int nh,
+                                            int nblocks, int *span, int stride, Live live) {
+    __shared__ int s_h[SPAN_BLOCKS + 1], s_box[32][6];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)blockDim.x >> 5;
+    const int b0 = blockIdx.x * SPAN_BLOCKS;
+    if (threadIdx.x <= SPAN_BLOCKS)
+        s_h[threadIdx.x] =
+            threadIdx.x < SPAN_BLOCKS && b0 + threadIdx.x < nblocks ? plan_history(blk, nh, b0 + threadIdx.x) : -1;
+    __syncthreads();
+    bool on[SPAN_BLOCKS];
+    uint32_t at[SPAN_BLOCKS];  // (a history holds fewer than 2^31 pixels)
+#pragma unroll
+    for (int q = 0; q < SPAN_BLOCKS; ++q) {
+        const int h = s_h[q];
+        on[q] = false;
+        at[q] = 0;
+        if (h < 0) continue;
+        const int64_t local = (int64_t)(b0 + q - blk[h]) * blockDim.x + threadIdx.x;
+        at[q] = (uint32_t)local;
+        on[q] = local < off[h + 1] - off[h] && live(h, off[h] + local);
+    }
+    int box[6] = {INT_MAX, -1, INT_MAX, -1, INT_MAX, -1};
+#pragma unroll
+    for (int q = 0; q < SPAN_BLOCKS; ++q) {
+        const int h = s_h[q];
+        if (h < 0) break;  // the same for the whole block
+        if (on[q]) {
+            const int4 dm = dims[h];
+            const uint32_t r = at[q] / (uint32_t)dm.x, z = r / (uint32_t)dm.y;
+            const int c[3] = {(int)(at[q] - r * (uint32_t)dm.x), (int)(r - z * (uint32_t)dm.y), (int)z};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                box[2 * a] = min(box[2 * a], c[a]);
+                box[2 * a + 1] = max(box[2 * a + 1], c[a]);
+            }
+        }
+        if (s_h[q + 1] == h) continue;
+        // the last of this history's: its box out
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const int v = k & 1 ? __reduce_max_sync(0xffffffffu, box[k]) : __reduce_min_sync(0xffffffffu, box[k]);
+            if (lane == 0) s_box[warp][k] = v;
+            box[k] = k & 1 ? -1 : INT_MAX;
+        }
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            const int k = threadIdx.x;
+            int v = s_box[0][k];
+            for (int w = 1; w < warps; ++w) v = k & 1 ? max(v, s_box[w][k]) : min(v, s_box[w][k]);
+            int *mine = span + (int64_t)h * stride, *to = mine + (PAIRS ? k : 3 * (k & 1) + (k >> 1));
+            const int have = __ldcg(to);
+            if (k & 1) {
+                if (v > have) atomicMax(to, v);
+            } else if (v < have) {
+                atomicMin(to, v);
+            }
+            if (PAIRS && k == 1 && v >= 0) mine[6] = 1;
+        }
+        __syncthreads();
+    }
+}
 
 // ------------------------------------------------------------------ Philox4x32-10
 // Salmon, Moraes, Dror, Shaw, "Parallel random numbers: as easy as 1, 2, 3"

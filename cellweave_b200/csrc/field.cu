@@ -35,19 +35,9 @@ __device__ __forceinline__ void locate(const int4 dm, int64_t local, int &x, int
 
 // The box around every free pixel (free_span, pde.rs:305-320).
 __global__ void k_span(const uint8_t *__restrict__ held, const int4 *dims, const int64_t *off, const int32_t *blk,
-                       int nh, Span *span) {
-    __shared__ int s_h;
-    if (threadIdx.x == 0) s_h = plan_history(blk, nh, blockIdx.x);
-    __syncthreads();
-    int h = s_h;
-    int64_t local = (int64_t)(blockIdx.x - blk[h]) * blockDim.x + threadIdx.x;
-    int64_t n = off[h + 1] - off[h];
-    bool ok = local < n && !held[off[h] + local];
-    int x = 0, y = 0, z = 0;
-    if (ok) locate(dims[h], local, x, y, z);
-    int box[6] = {ok ? x : INT_MAX, ok ? x : -1, ok ? y : INT_MAX, ok ? y : -1, ok ? z : INT_MAX, ok ? z : -1};
-    span_into<true>(box, &span[h].x0);
-    if (__syncthreads_or(ok) && threadIdx.x == 0) span[h].found = 1;
+                       int nh, int nblocks, Span *span) {
+    span_blocks<true>(dims, off, blk, nh, nblocks, &span->x0, sizeof(Span) / sizeof(int32_t),
+                      [&](int, int64_t i) { return !held[i]; });
 }
 
 __global__ void k_span_reset(Span *span, int nh) {
@@ -491,7 +481,8 @@ int field_span(cw_field_s *f, std::vector<Span> &spans) {
     if (rc != CW_OK) return rc;
     k_span_reset<<<(f->g.nh + 63) / 64, 64, 0, stream()>>>(f->d_span, f->g.nh);
     CW_LAUNCHED();
-    k_span<<<p.nblocks, T, 0, stream()>>>(f->held, f->g.d_dims, f->g.d_off, p.d_blk, f->g.nh, f->d_span);
+    k_span<<<(p.nblocks + SPAN_BLOCKS - 1) / SPAN_BLOCKS, T, 0, stream()>>>(f->held, f->g.d_dims, f->g.d_off, p.d_blk,
+                                                                            f->g.nh, p.nblocks, f->d_span);
     CW_LAUNCHED();
     spans.resize(f->g.nh);
     CW_CUDA(cudaMemcpyAsync(spans.data(), f->d_span, sizeof(Span) * f->g.nh, cudaMemcpyDeviceToHost, stream()));

@@ -523,26 +523,11 @@ __global__ void k_span_reset(int32_t *span, int nh) {
         span[6 * h + 3 + a] = -1;
     }
 }
+// (volumes: a plane visits its whole box)
 __global__ void k_span_occupied(const int32_t *grid, const int4 *dims, const int64_t *off, const int32_t *blk, int nh,
-                                int32_t *span) {
-    __shared__ int s_h;
-    if (threadIdx.x == 0) s_h = plan_history(blk, nh, blockIdx.x);
-    __syncthreads();
-    const int h = s_h;
-    const int4 dm = dims[h];
-    if (dm.z <= 1) return;  // the whole block: a plane visits its whole box
-    const int64_t local = (int64_t)(blockIdx.x - blk[h]) * blockDim.x + threadIdx.x;
-    int box[6] = {0x7fffffff, -1, 0x7fffffff, -1, 0x7fffffff, -1};
-    if (local < off[h + 1] - off[h] && grid[off[h] + local] != 0) {
-        const int64_t slice = (int64_t)dm.x * dm.y;
-        const int z = (int)(local / slice);
-        const int64_t r = local - (int64_t)z * slice;
-        const int y = (int)(r / dm.x), x = (int)(r - (int64_t)y * dm.x);
-        box[0] = box[1] = x;
-        box[2] = box[3] = y;
-        box[4] = box[5] = z;
-    }
-    span_into<false>(box, span + 6 * h);
+                                int nblocks, int32_t *span) {
+    span_blocks<false>(dims, off, blk, nh, nblocks, span, 6,
+                       [&](int h, int64_t i) { return dims[h].z > 1 && grid[i] != 0; });
 }
 __global__ void k_span_finish(int32_t *span, const int4 *dims, int nh) {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1503,7 +1488,8 @@ int lattice_span_enqueue(cw_lattice_s *l) {
     const int nh = (int)l->g.nh;
     k_span_reset<<<(nh + 127) / 128, 128, 0, stream()>>>(l->d_span, nh);
     CW_LAUNCHED();
-    k_span_occupied<<<p.nblocks, T, 0, stream()>>>(l->grid, l->g.d_dims, l->g.d_off, p.d_blk, nh, l->d_span);
+    k_span_occupied<<<(p.nblocks + SPAN_BLOCKS - 1) / SPAN_BLOCKS, T, 0, stream()>>>(
+        l->grid, l->g.d_dims, l->g.d_off, p.d_blk, nh, p.nblocks, l->d_span);
     CW_LAUNCHED();
     k_span_finish<<<(nh + 127) / 128, 128, 0, stream()>>>(l->d_span, l->g.d_dims, nh);
     CW_LAUNCHED();
