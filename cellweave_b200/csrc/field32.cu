@@ -40,7 +40,9 @@
 //
 // The narrow kernel (any width): 64 x 64 windows, a lane per column pair,
 // plain loads, one window per block.  Its launches, and the volumes', overlap
-// too: 2.56 -> 2.23 ms the relax of a 1023 x 769 sheet.
+// too: 2.56 -> 2.23 ms the relax of a 1023 x 769 sheet.  Its last launch adds the
+// correction as the others' do (two passes of the update, a colour each, took 12
+// us apiece where one residual takes 11): 2.23 -> 2.14 ms.
 //
 // Between warps, each warp publishes its top and bottom rows in shared memory
 // after every half-sweep (double-buffered, so one barrier per half-sweep).
@@ -89,7 +91,9 @@ __global__ void __launch_bounds__(32 * WARPS) k_sor32_tb(const float *__restrict
                                                          const int64_t *__restrict__ off,
                                                          const int32_t *__restrict__ blk, int nh,
                                                          const float *__restrict__ omega, const int32_t *done,
-                                                         int done_stride, int nhalf, int start_colour) {
+                                                         int done_stride, int nhalf, int zero_start,
+                                                         double *__restrict__ apply_c,
+                                                         const uint8_t *__restrict__ held, int floor) {
     constexpr int IN = WIN - 2 * DEPTH;  // interior side
     // edge rows each warp publishes, double-buffered by half-sweep parity:
     // [buffer][warp][0 top, 1 bottom][column]
@@ -121,8 +125,8 @@ __global__ void __launch_bounds__(32 * WARPS) k_sor32_tb(const float *__restrict
         d0[j] = d1[j] = r0[j] = r1[j] = i0[j] = i1[j] = 0.f;
         if (gy >= 0 && gy < dm.y) {
             const int64_t row = base + (int64_t)gy * dm.x + gx;
-            if (in0) { d0[j] = src[row]; r0[j] = rhs[row]; i0[j] = inv[row]; }
-            if (in1) { d1[j] = src[row + 1]; r1[j] = rhs[row + 1]; i1[j] = inv[row + 1]; }
+            if (in0) { d0[j] = zero_start ? 0.f : src[row]; r0[j] = rhs[row]; i0[j] = inv[row]; }
+            if (in1) { d1[j] = zero_start ? 0.f : src[row + 1]; r1[j] = rhs[row + 1]; i1[j] = inv[row + 1]; }
         }
     }
     auto publish = [&](int buf) {
@@ -141,7 +145,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_sor32_tb(const float *__restrict
         const float ab1 = warp > 0 ? edge[buf][warp - 1][1][2 * lane + 1] : 0.f;
         const float be0 = warp < WARPS - 1 ? edge[buf][warp + 1][0][2 * lane] : 0.f;
         const float be1 = warp < WARPS - 1 ? edge[buf][warp + 1][0][2 * lane + 1] : 0.f;
-        if (((start_colour + s) & 1) == 0)
+        if ((s & 1) == 0)
             half_sweep<0>(d0, d1, r0, r1, i0, i1, ab0, ab1, be0, be1, lm, rm, omc);
         else
             half_sweep<1>(d0, d1, r0, r1, i0, i1, ab0, ab1, be0, be1, lm, rm, omc);
@@ -156,8 +160,22 @@ __global__ void __launch_bounds__(32 * WARPS) k_sor32_tb(const float *__restrict
         if (ey < DEPTH || ey >= DEPTH + IN || gy >= dm.y) continue;
         const int64_t row = base + (int64_t)gy * dm.x + gx;
         const int ex = 2 * lane;
-        if (ex >= DEPTH && ex < DEPTH + IN && gx < dm.x) dst[row] = d0[j];
-        if (ex + 1 >= DEPTH && ex + 1 < DEPTH + IN && gx + 1 < dm.x) dst[row + 1] = d1[j];
+        const bool out0 = ex >= DEPTH && ex < DEPTH + IN && gx < dm.x;
+        const bool out1 = ex + 1 >= DEPTH && ex + 1 < DEPTH + IN && gx + 1 < dm.x;
+        if (apply_c) {
+            // a solve's last launch: c += d on the free pixels
+            if (out0 && !held[row]) {
+                const double c = apply_c[row] + (double)d0[j];
+                apply_c[row] = floor ? fmax(c, 0.0) : c;
+            }
+            if (out1 && !held[row + 1]) {
+                const double c = apply_c[row + 1] + (double)d1[j];
+                apply_c[row + 1] = floor ? fmax(c, 0.0) : c;
+            }
+            continue;
+        }
+        if (out0) dst[row] = d0[j];
+        if (out1) dst[row + 1] = d1[j];
     }
 }
 
@@ -737,7 +755,8 @@ __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
 }
 
 typedef void (*TbKernel)(const float *, float *, const float *, const float *, const int4 *, const int64_t *,
-                         const int32_t *, int, const float *, const int32_t *, int, int, int);
+                         const int32_t *, int, const float *, const int32_t *, int, int, int, double *,
+                         const uint8_t *, int);
 typedef void (*WideKernel)(const CUtensorMap *, int, float *, const int4 *, int, const int4 *, const int64_t *,
                            const float *, const int32_t *, int, int, int, double *, int, unsigned long long,
                            int, unsigned long long *, int);
@@ -955,7 +974,8 @@ int Sor32::init(cw_field_s *f, int d, const std::vector<double> &om, int window)
 
 int Sor32::sweeps(cw_field_s *f, int n, const int32_t *done, int done_stride, float *start, bool apply,
                   unsigned long long *corr, int corr_stride) {
-    if (apply && !wide && !vol) return fail(CW_ERR_CONFIG, "only the wide and volume FP32 kernels apply their correction");
+    if (apply && !wide && !vol && !blocked) 
+        return fail(CW_ERR_CONFIG, "one half-sweep per launch applies no correction");
     if (start) {  // begin from this (zeroed) buffer; the other is scratch
         ping = start;
         pong = start == f->d32a ? f->d32b : f->d32a;
@@ -1017,7 +1037,8 @@ int Sor32::sweeps(cw_field_s *f, int n, const int32_t *done, int done_stride, fl
         } else {
             CW_CUDA(launch_after(done_half > 0, tb_kernel(depth), tiles.nblocks, 32 * WARPS, 0, stream(), a, b,
                                  f->r32, f->inv32, f->g.d_dims, f->g.d_off, tiles.d_blk, f->g.nh, omega, done,
-                                 done_stride, dd, done_half & 1));
+                                 done_stride, dd, done_half == 0 ? 1 : 0, apply && remaining == dd ? f->c : nullptr,
+                                 f->held, f->floor ? 1 : 0));
         }
         CW_LAUNCHED();
         remaining -= dd;

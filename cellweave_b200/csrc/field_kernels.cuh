@@ -98,7 +98,7 @@ struct Sor32 {
     float *ping = nullptr, *pong = nullptr, *out = nullptr;
     int init(cw_field_s *f, int depth, const std::vector<double> &omega_per_history, int window = CW_WINDOW_AUTO);
     // n sweeps from the zeroed correction buffer `start` (or the last result);
-    // `apply` (wide only): the last launch adds the correction to the field's
+    // `apply` (blocked sweeps): the last launch adds the correction to the field's
     // values instead of writing it, and result() is null
     // corr (optional, apply only): per history, with stride corr_stride, the
     // largest |correction| the launch added, as the bits of a non-negative
