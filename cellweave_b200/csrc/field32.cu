@@ -27,7 +27,7 @@
 // and at y = k (64 - 2 DEPTH).
 //
 // What bounds it: at depth 8 the four sweeps' own instructions, not HBM (54 us
-// of traffic a launch on 64 histories of up to 1024^2, 64.6 Mpx), and next to
+// of traffic a launch on 64 histories of up to 1024^2, 22.3 M pixels), and next to
 // them what a window costs besides: the published rows, the barriers, the
 // look-up.  Sixteen rows a warp instead of eight halve the published rows and
 // the warps at a barrier per update and let two half-sweeps run unrolled;

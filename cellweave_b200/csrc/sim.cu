@@ -1025,7 +1025,7 @@ static int tune_depth(cw_sim_s *s) {
     // the time a sweep at every size)
     const bool volume = s->d[0] > 1;
     // the tall windows pay on many large planes (62.7 us a launch against 66.4
-    // on 64.6 Mpx) and only at the full depth, where the halo is widest
+    // on 22.3 M pixels) and only at the full depth, where the halo is widest
     for (int w : {CW_WINDOW_AUTO, CW_WINDOW_TALL, CW_WINDOW_64})
         for (int d : {4, 6, 8}) {
             if (volume && d != 4) continue;
