@@ -42,10 +42,10 @@ UNIT = "histories·MCS/s"
 # FP32 inner sweep, one pass through HBM: correction read 4 + write 4, right-hand side 4, inverse diagonal 4
 SOR_BYTES_PER_SITE_PASS = 16
 # DRAM bytes per site of one k_sor32_wide<8> launch on the campaign's oxygen
-# field, from ncu (dram__bytes_read.sum + dram__bytes_write.sum: 267.5 MB +
-# 65.5 MB over 22,282,240 sites), a launch that reads and writes the
+# field, from ncu (dram__bytes_read.sum + dram__bytes_write.sum: 267.6 MB +
+# 64.7 MB over 22,282,240 sites), a launch that reads and writes the
 # correction (neither the first nor the last of a solve)
-SOR_TRAFFIC_PER_SITE = 14.95
+SOR_TRAFFIC_PER_SITE = 14.91
 
 
 def parse():
