@@ -530,7 +530,7 @@ __global__ void k_sor32_half(float *__restrict__ dlt, const float *__restrict__ 
 // from such an edge equals S in-place half-sweeps of the whole history (as
 // k_sor32_half gives them, to the bit: the same sums in the same order).
 //
-// Measured on an oxygen field of 256^3 voxels (16-byte copies): 140 -> 41 us a
+// Measured on an oxygen field of 256^3 voxels (16-byte copies): 140 -> 39 us a
 // sweep against the kernel before, which kept the slices in shared memory, two
 // steps apart, and took 223 thread instructions an update (20 now); its HBM
 // floor at two sweeps a launch is 20 us, and the shared-memory pipe is busy 75 %
@@ -560,7 +560,8 @@ __device__ __forceinline__ void copy_async(uint32_t to, const float *from, bool 
 // the field); ANY: told at run time, for a launch of fewer half-sweeps.  Without
 // the other cases' code the unrolled steps fit the instruction cache (89 -> 62
 // us a sweep of 256^3 before the ring; the first and last launch of a
-// correction, both ANY before, 115 us on average, now 51 and 132).
+// correction, both ANY before: 115 us on average over a step's, now 51 and 132,
+// where the middle ones take 53; launches that find the field settled among them).
 enum VolKind { VOL_ANY, VOL_MIDDLE, VOL_FIRST, VOL_LAST };
 template <int NW, int ALIGN, int KIND>
 __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
