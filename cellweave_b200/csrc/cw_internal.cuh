@@ -64,9 +64,9 @@ class Join {
 #define CW_JOIN(h) ::cw::Join cw_join_(&(h)->hs)
 
 // Failure-test settings (cw_test_faults): all off by default.  wait_ns
-// shortens every bounded device wait (grid barriers, TMA copies) from its
-// 2 s; withhold_block keeps one block of a pass from arriving at its grid
-// barriers; max_rounds caps a pass's priority rounds; skip_tma makes the
+// shortens every bounded device wait (grid barriers, meetings, TMA copies) from
+// its 2 s; withhold_block keeps one block of a pass from arriving at its grid
+// barriers, and of a resident FP64 relax at its meetings; max_rounds caps a pass's priority rounds; skip_tma makes the
 // FP32 sweep kernels issue no copy, so that their waits run out.
 struct TestFaults {
     unsigned long long wait_ns = 0;

@@ -52,8 +52,6 @@ constexpr int SMEM_MAX = 220 * 1024;
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 constexpr long long LAUNCH_SWEEPS = 16384;  // the most sweeps one launch takes; a solve that needs more is launched again
 
-__device__ int g_resident_wait_failed;
-
 // One history's tiling: its swept box, the tiles along each axis, the window
 // sizes they need, and its first block.
 struct Part {
@@ -73,7 +71,9 @@ struct Args {
     long long max_sweeps;
     uint32_t *arrivals;           // per history: its blocks' meetings, counted up
     unsigned long long *slots;    // per history: three sets of SLOTS words, in turn
+    uint32_t *failed;             // set by a block whose meeting did not end in time
     unsigned long long wait_ns;
+    int withhold;                 // a block that never arrives at a meeting (failure tests; -1: none)
 };
 
 // The largest over a warp of non-negative doubles' bits, on every lane: the high
@@ -166,10 +166,14 @@ __device__ __forceinline__ void relax_pixels(const double (&t)[U], const double2
 }
 
 // The meeting of a history's blocks: the n-th ends when all have arrived n
-// times.  Bounded: false when it did not end in time.
-__device__ __forceinline__ bool meet(uint32_t *arrivals, uint32_t target, unsigned long long wait_ns, int *s_ok) {
+// times.  Bounded: false when it did not end in time, and on the block `withhold`,
+// which does not arrive.
+__device__ __forceinline__ bool meet(uint32_t *arrivals, uint32_t target, unsigned long long wait_ns, int withhold,
+                                     int *s_ok) {
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && (int)blockIdx.x == withhold) {
+        *s_ok = 0;
+    } else if (threadIdx.x == 0) {
         int ok = 1;
         // the block's writes, ordered before this thread by the barrier, are
         // released with the arrival; the acquiring load and the barrier behind
@@ -223,8 +227,8 @@ __device__ __forceinline__ void solve_rounds(const Args &a, const Part &pt, Load
     int cur = 0, settled = 0;
     double change = 0.0, resid = 0.0;
     auto met = [&]() -> bool {
-        if (meet(arrivals, (uint32_t)pt.nblocks * ++meetings, a.wait_ns, &S.ok)) return true;
-        if (tid == 0) atomicExch(&g_resident_wait_failed, 1);
+        if (meet(arrivals, (uint32_t)pt.nblocks * ++meetings, a.wait_ns, a.withhold, &S.ok)) return true;
+        if (tid == 0) atomicExch(a.failed, 1u);
         return false;
     };
     for (int round = 0; taken < a.max_sweeps; ++round) {
@@ -891,7 +895,7 @@ namespace cw {
 struct Resident64 {
     double *other = nullptr;
     Part *parts = nullptr;
-    uint32_t *words = nullptr;     // arrivals, then the slots
+    uint32_t *words = nullptr;     // arrivals, whether a meeting failed, then the slots
     std::vector<Part> host;
     std::vector<Span> spans;       // what the tilings were made for
     const void *coef[3] = {};
@@ -1028,7 +1032,8 @@ int relax64_resident(cw_field_s *f, const cw_relax_opts &o, const std::vector<Sp
     const FieldView fv = view(f);
     int rc = resident64_plan(f, r, fv, spans);
     if (rc != CW_OK || !r->served) return rc;
-    const size_t words = (size_t)nh + 1 + 2 * (size_t)nh * 3 * SLOTS;
+    const size_t slots = ((size_t)nh + 2) & ~(size_t)1;  // (64-bit words)
+    const size_t words = slots + 2 * (size_t)nh * 3 * SLOTS;
     if (!r->other || !r->words) {
         // a device without room for the scratch serves the solve by launches
         if (!r->other && cudaMalloc((void **)&r->other, sizeof(double) * (size_t)f->g.total) != cudaSuccess) {
@@ -1052,8 +1057,10 @@ int relax64_resident(cw_field_s *f, const cw_relax_opts &o, const std::vector<Sp
     a.nparts = (int)r->host.size();
     a.st = d_st;
     a.arrivals = r->words;
-    a.slots = (unsigned long long *)(r->words + ((nh + 1) & ~1u));
+    a.failed = r->words + nh;
+    a.slots = (unsigned long long *)(r->words + slots);
     a.wait_ns = test_faults().wait_ns ? test_faults().wait_ns : WAIT_NS;
+    a.withhold = test_faults().withhold_block;
     const Part &last = r->host.back();
     void *args[] = {&a};
     cudaLaunchConfig_t cfg = {};
@@ -1087,16 +1094,11 @@ int relax64_resident(cw_field_s *f, const cw_relax_opts &o, const std::vector<Sp
         }
         if (launched != cudaSuccess) return cuda_fail(launched, "cooperative launch");
         count_launch(1);
-        int failed = 0;
+        uint32_t failed = 0;
         CW_CUDA(cudaMemcpyAsync(hs.data(), d_st, sizeof(RelaxState) * nh, cudaMemcpyDeviceToHost, stream()));
-        CW_CUDA(cudaMemcpyFromSymbolAsync(&failed, g_resident_wait_failed, sizeof failed, 0, cudaMemcpyDeviceToHost,
-                                          stream()));
+        CW_CUDA(cudaMemcpyAsync(&failed, a.failed, sizeof failed, cudaMemcpyDeviceToHost, stream()));
         CW_CUDA(cudaStreamSynchronize(stream()));
-        if (failed) {
-            const int zero = 0;
-            CW_CUDA(cudaMemcpyToSymbol(g_resident_wait_failed, &zero, sizeof zero));
-            return fail(CW_ERR_TIMEOUT, "a block of the FP64 relax waited too long for its history's others");
-        }
+        if (failed) return fail(CW_ERR_TIMEOUT, "a block of the FP64 relax waited too long for its history's others");
         bool all = true;
         for (const RelaxState &s : hs) all = all && s.done;
         if (all) break;

@@ -96,7 +96,8 @@ uint64_t cw_launch_count(void);
  * make the library's bounded device waits run out without faulting the GPU.
  * wait_ns (1 ms to 2 s; 0: the default 2 s) limits every grid-barrier and
  * TMA-copy wait; withhold_block >= 0 keeps that block of each sublattice pass
- * from arriving at its grid barriers (the others give up: CW_ERR_TIMEOUT);
+ * from arriving at its grid barriers, and of an FP64 relax kept on chip at its
+ * meetings (the others give up: CW_ERR_TIMEOUT);
  * max_rounds > 0 caps a pass's priority rounds (past it: CW_ERR_SIMULATION);
  * skip_tma != 0 makes the FP32 sweeps issue no TMA copy, so their waits run
  * out (CW_ERR_TIMEOUT).  Every call replaces all four; (0, -1, 0, 0) is the
