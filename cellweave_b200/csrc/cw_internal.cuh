@@ -402,6 +402,7 @@ struct cw_lattice_s {
     unsigned long long *pchain = nullptr; // ncells lists of entries (null: passes by rounds)
     int32_t useg = 1;                     // pixels of a row a lane reads at once
     bool chain_tried = false;             // room for the lists was asked for
+    uint32_t plans = 0;                   // counts the plans made and the scratch taken: a captured sweep holds both
     int64_t plist_cap = 0;
     int32_t *d_vplan = nullptr;           // nh + 1: the pass plan (first chunk of each history)
     uint32_t *pctl = nullptr;             // control words, then 27 pass keys per history (lattice.cu)

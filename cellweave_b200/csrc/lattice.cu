@@ -1313,6 +1313,7 @@ int make_reach(int order, bool volume, int8_t *off, double *across) {
 }  // namespace
 
 int cw_lattice_s::build_plans() {
+    ++plans;
     bool volume = g.d[0] > 1;
     nreach = make_reach(order, volume, reach, &across);
     if (nreach == 0 && !copy_moore) {
@@ -1371,6 +1372,7 @@ int cw_lattice_s::ensure_scratch() {
     int rc;
     const int64_t need = (int64_t)pass_blocks * pass_seg;
     if (need > plist_cap) {
+        ++plans;
         dfree(plist);
         dfree(pidx);
         dfree(pmail);

@@ -104,6 +104,7 @@ struct cw_sim_s {
     cudaGraphExec_t gexec[3] = {nullptr, nullptr, nullptr};
     uint64_t gkernels[3] = {0, 0, 0};
     bool graphs = false;
+    uint32_t graph_plans = 0;    // the lattice's plans that the graphs hold
     int budget[2] = {0, 0};
     float *gstart[2] = {nullptr, nullptr};
     std::vector<cw_relax_stats> last_sig;
@@ -1404,10 +1405,13 @@ static int outer_budget(const std::vector<cw_relax_stats> &st, int inner) {
 
 static int build_graphs(cw_sim_s *s, const cw_relax_opts &o) {
     drop_graphs(s);
+    // what the sweeps allocate is allocated before the capture
+    int rc0;
+    if ((rc0 = s->lat->ensure_scratch()) != CW_OK) return rc0;
+    s->graph_plans = s->lat->plans;
     if (s->budget[0] <= 0) s->budget[0] = outer_budget(s->last, o.inner_sweeps);
     if (s->budget[1] <= 0) s->budget[1] = outer_budget(s->last_sig, o.inner_sweeps);
     // the factors the graphs will use: the configuration's or the tuned ones
-    int rc0;
     for (int fi = 0; fi < 2; ++fi) {
         cw_field_s *f = fi == 0 ? s->o2 : s->sig;
         if (!f) continue;
@@ -1514,6 +1518,8 @@ int cw_sim_step(cw_sim s, uint32_t nsteps) {
                               (!s->sig || !s->last_sig.empty()) && !s->wst && !s->nfc && c.o2_hold != 3 &&
                               !s->debris_on && !s->str && !s->track && !c.field_off;
         if (graph_ok) {
+            // (contact or copies set on the lattice since, or another scratch taken)
+            if (s->graphs && s->graph_plans != s->lat->plans) drop_graphs(s);
             if (!s->graphs && (rc = build_graphs(s, o)) != CW_OK) return rc;
             if ((rc = step_graph(s, o)) != CW_OK) return rc;
             continue;
