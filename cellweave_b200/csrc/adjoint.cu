@@ -133,22 +133,35 @@ __global__ void __launch_bounds__(RB) k_fit_forward(NetDev N, const double *x0, 
 
 // Vector-Jacobian product of the network's right-hand side at the lane's values
 // z with the adjoint a, for one node: a . df/d(z_node), and of node S the
-// oxygen's (gin).  `list` holds what the node takes part in, in file order: its
-// own terms (2 t) and the terms that read it (2 t + 1), a term that reads its
-// own node as both.  The rates' gradients (the first ntheta terms) go to gth,
-// each written by its own node's warp.
-__device__ __forceinline__ double vjp_node(const int4 *sterm, const double4 *spar, const uint32_t *list, int from,
-                                           int end, const double *z, const double *in, const double *a, double *gth,
-                                           int ntheta) {
+// oxygen's (gin).  The node takes part in its own terms, `own` to `own_end`, and
+// in those that read it, taken in file order, a term that reads its own node
+// first as its own: `list` holds all of it (2 t, and 2 t + 1 as what is read), or,
+// MERGED, the terms that read it alone.  The rates' gradients (the first ntheta
+// terms) go to gth, each written by its own node's warp.
+template <bool MERGED>
+__device__ __forceinline__ double vjp_node(const int4 *sterm, const double4 *spar, const uint16_t *list, int from,
+                                           int end, int own_term, int own_end, const double *z, const double *in,
+                                           const double *a, double *gth, int ntheta) {
     double g = 0.0;
-    for (int e = from; e < end; ++e) {
-        const int t = (int)(list[e] >> 1);
+    for (int e = from; e < end || (MERGED && own_term < own_end);) {
+        int t;
+        bool read;
+        if (MERGED) {
+            t = e < end ? (int)list[e] : INT_MAX;
+            read = own_term >= own_end || t < own_term;
+            if (read) ++e;
+            else t = own_term++;
+        } else {
+            t = (int)(list[e] >> 1);
+            read = list[e] & 1u;
+            ++e;
+        }
         const int4 tm = sterm[t];  // w: the term's own node
         const double ai = a[tm.w * RC];
         if (ai == 0.0) continue;
         const double4 p = spar[t];
         const double own = z[tm.w * RC], s = source_of(tm, z, in), k = p.x;
-        if (list[e] & 1u) {
+        if (read) {
             double gs = 0.0;
             switch (tm.x) {
             case CW_ACTIVATED_BY:
@@ -216,9 +229,9 @@ __device__ __forceinline__ double vjp_node(const int4 *sterm, const double4 *spa
 }
 
 // Shared bytes of a backward block.
-size_t backward_block(int S, int nterms, int ntheta) {
+size_t backward_block(int S, int nterms, int ntheta, bool merged) {
     return sizeof(double) * (9 * S + 6 + ntheta) * RC + nterms * (sizeof(int4) + sizeof(double4)) +
-           sizeof(int32_t) * (S + 1) + sizeof(uint32_t) * (2 * nterms + S + 2);
+           sizeof(int32_t) * (S + 1) + sizeof(uint32_t) * (S + 2) + sizeof(uint16_t) * (merged ? 1 : 2) * nterms;
 }
 
 // Reverse RK4 over one checkpointed segment of K steps, a lane per cell and a
@@ -234,7 +247,7 @@ size_t backward_block(int S, int nterms, int ntheta) {
 // 8 nodes and 40 steps (128 blocks of two warps); dealt to 8 warps
 // 0.89; of 16 nodes to 16 warps 12.3 -> 2.0 ms; 137,000 cells of 8 nodes, 8 steps,
 // 3.99 -> 1.88 ms.
-template <int G>
+template <int G, bool MERGED>
 __global__ void __launch_bounds__(32 * G)
     k_fit_backward(NetDev N, const double *ckm, const double *inputs, int64_t nc, int64_t node_stride,
                    int64_t cell_stride, int64_t in_stride, int64_t in_cell, int K, double dt, double *seg, double *lam,
@@ -247,7 +260,8 @@ __global__ void __launch_bounds__(32 * G)
     int4 *sterm = (int4 *)(sm + (9 * S + 6 + ntheta) * RC);
     double4 *spar = (double4 *)(sterm + N.nterms);
     int32_t *sptr = (int32_t *)(spar + N.nterms);
-    uint32_t *lptr = (uint32_t *)(sptr + S + 1), *list = lptr + S + 2;
+    uint32_t *lptr = (uint32_t *)(sptr + S + 1);
+    uint16_t *list = (uint16_t *)(lptr + S + 2);
     stage_terms(N, sterm, spar, sptr);
     __syncthreads();
     for (int i = threadIdx.x; i < S; i += 32 * G)
@@ -260,7 +274,7 @@ __global__ void __launch_bounds__(32 * G)
         uint32_t n = 0;
         for (int t = 0; t < N.nterms; ++t) {
             const int4 tm = sterm[t];
-            n += (tm.w == i) + (reads(tm) && tm.y == (i < S ? i : -1));
+            n += (!MERGED && tm.w == i) + (reads(tm) && tm.y == (i < S ? i : -1));
         }
         lptr[i + 1] = n;
     }
@@ -274,8 +288,8 @@ __global__ void __launch_bounds__(32 * G)
         uint32_t e = lptr[i];
         for (int t = 0; t < N.nterms; ++t) {
             const int4 tm = sterm[t];
-            if (tm.w == i) list[e++] = 2u * t;
-            if (reads(tm) && tm.y == (i < S ? i : -1)) list[e++] = 2u * t + 1u;
+            if (!MERGED && tm.w == i) list[e++] = (uint16_t)(2 * t);
+            if (reads(tm) && tm.y == (i < S ? i : -1)) list[e++] = (uint16_t)(MERGED ? t : 2 * t + 1);
         }
     }
     const int64_t c = (int64_t)blockIdx.x * RC + lane;
@@ -354,7 +368,9 @@ __global__ void __launch_bounds__(32 * G)
             const double share = stage > 2 ? dt / 3.0 : dt / 6.0, step = stage == 4 ? dt : 0.5 * dt;
             if (live)
                 for (int i = warp; i <= S; i += G) {
-                    const double g = vjp_node(sterm, spar, list, (int)lptr[i], (int)lptr[i + 1], z, in, a, gth, ntheta);
+                    const double g = vjp_node<MERGED>(sterm, spar, list, (int)lptr[i], (int)lptr[i + 1],
+                                                      MERGED && i < S ? sptr[i] : 0, MERGED && i < S ? sptr[i + 1] : 0,
+                                                      z, in, a, gth, ntheta);
                     if (i == S) {
                         gin += g * o2_slope;
                         continue;
@@ -376,17 +392,29 @@ __global__ void __launch_bounds__(32 * G)
     }
 }
 
-// Whether the device holds a network's backward step (beside 64 cells' columns), and the launch.
-int backward_fits(int S, int nterms) {
-    int dev = 0, most = 0;
+int max_block_bytes(int *most) {
+    int dev = 0;
     CW_CUDA(cudaGetDevice(&dev));
-    CW_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    CW_CUDA(cudaDeviceGetAttribute(most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    return CW_OK;
+}
+
+// Whether the device takes a network's backward step, and the launch.  The bound
+// is 64 cells' columns of 10 S + MAXTH numbers beside the terms.  With the lists
+// whole a block needs more than that where few nodes have thousands of terms
+// (52 bytes a term: 1 node of 4,238 terms where the bound allows 4,394); with the
+// lists of what reads a node alone (50 bytes) it needs less for every S, but takes
+// 3 % longer (8,192 cells of 8 nodes, 40 steps).
+int backward_fits(int S, int nterms) {
+    int most = 0;
+    const int rc = max_block_bytes(&most);
+    if (rc != CW_OK) return rc;
     if (sizeof(double) * (10 * S + MAXTH) * RB + nterms * (sizeof(int4) + sizeof(double4)) + sizeof(int32_t) * (S + 1) >
         (size_t)most)
         return CW_ERR_CONFIG;
     // (to the most there is: the attribute is the kernel's, whichever network it runs)
-    if (backward_block(S, nterms, MAXTH) > 48 * 1024)
-        for (auto k : {k_fit_backward<8>, k_fit_backward<16>})
+    if (backward_block(S, nterms, MAXTH, false) > 48 * 1024)
+        for (auto k : {k_fit_backward<8, false>, k_fit_backward<16, false>, k_fit_backward<8, true>})
             CW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     return CW_OK;
 }
@@ -394,14 +422,15 @@ int backward_fits(int S, int nterms) {
 int backward_launch(const NetDev &N, const double *ckm, const double *inputs, int64_t nc, int64_t node_stride,
                     int64_t cell_stride, int64_t in_stride, int64_t in_cell, int K, double dt, double *seg, double *lam,
                     double *gin, double *gth, int ntheta) {
+    int most = 0;
+    const int rc = max_block_bytes(&most);
+    if (rc != CW_OK) return rc;
     const unsigned grid = (unsigned)((nc + RC - 1) / RC);
-    const size_t smem = backward_block(N.S, N.nterms, ntheta);
-    if (N.S > 8)
-        k_fit_backward<16><<<grid, 512, smem, stream()>>>(N, ckm, inputs, nc, node_stride, cell_stride, in_stride,
-                                                          in_cell, K, dt, seg, lam, gin, gth, ntheta);
-    else
-        k_fit_backward<8><<<grid, 256, smem, stream()>>>(N, ckm, inputs, nc, node_stride, cell_stride, in_stride,
-                                                         in_cell, K, dt, seg, lam, gin, gth, ntheta);
+    const bool merged = backward_block(N.S, N.nterms, ntheta, false) > (size_t)most;
+    const size_t smem = backward_block(N.S, N.nterms, ntheta, merged);
+    auto k = merged ? k_fit_backward<8, true> : N.S > 8 ? k_fit_backward<16, false> : k_fit_backward<8, false>;
+    k<<<grid, !merged && N.S > 8 ? 512 : 256, smem, stream()>>>(N, ckm, inputs, nc, node_stride, cell_stride, in_stride,
+                                                                in_cell, K, dt, seg, lam, gin, gth, ntheta);
     CW_LAUNCHED();
     return CW_OK;
 }

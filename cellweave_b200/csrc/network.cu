@@ -34,9 +34,9 @@ size_t rk4_block(int S, int nterms) {
 // added in file order by one thread: the reference's operations in its order.
 // A stage's values live in shared memory, [node][lane], in two buffers turn by
 // turn, so a stage is one barrier; the six inputs stand clamped behind them.
-// nets null: every cell under N, its terms in shared memory; else cell c under
-// nets[clone[c]], its terms read from global memory (a network's tables are a
-// few KB: they stay in L1).
+// Not CLONES: every cell under N, its terms in shared memory; else cell c under
+// nets[clone[c]] (nets null: under N), its terms read from global memory (a
+// network's tables are a few KB: they stay in L1).
 // state: node i of cell c at state[i * node_stride + c * cell_stride], input q
 // at inputs[q * in_stride + c * in_cell]; alive (optional): cells whose entry is
 // zero are left as they are.
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(32 * G, 40 / G)
     const int32_t *ptr = sptr;
     if (CLONES) {
         if (live) {
-            const NetDev M = nets[clone[c]];
+            const NetDev M = nets ? nets[clone[c]] : N;
             term = M.term;
             par = M.par;
             ptr = M.node_ptr;
@@ -130,18 +130,22 @@ int rk4_launch(const NetDev &N, const NetDev *nets, const int32_t *clone, int S,
 int rk4_cells(const NetDev &N, const NetDev *nets, const int32_t *clone, int S, double *state, const double *inputs,
               int64_t ncells, int64_t node_stride, int64_t cell_stride, int64_t in_stride, int64_t in_cell, double dt,
               int substeps, const uint8_t *alive) {
-    int dev = 0, nsm = 0;
+    int dev = 0, nsm = 0, most = 0;
     CW_CUDA(cudaGetDevice(&dev));
     CW_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    CW_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    // a network whose terms leave no room for a cell's columns beside them (one
+    // node of 4,790 terms or more) reads them where they are
+    const bool far = nets || rk4_block(S, N.nterms) > (size_t)most;
     const int64_t nblocks = (ncells + RC - 1) / RC;
     // A warp per node up to 16 while the blocks are few, for the shortest chain
     // (5,000 cells of 12 nodes 78 us against 120 with 8 warps); 8 warps where the
     // blocks fill the device, which then holds more cells at a time (40,000 cells
     // of 16 nodes 366 us against 425 with 16); 4 for many cells of few nodes, for
     // fewer warps at a barrier (400,000 cells of 8 nodes 918 us against 971 with 8).
-    auto go = S > 8 && nblocks <= 2 * nsm     ? (nets ? rk4_launch<16, true> : rk4_launch<16, false>)
-              : S <= 8 && nblocks > 16 * nsm ? (nets ? rk4_launch<4, true> : rk4_launch<4, false>)
-                                             : (nets ? rk4_launch<8, true> : rk4_launch<8, false>);
+    auto go = S > 8 && nblocks <= 2 * nsm     ? (far ? rk4_launch<16, true> : rk4_launch<16, false>)
+              : S <= 8 && nblocks > 16 * nsm ? (far ? rk4_launch<4, true> : rk4_launch<4, false>)
+                                             : (far ? rk4_launch<8, true> : rk4_launch<8, false>);
     return go(N, nets, clone, S, state, inputs, ncells, node_stride, cell_stride, in_stride, in_cell, dt, substeps,
               alive);
 }
