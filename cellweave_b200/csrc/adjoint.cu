@@ -169,7 +169,7 @@ __device__ __forceinline__ double vjp_node(const int4 *sterm, const double4 *spa
                 double ddrv = 1.0;
                 if (tm.z) {
                     ddrv = 0.0;
-                    if (s > 0.0) {
+                    if (!(s <= 0.0)) {  // (and a NaN stays one)
                         const double sn = tm.z == SQUARE ? s * s : pow(s, p.y);
                         const double dsn = tm.z == SQUARE ? 2.0 * s : p.y * pow(s, p.y - 1.0);
                         const double den = p.z + sn;
@@ -197,7 +197,7 @@ __device__ __forceinline__ double vjp_node(const int4 *sterm, const double4 *spa
                 double drv = s;
                 if (tm.z) {
                     drv = 0.0;
-                    if (s > 0.0) {
+                    if (!(s <= 0.0)) {  // (and a NaN stays one)
                         const double sn = tm.z == SQUARE ? s * s : pow(s, p.y);
                         drv = sn / (p.z + sn);
                     }
