@@ -271,52 +271,80 @@ __global__ void k_colour_order(const uint2 *keys, int nh, int ncol, uint32_t *mc
     }
 }
 
-// The rows (y, z) that hold pixels of colour `colour` inside the box b = (x0,
-// y0, z0, x1, y1, z1) (inclusive) of a history: row `row` of them, its first
-// such pixel fx, their spacing `step` and count nx; false past the last row.
+// The rows (y, z) that hold pixels of a colour inside the box b = (x0, y0, z0,
+// x1, y1, z1) (inclusive) of a history, `rows` of them (none in an empty box).
 // Colour classes: the chessboard (x + y + z) mod 2 for period 0, else the
 // residues of x, y, z modulo the period.  (32-bit index arithmetic: a
 // history holds fewer than 2^31 pixels.)
-__device__ __forceinline__ bool colour_row(const int (&b)[6], int period, int colour, uint32_t row, int &y, int &z,
-                                           int &fx, int &step, int &nx) {
-    if (b[3] < b[0] || b[4] < b[1] || b[5] < b[2]) return false;
-    if (period == 0) {
-        const uint32_t wy = (uint32_t)(b[4] - b[1] + 1);
-        if (row >= wy * (uint32_t)(b[5] - b[2] + 1)) return false;
-        y = b[1] + (int)(row % wy);
-        z = b[2] + (int)(row / wy);
-        fx = b[0] + ((colour - b[0] - y - z) & 1);
-        step = 2;
-        nx = fx <= b[3] ? (b[3] - fx) / 2 + 1 : 0;
-        return true;
-    }
-    const int c[3] = {colour % period, (colour / period) % period, colour / (period * period)};
-    int f[3];
-    uint32_t n[3];
+struct ColourRows {
+    uint32_t rows, ny;  // rows, and how many of them a slice has
+    int f[3], step;     // the first pixel along each axis (chessboard: of the box) and the spacing
+    int last, nx0;      // the box's last x; a row's count of the colour (chessboard: its colour)
+    bool board;
+    __device__ __forceinline__ ColourRows(const int (&b)[6], int period, int colour) {
+        board = period == 0;
+        step = board ? 2 : period;
+        last = b[3];
+        nx0 = colour;
+        uint32_t n[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        f[a] = b[a] + ((c[a] - b[a] % period + period) % period);
-        n[a] = f[a] <= b[3 + a] ? (uint32_t)((b[3 + a] - f[a]) / period + 1) : 0u;
+        for (int a = 0; a < 3; ++a) {
+            f[a] = b[a];
+            n[a] = b[a] <= b[3 + a] ? (uint32_t)(b[3 + a] - b[a] + 1) : 0u;
+        }
+        if (!board) {
+            const int c[3] = {colour % period, (colour / period) % period, colour / (period * period)};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                f[a] = b[a] + ((c[a] - b[a] % period + period) % period);
+                n[a] = f[a] <= b[3 + a] ? (uint32_t)((b[3 + a] - f[a]) / period + 1) : 0u;
+            }
+            nx0 = (int)n[0];
+        }
+        ny = n[1];
+        rows = n[0] ? n[1] * n[2] : 0u;
     }
-    if (n[0] == 0 || n[1] == 0 || n[2] == 0 || row >= n[1] * n[2]) return false;
-    y = f[1] + period * (int)(row % n[1]);
-    z = f[2] + period * (int)(row / n[1]);
-    fx = f[0];
-    step = period;
-    nx = (int)n[0];
-    return true;
-}
+    // row `row` (below `rows`): its y and z, its first pixel of the colour and their count
+    __device__ __forceinline__ void at(uint32_t row, int &y, int &z, int &fx, int &nx) const {
+        const uint32_t q = rows == ny ? 0u : row / ny;
+        y = (int)(row - q * ny);
+        z = (int)q;
+        if (board) {
+            y += f[1];
+            z += f[2];
+            fx = f[0] + ((nx0 - f[0] - y - z) & 1);
+            nx = fx <= last ? (last - fx) / 2 + 1 : 0;
+        } else {
+            y = f[1] + step * y;
+            z = f[2] + step * z;
+            fx = f[0];
+            nx = nx0;
+        }
+    }
+};
 
-// Segments of 32 `useg` pixels of one colour that a row of a box of side wx
-// takes at most, and a box's items (rows times segments).
-__host__ __device__ __forceinline__ int64_t colour_segments(int64_t wx, int period, int useg) {
-    const int64_t n = period == 0 ? (wx + 1) / 2 : (wx + period - 1) / period;
-    return (n + 32 * useg - 1) / (32 * useg);
-}
+// How the pixels of one colour in a box of side wx are dealt to items of 32 `useg`
+// of them: a row's pixels (`n` at most) in `segs` items of their own, or, where
+// that would leave more than an eighth of the lanes without a pixel, the rows one
+// behind another (a division a pixel).  4,096 histories of 64 x 64, a Monte Carlo
+// step, rows in segments of 128 and the histories' plan walked one at a time ->
+// this and 32 histories a step: 3.36 -> 2.10 ms (order 3: 6.30 -> 3.08), and a
+// quarter of the scratch.
+struct ColourItems {
+    uint32_t n, segs;
+    bool packed;
+    __host__ __device__ __forceinline__ ColourItems(uint32_t wx, int period, int useg) {
+        n = period == 0 ? (wx + 1) / 2 : (wx + period - 1) / period;  // (a side is below 2^16)
+        segs = (n + 32 * useg - 1) / (32 * useg);
+        packed = segs * 32 * useg * 8 > n * 9;
+    }
+};
+// A box's items.
 __host__ __device__ __forceinline__ int64_t colour_items(int64_t wx, int64_t wy, int64_t wz, int period, int useg) {
     if (wx <= 0 || wy <= 0 || wz <= 0) return 0;
     const int64_t rows = period == 0 ? wy * wz : ((wy + period - 1) / period) * ((wz + period - 1) / period);
-    return rows * colour_segments(wx, period, useg);
+    const ColourItems it((uint32_t)wx, period, useg);
+    return it.packed ? (rows * it.n + 32 * useg - 1) / (32 * useg) : rows * it.segs;
 }
 
 // MurmurHash3's 32-bit finaliser (Appleby): a bijection of 32-bit words, so
@@ -398,7 +426,7 @@ struct Terms {
 
 constexpr int PT = 512;            // threads of a pass block; one block per SM
 constexpr int PW = PT / 32;        // its warps, an item (a row's segment) each of a chunk
-constexpr int UMAX = 4;            // pixels of a row a lane reads at once at most
+constexpr int UMAX = 4;            // pixels a lane reads at once at most
 constexpr int PEND = 3072;         // pending attempts a block lists in shared memory (rounds)
 constexpr int PLAN_SMEM = 1024;    // pass plans of up to 1023 histories sit in shared memory
 constexpr int CHAIN = 64;          // attempts a cell's list holds
@@ -631,9 +659,9 @@ struct PassShared {
 // attempts meet only through the records of a cell they both involve (volume,
 // surface).
 //
-// Propose: each warp takes rows' segments of the colour, a lane up to UMAX
-// pixels at once, and gathers the pixels that border another id; 32 of those
-// at a time draw their attempt.  An attempt that copies (source and copied ids
+// Propose: each warp takes items of the colour's pixels (a row's segment, or
+// short rows one behind another), a lane up to UMAX pixels at once, and gathers
+// those that border another id; 32 of them at a time draw their attempt.  An attempt that copies (source and copied ids
 // differ, neither the obstacle) is packed into its block's segment and listed
 // with its cells (not the medium).
 //
@@ -759,84 +787,113 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
             int have = 0;  // pixels gathered, the same in every lane
             int h = h0;    // a block's chunks come in increasing order: its history only moves forward
             for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-                while (h + 1 < nh && plan[h + 1] <= vb) ++h;
+                // (32 histories a step: one at a time, a batch of thousands waited for
+                // its plan longer than for its pixels)
+                for (int passed = 32; passed == 32; h += passed)
+                    passed = __popc(__ballot_sync(0xffffffffu, plan[min(h + 1 + lane, nh)] <= vb));
                 const int4 dm = __ldg(L.dims + h);
                 int box[6] = {0, 0, 0, dm.x - 1, dm.y - 1, dm.z - 1};
                 if (L.span && dm.z > 1)
 #pragma unroll
                     for (int a = 0; a < 6; ++a) box[a] = __ldg(L.span + 6 * h + a);
                 const uint32_t item = (uint32_t)(vb - plan[h]) * PW + (uint32_t)warp;
-                const uint32_t segs = (uint32_t)colour_segments(box[3] - box[0] + 1, L.period, S.useg);
-                const uint32_t row = segs ? item / segs : 0u;
-                int y = 0, z = 0, fx = 0, step = 0, nx = 0;
-                if (segs == 0 || !colour_row(box, L.period, __ldg(perm + h * L.ncol + pass), row, y, z, fx, step, nx)) continue;
-                const int j0 = (int)(item - row * segs) * 32 * S.useg + lane;
-                const int32_t *g = L.grid + __ldg(L.off + h) + ((int64_t)z * dm.y + y) * dm.x;
+                const ColourItems items((uint32_t)(box[3] - box[0] + 1), L.period, S.useg);
+                const ColourRows rows(box, L.period, __ldg(perm + h * L.ncol + pass));
+                if (rows.rows == 0u) continue;
+                const int32_t *const hist = L.grid + __ldg(L.off + h);
                 const int64_t w = dm.x, slice = (int64_t)dm.x * dm.y;
-                const bool up = y > 0, down = y + 1 < dm.y, in = z > 0, out = z + 1 < dm.z;
                 // every pixel's neighbours read at once (no read waits on another's
                 // test); a pixel whose copy neighbours all hold its own id cannot copy
                 bool edge[UMAX];
-                int xs[UMAX];
+                uint32_t xy[UMAX], hz[UMAX];
                 int32_t src[UMAX];
-                if (!L.copy_moore) {
-                    int32_t nb[UMAX][6];
-                    unsigned there[UMAX];
+                auto read = [&](auto packed) {
+                    constexpr bool PACKED = decltype(packed)::value;
+                    const uint32_t k0 = item * 32u * (uint32_t)S.useg + (uint32_t)lane;
+                    uint32_t row = 0, j0 = 0;
+                    int x = 0, y = 0, z = 0, fx = 0, nx = 0;
+                    if (!PACKED) {
+                        row = item / items.segs;
+                        j0 = k0 - row * items.segs * 32u * (uint32_t)S.useg;
+                        if (row < rows.rows) rows.at(row, y, z, fx, nx);
+                    }
+                    // the lane's pixel u into (x, y, z); false without one
+                    auto pixel = [&](int u) -> bool {
+                        uint32_t j = j0 + 32u * (uint32_t)u;
+                        if (PACKED) {
+                            row = (k0 + 32u * (uint32_t)u) / items.n;
+                            j = k0 + 32u * (uint32_t)u - row * items.n;
+                            nx = 0;
+                            if (row < rows.rows) rows.at(row, y, z, fx, nx);
+                        }
+                        x = fx + rows.step * (int)j;
+                        return u < S.useg && (int)j < nx;
+                    };
+                    if (!L.copy_moore) {
+                        int32_t nb[UMAX][6];
+                        unsigned there[UMAX];
 #pragma unroll
-                    for (int u = 0; u < UMAX; ++u) {
-                        const int j = j0 + 32 * u;
-                        const bool live = u < S.useg && j < nx;
-                        const int x = xs[u] = fx + step * j;
-                        src[u] = OBST;
-                        if (live) src[u] = g[x];
-                        // (not `: src[u]`: taking the pixel's own id where there is no
-                        // neighbour holds every later read until that id has come)
-                        const bool has[6] = {live && up, live && down, live && x > 0, live && x + 1 < dm.x, live && in,
-                                             live && out};
-                        const int64_t to[6] = {-w, w, -1, 1, -slice, slice};
-                        there[u] = 0u;
+                        for (int u = 0; u < UMAX; ++u) {
+                            const bool live = pixel(u);
+                            const int32_t *const g = hist + ((int64_t)z * dm.y + y) * dm.x;
+                            xy[u] = (uint32_t)x | ((uint32_t)y << 16);
+                            hz[u] = (uint32_t)h | ((uint32_t)z << 16);
+                            src[u] = OBST;
+                            if (live) src[u] = g[x];
+                            // (not `: src[u]`: taking the pixel's own id where there is no
+                            // neighbour holds every later read until that id has come)
+                            const bool has[6] = {live && y > 0, live && y + 1 < dm.y, live && x > 0,
+                                                 live && x + 1 < dm.x, live && z > 0, live && z + 1 < dm.z};
+                            const int64_t to[6] = {-w, w, -1, 1, -slice, slice};
+                            there[u] = 0u;
 #pragma unroll
-                        for (int q = 0; q < 6; ++q) {
-                            nb[u][q] = 0;
-                            if (has[q]) {
-                                nb[u][q] = g[x + to[q]];
-                                there[u] |= 1u << q;
+                            for (int q = 0; q < 6; ++q) {
+                                nb[u][q] = 0;
+                                if (has[q]) {
+                                    nb[u][q] = g[x + to[q]];
+                                    there[u] |= 1u << q;
+                                }
                             }
                         }
-                    }
 #pragma unroll
-                    for (int u = 0; u < UMAX; ++u) {
-                        edge[u] = false;
+                        for (int u = 0; u < UMAX; ++u) {
+                            edge[u] = false;
 #pragma unroll
-                        for (int q = 0; q < 6; ++q) edge[u] |= ((there[u] >> q) & 1u) && nb[u][q] != src[u];
-                        edge[u] = edge[u] && src[u] != OBST;
-                    }
-                } else {
-#pragma unroll 1
-                    for (int u = 0; u < UMAX; ++u) {
-                        const int j = j0 + 32 * u;
-                        const int x = fx + step * j;
-                        bool e = false;
-                        int32_t own = OBST;
-                        if (u < S.useg && j < nx) {
-                            own = g[x];
-                            const Moore mo = moore_of(dm, x, y, z);
-                            if (own != OBST)
-                                for (int q = 0; q < 27; ++q)
-                                    if ((mo.mask >> q) & 1u) e |= g[x + mo.step(q)] != own;
+                            for (int q = 0; q < 6; ++q) edge[u] |= ((there[u] >> q) & 1u) && nb[u][q] != src[u];
+                            edge[u] = edge[u] && src[u] != OBST;
                         }
+                    } else {
+#pragma unroll 1
+                        for (int u = 0; u < UMAX; ++u) {
+                            bool e = false;
+                            int32_t own = OBST;
+                            if (pixel(u)) {
+                                const int32_t *const g = hist + ((int64_t)z * dm.y + y) * dm.x;
+                                own = g[x];
+                                const Moore mo = moore_of(dm, x, y, z);
+                                if (own != OBST)
+                                    for (int q = 0; q < 27; ++q)
+                                        if ((mo.mask >> q) & 1u) e |= g[x + mo.step(q)] != own;
+                            }
 #pragma unroll
-                        for (int v = 0; v < UMAX; ++v)
-                            if (v == u) { edge[v] = e; xs[v] = x; src[v] = own; }
+                            for (int v = 0; v < UMAX; ++v)
+                                if (v == u) {
+                                    edge[v] = e;
+                                    xy[v] = (uint32_t)x | ((uint32_t)y << 16);
+                                    hz[v] = (uint32_t)h | ((uint32_t)z << 16);
+                                    src[v] = own;
+                                }
+                        }
                     }
-                }
+                };
+                if (items.packed) read(std::true_type());
+                else read(std::false_type());
 #pragma unroll
                 for (int u = 0; u < UMAX; ++u) {
                     const unsigned m = __ballot_sync(0xffffffffu, edge[u]);
                     if (edge[u])
                         gathered[have + __popc(m & ((1u << lane) - 1u))] =
-                            make_uint4((uint32_t)h | ((uint32_t)z << 16), (uint32_t)xs[u] | ((uint32_t)y << 16),
-                                       (uint32_t)src[u], 0u);
+                            make_uint4(hz[u], xy[u], (uint32_t)src[u], 0u);
                     have += __popc(m);
                     if (have >= 32) {
                         __syncwarp();
@@ -1341,15 +1398,21 @@ int cw_lattice_s::build_plans() {
     // the pass plan: chunks of PW items, as many as the largest colour of each
     // history's box holds (a plane's plan; in a volume a bound of the plan the
     // device takes from the occupied span every Monte Carlo step).  A lane of an
-    // item reads as many pixels (4, 2 or 1) as still give every block four chunks.
+    // item reads as many pixels (4, 2 or 1) as still give every block four chunks
+    // and add no more than an eighth to the chunks' pixels (a history's last chunk
+    // is rounded up).
     std::vector<int32_t> vp(g.nh + 1, 0);
-    for (useg = UMAX; useg >= 1; useg /= 2) {
+    auto chunks = [&](int per) {
         for (uint32_t k = 0; k < g.nh; ++k) {
-            const int64_t items = colour_items(g.w[k], g.h[k], g.d[k], period, useg);
+            const int64_t items = colour_items(g.w[k], g.h[k], g.d[k], period, per);
             vp[k + 1] = vp[k] + (int32_t)((items + PW - 1) / PW);
         }
-        if (useg == 1 || vp[g.nh] >= 4 * pass_grid) break;
-    }
+        return (int64_t)vp[g.nh] * per;
+    };
+    const int64_t least = chunks(1);
+    for (useg = UMAX; useg > 1; useg /= 2)
+        if (chunks(useg) * 8 <= least * 9 && vp[g.nh] >= 4 * pass_grid) break;
+    if (useg == 1) chunks(1);
     // the pass scratch: a block's segment holds every pixel of the chunks it
     // visits, (chunks / blocks launched, rounded up) items of 32 useg
     const int32_t nvb = vp[g.nh];

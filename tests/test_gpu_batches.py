@@ -1,0 +1,75 @@
+"""The sublattice passes over batches and lattices of many shapes (GPU): rows
+shorter than what a warp reads at once, one behind another; thousands of
+histories; cells' lists of every length; passes long enough that the blocks
+share out anew; and the memory that they take.  Grids and records are the
+oracle's, to the bit.
+"""
+import numpy as np
+import pytest
+
+import cellweave_b200 as cw
+from cellweave_b200 import seeding
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+J3 = np.array([[0, 16, 16], [16, 8, 12], [16, 12, 8]], float)
+
+
+def packed(shape, side, seed, skip=0.2):
+    w, h, d = shape
+    grid, rec = seeding.empty(w, h, d), seeding.Records()
+    rng = np.random.default_rng(seed)
+    sz = min(side, d)
+    for z in range(0, d - sz + 1, sz):
+        for y in range(0, h - side + 1, side):
+            for x in range(0, w - side + 1, side):
+                if rng.random() >= skip:
+                    seeding.add_block(grid, rec, 1 + int(rng.integers(2)), (x, y), side, side, lam=1.3, z=z, depth=sz)
+    return grid, rec
+
+
+def same_as_the_oracle(lat, k, grid, rec, order, steps, seed):
+    d, h, w = grid.shape
+    o = O.Lattice(grid, (w, h, d), len(rec), J3, 10.0, order)
+    o.type[:], o.volume[:], o.target[:], o.lam[:] = rec.arrays()
+    o.mcs_checkerboard(seed, 0, steps)
+    got = lat.grid(k)
+    np.testing.assert_array_equal(got.reshape(-1), o.grid)
+    np.testing.assert_array_equal(lat.cells(len(rec), k)["volume"][1:], o.volume[1:])
+    assert (got != grid).any()
+
+
+# 1 to 128 pixels of a colour in a row, whole and cut short; more histories than
+# a block keeps the plan of in shared memory
+@pytest.mark.parametrize("shapes,order", [([(31, 9, 1), (64, 64, 1), (5, 70, 1), (130, 33, 1), (256, 20, 1)], 2),
+                                          ([(33, 40, 1), (64, 30, 1), (7, 7, 1), (300, 21, 1)], 1),
+                                          ([(48, 48, 1), (100, 30, 1), (200, 17, 1)], 3),
+                                          ([(20, 24, 22), (9, 33, 8), (66, 12, 10)], 1),
+                                          ([(20, 24, 22), (9, 33, 8), (70, 12, 10)], 2)])
+@pytest.mark.parametrize("copies", [1, 300])
+def test_batches_of_short_rows(shapes, order, copies):
+    side = 4
+    base = [packed(s, side, 11 + k) for k, s in enumerate(shapes)]
+    n = len(shapes) * copies
+    grids = [base[k % len(shapes)][0] for k in range(n)]
+    recs = [base[k % len(shapes)][1] for k in range(n)]
+    lat = cw.CpmLattice.from_grids(grids, recs, 10.0, J3, order, seeds=list(range(100, 100 + n)))
+    lat.monte_carlo_step(3)
+    for k in {0, 1, len(shapes) - 1, n // 2, n - 2, n - 1}:
+        same_as_the_oracle(lat, k, grids[k], recs[k], order, 3, 100 + k)
+
+
+def test_the_scratch_of_short_rows_follows_their_pixels():
+    torch = pytest.importorskip("torch")
+    grid, rec = packed((64, 64, 1), 7, 1)
+    n = 2048
+    lat = cw.CpmLattice.from_grids([grid] * n, [rec] * n, 10.0, J3, 2, seeds=list(range(n)))
+    before = torch.cuda.mem_get_info()[0]
+    lat.monte_carlo_step(1)
+    taken = before - torch.cuda.mem_get_info()[0]
+    # a colour's pixels: a quarter of the sites.  152 bytes each, an eighth for
+    # chunks' ends and one chunk of 2,048 for each of up to 148 blocks; 516 + 16
+    # bytes a record; 2 MB for each of six allocations
+    pixels = n * 64 * 64 // 4
+    assert taken <= 152 * (pixels * 9 // 8 + 148 * 2048) + 532 * n * len(rec) + (12 << 20)
