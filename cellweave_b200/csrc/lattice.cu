@@ -928,7 +928,10 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                 if (a.cd != NONE) S.count[a.cd] = 0u;
             }
         };
-        // ---- link: a warp takes a cell's whole list, an entry or two a lane; each
+        // ---- link: G lanes of a warp take a cell's whole list, as many cells at once
+        // as that leaves room for (a cell waits for its list and then for an
+        // exchange; one cell a warp, dense planes of 16.8 M pixels took 2.00 ms a
+        // step, now 1.69, and 2.70 -> 1.87 with the nine passes of order 3); each
         // entry's follower into its attempt, and the cell's records to the first
         if (linked) {
             uint32_t *const found = (uint32_t *)P.edge[warp];
@@ -944,31 +947,39 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                 if (lane < m) S.idx[at + lane] = found[lane];
                 __syncwarp();
             };
-            // (a warp's cells lie a stride apart: those with attempts are often the
-            // first of the records)
             const int64_t stride = (int64_t)gridDim.x * PW;
-            for (int64_t c0 = blockIdx.x * PW + warp; c0 < S.ncells; c0 += 32 * stride) {
-                const uint32_t cnt = c0 + lane * stride < S.ncells ? __ldcg(S.count + c0 + lane * stride) : 0u;
-                for (unsigned live = __ballot_sync(0xffffffffu, cnt != 0u); live; live &= live - 1u) {
-                    const int q = __ffs(live) - 1;
-                    const uint32_t k = __shfl_sync(0xffffffffu, cnt, q);
-                    const size_t c = (size_t)(c0 + q * stride);
-                    const unsigned long long *list = S.chain + c * CHAIN;
-                    const int32_t vol = __ldcg(L.volume + c), surf = surf_on ? __ldcg(L.surface + c) : 0;
-                    unsigned long long mine2[2] = {lane < k ? __ldcg(list + lane) : 0ull,
-                                                   lane + 32 < k ? __ldcg(list + 32 + lane) : 0ull};
-                    if (!records_fit(vol, surf)) P.odd = 1u;
+            // the cells c0 + q stride, `cnt` attempts each (lane q's), for the bits q of `live`
+            auto link = [&](auto lanes, unsigned live, uint32_t cnt, int64_t c0) {
+                constexpr int G = decltype(lanes)::value;
+                const int group = lane / G, gl = lane % G;
+                while (live) {
+                    int q = -1;  // this group's cell
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
+                    for (int g = 0; g < 32 / G; ++g) {
+                        if (g == group && live) q = __ffs(live) - 1;
+                        live &= live - 1u;
+                    }
+                    const uint32_t listed = __shfl_sync(0xffffffffu, cnt, q & 31), k = q >= 0 ? listed : 0u;
+                    const uint32_t longest = G == 32 ? k : __reduce_max_sync(0xffffffffu, k);
+                    const size_t c = q >= 0 ? (size_t)(c0 + q * stride) : 0;
+                    const unsigned long long *entries = S.chain + c * CHAIN;
+                    const int32_t vol = __ldcg(L.volume + c), surf = surf_on ? __ldcg(L.surface + c) : 0;
+                    unsigned long long mine2[2] = {gl < k ? __ldcg(entries + gl) : 0ull, 0ull};
+                    if (G == 32 && lane + 32 < k) mine2[1] = __ldcg(entries + 32 + lane);
+                    if (k && !records_fit(vol, surf)) P.odd = 1u;
+#pragma unroll
+                    for (int half = 0; half < (G == 32 ? 2 : 1); ++half) {
                         if (half && k <= 32) break;
                         const unsigned long long own = mine2[half];
                         const uint32_t prio = (uint32_t)(own >> 32);
                         unsigned long long below = 0ull;
-                        bool followed = false, first = lane + 32u * half < k;
-                        for (uint32_t j = 0; j < k; ++j) {
+                        bool followed = false, first = gl + 32u * half < k;
+                        for (uint32_t j = 0; j < longest; ++j) {
                             // (a cell's attempts have distinct priorities)
-                            const unsigned long long x = __shfl_sync(0xffffffffu, j < 32 ? mine2[0] : mine2[1], j & 31);
+                            const unsigned long long x =
+                                __shfl_sync(0xffffffffu, G < 32 || j < 32 ? mine2[0] : mine2[1], j & 31, G);
                             const uint32_t xp = (uint32_t)(x >> 32);
+                            if (G < 32 && j >= k) continue;
                             if (xp > prio) first = false;
                             if (xp < prio && (!followed || x > below)) {
                                 below = x;
@@ -977,7 +988,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                         }
                         bool ready = false;
                         const uint32_t id = ((uint32_t)own >> 2);
-                        if (lane + 32u * half < k) {
+                        if (gl + 32u * half < k) {
                             if (followed) (own & 1ull ? S.list[id].next_d : S.list[id].next_s) = (uint32_t)below;
                             if (first) {
                                 const unsigned long long box = pack_records(vol, surf, 0u);
@@ -987,15 +998,27 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                             }
                         }
                         // (at most one a list)
-                        if (__any_sync(0xffffffffu, ready)) {
-                            if (ready) found[have] = id;
-                            if (++have == 32) {
-                                flush(32);
-                                have = 0;
-                            }
+                        const unsigned some = __ballot_sync(0xffffffffu, ready);
+                        if (ready) found[have + __popc(some & ((1u << lane) - 1u))] = id;
+                        have += __popc(some);
+                        if (have >= 32) {
+                            flush(32);
+                            const uint32_t rest = found[32 + lane];
+                            __syncwarp();
+                            found[lane] = rest;
+                            have -= 32;
                         }
                     }
                 }
+            };
+            // (a warp's cells lie a stride apart: those with attempts are often the
+            // first of the records)
+            for (int64_t c0 = blockIdx.x * PW + warp; c0 < S.ncells; c0 += 32 * stride) {
+                const uint32_t cnt = c0 + lane * stride < S.ncells ? __ldcg(S.count + c0 + lane * stride) : 0u;
+                link(std::integral_constant<int, 4>(), __ballot_sync(0xffffffffu, cnt - 1u < 4u), cnt, c0);
+                link(std::integral_constant<int, 8>(), __ballot_sync(0xffffffffu, cnt - 5u < 4u), cnt, c0);
+                link(std::integral_constant<int, 16>(), __ballot_sync(0xffffffffu, cnt - 9u < 8u), cnt, c0);
+                link(std::integral_constant<int, 32>(), __ballot_sync(0xffffffffu, cnt > 16u), cnt, c0);
             }
             if (have) flush(have);
         }

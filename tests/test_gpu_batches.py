@@ -73,3 +73,18 @@ def test_the_scratch_of_short_rows_follows_their_pixels():
     # bytes a record; 2 MB for each of six allocations
     pixels = n * 64 * 64 // 4
     assert taken <= 152 * (pixels * 9 // 8 + 148 * 2048) + 532 * n * len(rec) + (12 << 20)
+
+
+# cells whose lists hold about 2 to 50 attempts a pass, side by side
+@pytest.mark.parametrize("order", [1, 2, 3])
+def test_lists_of_every_length(order):
+    grid, rec = seeding.empty(400, 300, 1), seeding.Records()
+    rng = np.random.default_rng(4)
+    for x0, side in ((0, 2), (60, 4), (120, 7), (190, 12), (260, 20), (330, 30)):
+        for y in range(0, 300 - side + 1, side):
+            for x in range(x0, x0 + 60 - side + 1, side):
+                if rng.random() < 0.9:
+                    seeding.add_block(grid, rec, 1 + int(rng.integers(2)), (x, y), side, side, lam=1.0)
+    lat = cw.CpmLattice.from_grids([grid], [rec], 10.0, J3, order, seeds=[77])
+    lat.monte_carlo_step(4)
+    same_as_the_oracle(lat, 0, grid, rec, order, 4, 77)
