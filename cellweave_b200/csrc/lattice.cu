@@ -430,6 +430,7 @@ constexpr int UMAX = 4;            // pixels a lane reads at once at most
 constexpr int PEND = 3072;         // pending attempts a block lists in shared memory (rounds)
 constexpr int PLAN_SMEM = 1024;    // pass plans of up to 1023 histories sit in shared memory
 constexpr int CHAIN = 64;          // attempts a cell's list holds
+constexpr int TURNS = 64;          // attempts a lane runs before its warp shares out what it holds
 constexpr int MAX_ROUNDS = 256;
 constexpr uint32_t ROUND_SPAN = MAX_ROUNDS + 2;  // claim tags one pass may use
 // passes before the claim tags would overflow 32 bits: the pass that reaches
@@ -675,7 +676,8 @@ struct PassShared {
 // runs the attempt.  The last attempt on a cell writes its records.  So every
 // attempt runs after all of higher priority that share a cell with it, which
 // is the sequence in decreasing priority, whatever the thread schedule, and
-// nothing waits: the blocks meet three times a pass.
+// nothing waits: the blocks meet three times a pass, and once more for every
+// TURNS attempts that a lane runs in turn.
 //
 // Rounds: a pass with a cell of more than CHAIN attempts (or records past
 // pack_records' ranges), or without room for the lists, runs by claims: every
@@ -1093,123 +1095,164 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
             // ---- run the chains: a lane takes what it made ready, else its spare or
             // its stack, else its next of the list, else another lane's spare
             // (dealt one to a warp, then a second to each: the chains of a warp
-            // wait for one another's reads, and its idle lanes take their branches)
+            // wait for one another's reads, and its idle lanes take their branches).
+            // A warp that has made TURNS puts what it holds back into the list, and
+            // the blocks meet and share that out anew: what follows an attempt stays
+            // with the warp that ran it, so that of many attempts a few warps came to
+            // hold the most (a 256^3 volume of 125-voxel cells, order 1: 2,800 turns
+            // for one warp, 42 on average; 10.6 -> 2.7 ms a step).
             const uint32_t warps = gridDim.x * PW, stride = 32u * warps;
-            uint32_t at = blockIdx.x * PW + warp + lane * warps;
-            uint32_t id = NONE, spare = NONE, top = NONE, listed = at < left ? __ldcg(S.idx + at) : NONE;
-            // the records that the current attempt and the spare were handed
-            unsigned long long box_s = 0ull, box_d = 0ull, spare_s = 0ull, spare_d = 0ull;
-            for (;;) {
-                if (id == NONE) {
-                    if (spare != NONE) {
-                        id = spare;
-                        box_s = spare_s;
-                        box_d = spare_d;
-                        spare = NONE;
-                    } else if (top != NONE || listed != NONE) {
-                        if (top != NONE) {
-                            id = top;
-                            top = S.link[id];
-                        } else {
-                            id = listed;
-                            at += stride;
-                            listed = at < left ? __ldcg(S.idx + at) : NONE;
+            uint32_t begin = 0;  // the list's part that has not been run: [begin, begin + left)
+            do {
+                if (threadIdx.x == 0) P.ready = 0u;
+                __syncthreads();
+                const uint32_t end = begin + left;
+                uint32_t at = begin + blockIdx.x * PW + warp + lane * warps;
+                uint32_t id = NONE, spare = NONE, top = NONE, listed = at < end ? __ldcg(S.idx + at) : NONE;
+                // the records that the current attempt and the spare were handed
+                unsigned long long box_s = 0ull, box_d = 0ull, spare_s = 0ull, spare_d = 0ull;
+                auto stack = [&](uint32_t what, unsigned long long s, unsigned long long d) {
+                    S.mail[what] = make_ulonglong2(s, d);
+                    S.link[what] = top;
+                    top = what;
+                };
+                for (int turn = 0;; ++turn) {
+                    const bool sharing = turn >= TURNS;
+                    if (sharing) {
+                        // the rest of the warp's part of the list first, so that an
+                        // attempt is listed once: as it is linked or as it is put back
+                        if (listed != NONE && id != NONE) {
+                            stack(id, box_s, box_d);
+                            id = NONE;
                         }
-                        const ulonglong2 b = __ldcg(S.mail + id);
-                        box_s = b.x;
-                        box_d = b.y;
-                    }
-                }
-                const unsigned idle = __ballot_sync(0xffffffffu, id == NONE);
-                if (idle) {
-                    const unsigned rich = __ballot_sync(0xffffffffu, spare != NONE), below = (1u << lane) - 1u;
-                    if (rich) {
-                        const int m = min(__popc(idle), __popc(rich)), ri = __popc(idle & below), rr = __popc(rich & below);
-                        const bool takes = ((idle >> lane) & 1u) && ri < m, gives = ((rich >> lane) & 1u) && rr < m;
-                        const int from = takes ? (int)__fns(rich, 0, ri + 1) : lane;
-                        const uint32_t got = __shfl_sync(0xffffffffu, spare, from);
-                        const unsigned long long gs = __shfl_sync(0xffffffffu, spare_s, from),
-                                                 gd = __shfl_sync(0xffffffffu, spare_d, from);
-                        if (gives) spare = NONE;
-                        if (takes) {
-                            id = got;
-                            box_s = gs;
-                            box_d = gd;
+                        if (!__any_sync(0xffffffffu, listed != NONE)) {
+                            auto put_back = [&](uint32_t what) {
+                                const unsigned m = __ballot_sync(0xffffffffu, what != NONE);
+                                uint32_t to = 0;
+                                if (lane == 0 && m) {
+                                    to = atomicAdd(S.ctl + CTL_READY + (pass & 1), (uint32_t)__popc(m));
+                                    atomicAdd(&P.ready, (uint32_t)__popc(m));
+                                }
+                                to = __shfl_sync(0xffffffffu, to, 0) + __popc(m & ((1u << lane) - 1u));
+                                if (what != NONE) S.idx[to] = what;
+                                return m != 0u;
+                            };
+                            if (id != NONE) stack(id, box_s, box_d);
+                            if (spare != NONE) stack(spare, spare_s, spare_d);
+                            while (put_back(top))
+                                if (top != NONE) top = S.link[top];
+                            break;
                         }
-                    } else if (idle == 0xffffffffu) {
-                        break;
                     }
-                }
-                if (id != NONE) {
-                    Terms a;
-                    a.read(S.list + id, surf_on);
-                    const uint32_t cs = a.cs, cd = a.cd;
-                    uint32_t depth = 0;
-                    int32_t vs = 0, ss = 0, vd = 0, sd = 0;
-                    auto open = [&](unsigned long long b, uint32_t c, int32_t &vol, int32_t &surf) {
-                        if (c == NONE) return;
-                        vol = (int32_t)((uint32_t)b << 4) >> 4;
-                        surf = (int32_t)((uint32_t)(b >> 28) << 7) >> 7;
-                        depth = max(depth, (uint32_t)(b >> 53) & 1023u);
-                    };
-                    open(box_s, cs, vs, ss);
-                    open(box_d, cd, vd, sd);
-                    attempt(a, vs, ss, vd, sd);
-                    depth += 1;
-                    most = max(most, depth);
-                    const uint32_t next[2] = {cs == NONE ? NONE : a.next_s, cd == NONE ? NONE : a.next_d};
-                    const unsigned long long send[2] = {pack_records(vs, ss, depth), pack_records(vd, sd, depth)};
-                    unsigned long long met[2] = {0ull, 0ull};
+                    if (id == NONE) {
+                        if (spare != NONE && !(sharing && listed != NONE)) {
+                            id = spare;
+                            box_s = spare_s;
+                            box_d = spare_d;
+                            spare = NONE;
+                        } else if (top != NONE || listed != NONE) {
+                            if (top != NONE && !(sharing && listed != NONE)) {
+                                id = top;
+                                top = S.link[id];
+                            } else {
+                                id = listed;
+                                at += stride;
+                                listed = at < end ? __ldcg(S.idx + at) : NONE;
+                            }
+                            const ulonglong2 b = __ldcg(S.mail + id);
+                            box_s = b.x;
+                            box_d = b.y;
+                        }
+                    }
+                    const unsigned idle = __ballot_sync(0xffffffffu, id == NONE);
+                    if (idle) {
+                        const unsigned rich = __ballot_sync(0xffffffffu, spare != NONE), below = (1u << lane) - 1u;
+                        if (rich) {
+                            const int m = min(__popc(idle), __popc(rich)), ri = __popc(idle & below), rr = __popc(rich & below);
+                            const bool takes = ((idle >> lane) & 1u) && ri < m, gives = ((rich >> lane) & 1u) && rr < m;
+                            const int from = takes ? (int)__fns(rich, 0, ri + 1) : lane;
+                            const uint32_t got = __shfl_sync(0xffffffffu, spare, from);
+                            const unsigned long long gs = __shfl_sync(0xffffffffu, spare_s, from),
+                                                     gd = __shfl_sync(0xffffffffu, spare_d, from);
+                            if (gives) spare = NONE;
+                            if (takes) {
+                                id = got;
+                                box_s = gs;
+                                box_d = gd;
+                            }
+                        } else if (idle == 0xffffffffu) {
+                            break;
+                        }
+                    }
+                    if (id != NONE) {
+                        Terms a;
+                        a.read(S.list + id, surf_on);
+                        const uint32_t cs = a.cs, cd = a.cd;
+                        uint32_t depth = 0;
+                        int32_t vs = 0, ss = 0, vd = 0, sd = 0;
+                        auto open = [&](unsigned long long b, uint32_t c, int32_t &vol, int32_t &surf) {
+                            if (c == NONE) return;
+                            vol = (int32_t)((uint32_t)b << 4) >> 4;
+                            surf = (int32_t)((uint32_t)(b >> 28) << 7) >> 7;
+                            depth = max(depth, (uint32_t)(b >> 53) & 1023u);
+                        };
+                        open(box_s, cs, vs, ss);
+                        open(box_d, cd, vd, sd);
+                        attempt(a, vs, ss, vd, sd);
+                        depth += 1;
+                        most = max(most, depth);
+                        const uint32_t next[2] = {cs == NONE ? NONE : a.next_s, cd == NONE ? NONE : a.next_d};
+                        const unsigned long long send[2] = {pack_records(vs, ss, depth), pack_records(vd, sd, depth)};
+                        unsigned long long met[2] = {0ull, 0ull};
 #pragma unroll
-                    for (int side = 0; side < 2; ++side)
-                        if (next[side] != NONE) {
+                        for (int side = 0; side < 2; ++side)
+                            if (next[side] != NONE) {
+                                const uint32_t to = next[side] >> 2;
+                                // its terms into L1 while the exchange is on its way
+                                const char *line = (const char *)(S.list + to);
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) {
+                                    uint32_t t;
+                                    if (q < 3 || surf_on) asm volatile("ld.global.u32 %0, [%1];" : "=r"(t) : "l"(line + 32 * q) : "memory");
+                                }
+                                if (!(next[side] & 2u)) met[side] = atomicExch(&S.mail[to].x, send[side]);
+                            }
+                        // the last attempt on a cell writes its records
+                        if (cs != NONE && next[0] == NONE) {
+                            L.volume[cs] = vs;
+                            if (surf_on) L.surface[cs] = ss;
+                            S.count[cs] = 0u;
+                        }
+                        if (cd != NONE && next[1] == NONE) {
+                            L.volume[cd] = vd;
+                            if (surf_on) L.surface[cd] = sd;
+                            S.count[cd] = 0u;
+                        }
+                        id = NONE;
+#pragma unroll
+                        for (int side = 0; side < 2; ++side) {
+                            if (next[side] == NONE || !((next[side] & 2u) || met[side])) continue;
                             const uint32_t to = next[side] >> 2;
-                            // its terms into L1 while the exchange is on its way
-                            const char *line = (const char *)(S.list + to);
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                uint32_t t;
-                                if (q < 3 || surf_on) asm volatile("ld.global.u32 %0, [%1];" : "=r"(t) : "l"(line + 32 * q) : "memory");
+                            const unsigned long long bs = (next[side] & 1u) ? met[side] : send[side],
+                                                     bd = (next[side] & 1u) ? send[side] : met[side];
+                            if (id == NONE) {
+                                id = to;
+                                box_s = bs;
+                                box_d = bd;
+                            } else {
+                                if (spare != NONE) stack(spare, spare_s, spare_d);
+                                spare = to;
+                                spare_s = bs;
+                                spare_d = bd;
                             }
-                            if (!(next[side] & 2u)) met[side] = atomicExch(&S.mail[to].x, send[side]);
-                        }
-                    // the last attempt on a cell writes its records
-                    if (cs != NONE && next[0] == NONE) {
-                        L.volume[cs] = vs;
-                        if (surf_on) L.surface[cs] = ss;
-                        S.count[cs] = 0u;
-                    }
-                    if (cd != NONE && next[1] == NONE) {
-                        L.volume[cd] = vd;
-                        if (surf_on) L.surface[cd] = sd;
-                        S.count[cd] = 0u;
-                    }
-                    id = NONE;
-#pragma unroll
-                    for (int side = 0; side < 2; ++side) {
-                        if (next[side] == NONE || !((next[side] & 2u) || met[side])) continue;
-                        const uint32_t to = next[side] >> 2;
-                        const unsigned long long bs = (next[side] & 1u) ? met[side] : send[side],
-                                                 bd = (next[side] & 1u) ? send[side] : met[side];
-                        if (id == NONE) {
-                            id = to;
-                            box_s = bs;
-                            box_d = bd;
-                        } else {
-                            if (spare != NONE) {
-                                S.mail[spare] = make_ulonglong2(spare_s, spare_d);
-                                S.link[spare] = top;
-                                top = spare;
-                            }
-                            spare = to;
-                            spare_s = bs;
-                            spare_d = bd;
                         }
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
-            }
-            if (!grid_barrier(S, bar++, 0u, 0u, &left, &flags, P.word)) { gave_up(); return; }
+                begin = end;
+                __syncthreads();
+                if (!grid_barrier(S, bar++, P.ready, 0u, &left, &flags, P.word)) { gave_up(); return; }
+            } while (left != 0u);
             continue;
         }
         // ---- rounds

@@ -88,3 +88,13 @@ def test_lists_of_every_length(order):
     lat = cw.CpmLattice.from_grids([grid], [rec], 10.0, J3, order, seeds=[77])
     lat.monte_carlo_step(4)
     same_as_the_oracle(lat, 0, grid, rec, order, 4, 77)
+
+
+def test_a_pass_of_many_turns():
+    # 125-voxel cells filling a volume, two colours: a quarter of a million attempts a
+    # pass, and some 90 that follow one another
+    shape = (128, 128, 128)
+    grid, rec = packed(shape, 5, 9, skip=0.05)
+    lat = cw.CpmLattice.from_grids([grid], [rec], 10.0, J3, 1, seeds=[5])
+    lat.monte_carlo_step(2)
+    same_as_the_oracle(lat, 0, grid, rec, 1, 2, 5)
