@@ -395,13 +395,13 @@ struct cw_lattice_s {
     int32_t *d_flag = nullptr;       // scratch flag / counters
     // scratch of the sublattice passes (lattice.cu): claims, attempts, the cells' lists, control words
     unsigned long long *claim = nullptr;  // 2 * ncells
-    uint4 *plist = nullptr;               // plist_cap attempts of 8 uint4
+    uint4 *plist = nullptr;               // plist_cap attempts of 8 uint4 (3 where lean)
     ulonglong2 *pmail = nullptr;          // plist_cap mailboxes
     uint32_t *pidx = nullptr;             // 2 * plist_cap attempt indices
     uint32_t *pcount = nullptr;           // ncells: attempts listed
-    unsigned long long *pchain = nullptr; // ncells lists of entries (null: passes by rounds)
+    unsigned long long *pchain = nullptr; // ncells lists of entries
     int32_t useg = 1;                     // pixels of a row a lane reads at once
-    bool chain_tried = false;             // room for the lists was asked for
+    bool lean = false;                    // every pass by rounds, attempts of 3 uint4, no mailboxes or lists
     uint32_t plans = 0;                   // counts the plans made and the scratch taken: a captured sweep holds both
     int64_t plist_cap = 0;
     int32_t *d_vplan = nullptr;           // nh + 1: the pass plan (first chunk of each history)

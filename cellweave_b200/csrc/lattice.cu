@@ -384,6 +384,21 @@ struct __align__(128) Attempt {
 };
 static_assert(sizeof(Attempt) == 128, "an attempt is one line");
 
+// The same for a sweep that runs every pass by rounds in little memory: what the
+// cells' records hold is read there.
+struct __align__(16) LeanAttempt {
+    uint32_t cs, cd, prio;
+    int32_t dst;
+    int64_t gi;
+    uint32_t u0, u1;
+    union {
+        double contact;
+        uint2 where;  // until the contact is taken
+    };
+    int32_t dsurf, src;
+};
+static_assert(sizeof(LeanAttempt) == 48, "a lean attempt is three 16-byte words");
+
 // What running an attempt takes, read by words of 16 bytes (a copy of the
 // struct goes through local memory).
 struct Terms {
@@ -422,6 +437,31 @@ struct Terms {
             tsd = w6.y;
         }
     }
+    __device__ __forceinline__ void read(const LeanAttempt *a, const LatView &L, bool surface) {
+        const int4 w0 = ((const int4 *)a)[0], w1 = ((const int4 *)a)[1];
+        cs = (uint32_t)w0.x;
+        cd = (uint32_t)w0.y;
+        dst = w0.w;
+        gi = (int64_t)(((uint64_t)(uint32_t)w1.y << 32) | (uint32_t)w1.x);
+        u0 = (uint32_t)w1.z;
+        u1 = (uint32_t)w1.w;
+        contact = a->contact;
+        dsurf = a->dsurf;
+        limit = (double)NAN;  // (the exponential is taken)
+        ls = ld = lss = lsd = 0.0;
+        ts = td = tss = tsd = 0;
+        next_s = next_d = NONE;
+        if (cs != NONE) {
+            ts = __ldg(L.target + cs);
+            ls = __ldg(L.lambda + cs);
+            if (surface) { tss = __ldg(L.tsurf + cs); lss = __ldg(L.lsurf + cs); }
+        }
+        if (cd != NONE) {
+            td = __ldg(L.target + cd);
+            ld = __ldg(L.lambda + cd);
+            if (surface) { tsd = __ldg(L.tsurf + cd); lsd = __ldg(L.lsurf + cd); }
+        }
+    }
 };
 
 constexpr int PT = 512;            // threads of a pass block; one block per SM
@@ -447,12 +487,12 @@ constexpr unsigned long long BARRIER_NS = 2000000000ull;
 // needs clearing.
 struct PassScratch {
     unsigned long long *claim[2];  // ncells each
-    Attempt *list;
+    void *list;                    // Attempt, or LeanAttempt without chains
     ulonglong2 *mail;              // per attempt
     uint32_t *idx, *link;          // per attempt: the blocks' lists (ready; pending, even rounds) and the lanes'
                                    // stacks (pending, odd rounds)
     uint32_t *count;               // per cell: the attempts listed (zero between passes)
-    unsigned long long *chain;     // per cell: CHAIN entries; null: every pass by rounds
+    unsigned long long *chain;     // per cell: CHAIN entries
     uint32_t seg;
     int32_t useg;                  // pixels a lane of an item reads (1 to UMAX)
     int64_t ncells;
@@ -680,7 +720,8 @@ struct PassShared {
 // TURNS attempts that a lane runs in turn.
 //
 // Rounds: a pass with a cell of more than CHAIN attempts (or records past
-// pack_records' ranges), or without room for the lists, runs by claims: every
+// pack_records' ranges), and every pass where there is no room for the lists
+// (LEAN), runs by claims: every
 // attempt claims its cells with its priority, one that holds all its claims
 // runs against the live records, the others claim again, a meeting of the
 // blocks between rounds.  The same sequence.
@@ -695,6 +736,7 @@ struct PassShared {
 // attempts deep) 1,750 -> 650 us, the 256^3 spheroid 1,830 -> 667, a 300 x 300
 // tissue (4 sub-sweeps of 2 passes) 840 -> 322, 256 x 256 265 -> 109, the 2048 x
 // 2048 cord 757 -> 426, the campaign's 22.3 M pixels 1,490 -> 1,360.
+template <bool LEAN>
 __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int nh, const int32_t *perm,
                                                      const uint32_t *mcs_cur, PassScratch S) {
     // a sweep queued after one that gave up does nothing: the barrier's words,
@@ -713,7 +755,9 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
     const uint32_t mcs = *mcs_cur;
     const uint32_t *pass_key = S.ctl + CTL_KEYS;
     const uint32_t id0 = blockIdx.x * S.seg;  // this block's first attempt
-    Attempt *const mine = S.list + id0;
+    using Record = std::conditional_t<LEAN, LeanAttempt, Attempt>;
+    Record *const mine = (Record *)S.list + id0;
+    Attempt *const list = (Attempt *)S.list;  // (chains)
     const int h0 = blockIdx.x < nvb ? plan_find(plan, nh, blockIdx.x) : 0;
     uint32_t seq = S.ctl[CTL_SEQ], bar = 0, left = 0, most = 0;
     const bool surf_on = L.surface_on != 0;
@@ -764,7 +808,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
             if (!copies) return;
             const uint32_t prio = fmix32((uint32_t)i ^ pkey);
             const uint32_t cs = src > 0 ? c0 + (uint32_t)src : NONE, cd = dst > 0 ? c0 + (uint32_t)dst : NONE;
-            if (S.chain) {
+            if constexpr (!LEAN) {
                 // both places taken at once
                 uint32_t ks = 0, kd = 0;
                 if (cs != NONE) ks = atomicAdd(S.count + cs, 1u);
@@ -776,8 +820,15 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                 if (max(ks, kd) >= CHAIN) P.odd = 1u;
                 S.mail[id0 + e] = make_ulonglong2(0ull, 0ull);
             }
-            int4 *const w = (int4 *)(mine + e);
             const int64_t gi = off + i;
+            if constexpr (LEAN) {
+                int4 *const w = (int4 *)(mine + e);
+                w[0] = make_int4((int)cs, (int)cd, (int)prio, dst);
+                w[1] = make_int4((int)(uint32_t)gi, (int)(gi >> 32), (int)r.y, (int)r.z);
+                w[2] = make_int4((int)px.x, (int)px.y, 0, src);
+                return;
+            }
+            int4 *const w = (int4 *)(mine + e);
             w[2] = make_int4(0, 0, (int)cs, (int)cd);
             w[3] = make_int4((int)NONE, (int)NONE, dst, 0);
             w[4] = make_int4((int)(uint32_t)gi, (int)(gi >> 32), (int)r.y, (int)r.z);
@@ -918,14 +969,14 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
         // (the next pass's count: last used by the pass before, which is over)
         if (blockIdx.x == 0 && threadIdx.x == 0) S.ctl[CTL_READY + ((pass + 1) & 1)] = 0u;
         if (left == 0) continue;
-        bool linked = S.chain != nullptr && flags == 0u;
+        bool linked = !LEAN && flags == 0u;
         const uint32_t tag0 = seq * ROUND_SPAN;  // round r claims with tag tag0 + r
         // round 1's claims
-        auto claim_first = [&](const Attempt &a) {
+        auto claim_first = [&](const Record &a) {
             const unsigned long long claim = ((unsigned long long)(tag0 + 1u) << 32) | a.prio;
             if (a.cs != NONE) atomicMax(S.claim[1] + a.cs, claim);
             if (a.cd != NONE) atomicMax(S.claim[1] + a.cd, claim);
-            if (S.chain) {
+            if (!LEAN) {
                 if (a.cs != NONE) S.count[a.cs] = 0u;
                 if (a.cd != NONE) S.count[a.cd] = 0u;
             }
@@ -935,7 +986,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
         // exchange; one cell a warp, dense planes of 16.8 M pixels took 2.00 ms a
         // step, now 1.69, and 2.70 -> 1.87 with the nine passes of order 3); each
         // entry's follower into its attempt, and the cell's records to the first
-        if (linked) {
+        if constexpr (!LEAN) if (linked) {
             uint32_t *const found = (uint32_t *)P.edge[warp];
             uint32_t have = 0;  // ready attempts found and not yet in the list, the same in every lane
             auto flush = [&](uint32_t m) {
@@ -991,7 +1042,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                         bool ready = false;
                         const uint32_t id = ((uint32_t)own >> 2);
                         if (gl + 32u * half < k) {
-                            if (followed) (own & 1ull ? S.list[id].next_d : S.list[id].next_s) = (uint32_t)below;
+                            if (followed) (own & 1ull ? list[id].next_d : list[id].next_s) = (uint32_t)below;
                             if (first) {
                                 const unsigned long long box = pack_records(vol, surf, 0u);
                                 unsigned long long met = 0ull;
@@ -1029,14 +1080,27 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
         // read before anything is written: a write between two reads that it might
         // change holds the second until the first has come.
         for (uint32_t e = threadIdx.x; e < n; e += PT) {
-            Attempt *const a = mine + e;
+            Record *const a = mine + e;
             if (!linked) claim_first(*a);
-            const int4 w2 = ((const int4 *)a)[2], w3 = ((const int4 *)a)[3], w4 = ((const int4 *)a)[4], w6 = ((const int4 *)a)[6],
-                       w7 = ((const int4 *)a)[7];
-            const uint32_t cs = (uint32_t)w2.z, cd = (uint32_t)w2.w;
-            const int32_t dst = w3.z, src = w6.w;
-            const int hh = w7.x & 0xFFFF;
-            const int x = w7.y & 0xFFFF, y = (int)((uint32_t)w7.y >> 16), z = (int)((uint32_t)w7.x >> 16);
+            uint32_t cs = 0, cd = 0;
+            int32_t dst, src;
+            uint2 where, u = make_uint2(0u, 0u);
+            if constexpr (LEAN) {
+                dst = a->dst;
+                src = a->src;
+                where = a->where;
+            } else {
+                const int4 w2 = ((const int4 *)a)[2], w3 = ((const int4 *)a)[3], w4 = ((const int4 *)a)[4],
+                           w6 = ((const int4 *)a)[6], w7 = ((const int4 *)a)[7];
+                cs = (uint32_t)w2.z;
+                cd = (uint32_t)w2.w;
+                dst = w3.z;
+                src = w6.w;
+                where = make_uint2((uint32_t)w7.x, (uint32_t)w7.y);
+                u = make_uint2((uint32_t)w4.z, (uint32_t)w4.w);
+            }
+            const int hh = (int)(where.x & 0xFFFFu);
+            const int x = (int)(where.y & 0xFFFFu), y = (int)(where.y >> 16), z = (int)(where.x >> 16);
             const int4 dm = __ldg(L.dims + hh);
             const int64_t c0 = __ldg(L.cell_off + hh), cap = __ldg(L.cell_off + hh + 1) - c0;
             const int64_t i = ((int64_t)z * dm.y + y) * dm.x + x;
@@ -1044,12 +1108,12 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
             const Vn vn = vn_of(dm, x, y, z);
             int32_t ts = 0, td = 0, tss = 0, tsd = 0;
             double ls = 0.0, ld = 0.0, lss = 0.0, lsd = 0.0;
-            if (cs != NONE) {
+            if (!LEAN && cs != NONE) {
                 ts = __ldg(L.target + cs);
                 ls = __ldg(L.lambda + cs);
                 if (surf_on) { tss = __ldg(L.tsurf + cs); lss = __ldg(L.lsurf + cs); }
             }
-            if (cd != NONE) {
+            if (!LEAN && cd != NONE) {
                 td = __ldg(L.target + cd);
                 ld = __ldg(L.lambda + cd);
                 if (surf_on) { tsd = __ldg(L.tsurf + cd); lsd = __ldg(L.lsurf + cd); }
@@ -1059,14 +1123,20 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
             double num;
             const double contact = contact_delta(g, dm, x, y, z, src, dst, L.type + c0, cap, P.J, L.K, P.reach, L.nreach,
                                                  L.across, i, vn, &num);
-            const double limit = accept_limit((uint32_t)w4.z, (uint32_t)w4.w, L.temperature);
+            const int32_t surfs = (int32_t)((uint32_t)(uint16_t)(int16_t)ds | ((uint32_t)(uint16_t)(int16_t)dd << 16));
+            a->dsurf = surfs;
+            if constexpr (LEAN) {
+                a->contact = contact;
+                continue;
+            } else {
+            const double limit = accept_limit(u.x, u.y, L.temperature);
             ((double2 *)a)[0] = make_double2(contact, limit);
             ((double2 *)a)[1] = make_double2(ls, ld);
             *(int2 *)&a->ts = make_int2(ts, td);
-            a->dsurf = (int32_t)((uint32_t)(uint16_t)(int16_t)ds | ((uint32_t)(uint16_t)(int16_t)dd << 16));
             if (surf_on) {
                 ((double2 *)a)[5] = make_double2(lss, lsd);
                 *(int2 *)&a->tss = make_int2(tss, tsd);
+            }
             }
         }
         __syncthreads();
@@ -1091,7 +1161,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
             sd += dd;
             return true;
         };
-        if (linked) {
+        if constexpr (!LEAN) if (linked) {
             // ---- run the chains: a lane takes what it made ready, else its spare or
             // its stack, else its next of the list, else another lane's spare
             // (dealt one to a warp, then a second to each: the chains of a warp
@@ -1186,7 +1256,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                     }
                     if (id != NONE) {
                         Terms a;
-                        a.read(S.list + id, surf_on);
+                        a.read(list + id, surf_on);
                         const uint32_t cs = a.cs, cd = a.cd;
                         uint32_t depth = 0;
                         int32_t vs = 0, ss = 0, vd = 0, sd = 0;
@@ -1209,7 +1279,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                             if (next[side] != NONE) {
                                 const uint32_t to = next[side] >> 2;
                                 // its terms into L1 while the exchange is on its way
-                                const char *line = (const char *)(S.list + to);
+                                const char *line = (const char *)(list + to);
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     uint32_t t;
@@ -1277,7 +1347,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                 const uint32_t k = has ? (r == 1 ? e : pin[e]) : 0u;
                 bool again = false;
                 if (has) {
-                    const Attempt &a = mine[k];
+                    const Record &a = mine[k];
                     const unsigned long long key = ((unsigned long long)(tag0 + r) << 32) | a.prio;
                     unsigned long long ks = key, kd = key;
                     if (a.cs != NONE) ks = __ldcg(cl + a.cs);
@@ -1287,7 +1357,8 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                         if (a.cs != NONE) { vs = L.volume[a.cs]; if (surf_on) ss = L.surface[a.cs]; }
                         if (a.cd != NONE) { vd = L.volume[a.cd]; if (surf_on) sd = L.surface[a.cd]; }
                         Terms t;
-                        t.read(&a, surf_on);
+                        if constexpr (LEAN) t.read(&a, L, surf_on);
+                        else t.read(&a, surf_on);
                         if (attempt(t, vs, ss, vd, sd)) {
                             // the records: its cells are its own this round
                             if (a.cs != NONE) { L.volume[a.cs] = vs; if (surf_on) L.surface[a.cs] = ss; }
@@ -1456,7 +1527,7 @@ int cw_lattice_s::build_plans() {
     int rc;
     if (pass_grid == 0) {
         int per_sm = 0, dev = 0, nsm = 0;
-        CW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_cpm_sweep, PT, 0));
+        CW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_cpm_sweep<false>, PT, 0));
         CW_CUDA(cudaGetDevice(&dev));
         CW_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         pass_grid = std::max(1, per_sm > 0 ? nsm : 0);
@@ -1499,37 +1570,50 @@ int cw_lattice_s::build_plans() {
 // usually has).
 int cw_lattice_s::ensure_scratch() {
     int rc;
-    const int64_t need = (int64_t)pass_blocks * pass_seg;
-    if (need > plist_cap) {
-        ++plans;
-        dfree(plist);
-        dfree(pidx);
-        dfree(pmail);
-        plist_cap = 0;
-        if ((rc = dalloc(&plist, sizeof(Attempt) / sizeof(uint4) * (size_t)need)) != CW_OK) return rc;
-        if ((rc = dalloc(&pidx, 2 * (size_t)need)) != CW_OK) return rc;
-        if ((rc = dalloc(&pmail, (size_t)need)) != CW_OK) return rc;
-        plist_cap = need;
-    }
     if (!claim) {
         if ((rc = dalloc(&claim, 2 * (size_t)ncells)) != CW_OK) return rc;
         CW_CUDA(cudaMemsetAsync(claim, 0, sizeof(unsigned long long) * 2 * (size_t)ncells, stream()));
     }
-    // the cells' lists, 512 bytes a record: a batch of so many records that they
-    // would take more than 1 GiB, or a device without the room, runs its passes
-    // by rounds (so does one of more than 2^30 attempts, which a list's entry
-    // does not number)
-    if (!chain_tried && ncells * (int64_t)(CHAIN * sizeof(unsigned long long)) <= (1ll << 30)) {
-        chain_tried = true;
-        if (cudaMalloc((void **)&pcount, sizeof(uint32_t) * (size_t)ncells) != cudaSuccess ||
-            cudaMalloc((void **)&pchain, sizeof(unsigned long long) * CHAIN * (size_t)ncells) != cudaSuccess) {
-            (void)cudaGetLastError();
-            dfree(pcount);
-            pchain = nullptr;
-        } else {
-            CW_CUDA(cudaMemsetAsync(pcount, 0, sizeof(uint32_t) * (size_t)ncells, stream()));
+    const int64_t need = (int64_t)pass_blocks * pass_seg;
+    if (need <= plist_cap) return CW_OK;
+    ++plans;
+    dfree(plist);
+    dfree(pidx);
+    dfree(pmail);
+    plist_cap = 0;
+    // By chains: 152 bytes a pixel slot of a colour, and the cells' lists, 516
+    // bytes a record, where all this is at most a quarter of the memory that is
+    // free (and a list's entry can number the attempts).  Else, or where it could
+    // not be had, by rounds: 56 bytes a slot, as fast within a twentieth on large
+    // lattices (3.79 ms a step of 33.6 M pixels against 3.61) and half as fast on
+    // small ones.
+    const size_t chains = (sizeof(Attempt) + sizeof(ulonglong2) + 2 * sizeof(uint32_t)) * (size_t)need;
+    const size_t lists = pchain ? 0 : (CHAIN * sizeof(unsigned long long) + sizeof(uint32_t)) * (size_t)ncells;
+    size_t unused = 0, whole = 0;
+    CW_CUDA(cudaMemGetInfo(&unused, &whole));
+    lean = need >= (1ll << 30) || chains + lists > unused / 4;
+    if (!lean) {
+        auto take = [](auto **p, size_t n) {
+            return *p || cudaMalloc((void **)p, sizeof(**p) * n) == cudaSuccess;
+        };
+        const bool counts = pcount == nullptr;
+        if (take(&plist, sizeof(Attempt) / sizeof(uint4) * (size_t)need) && take(&pidx, 2 * (size_t)need) &&
+            take(&pmail, (size_t)need) && take(&pcount, (size_t)ncells) && take(&pchain, CHAIN * (size_t)ncells)) {
+            if (counts) CW_CUDA(cudaMemsetAsync(pcount, 0, sizeof(uint32_t) * (size_t)ncells, stream()));
+            plist_cap = need;
+            return CW_OK;
         }
+        (void)cudaGetLastError();
+        lean = true;
+        dfree(plist);
+        dfree(pidx);
+        dfree(pmail);
     }
+    dfree(pcount);
+    dfree(pchain);
+    if ((rc = dalloc(&plist, sizeof(LeanAttempt) / sizeof(uint4) * (size_t)need)) != CW_OK) return rc;
+    if ((rc = dalloc(&pidx, 2 * (size_t)need)) != CW_OK) return rc;
+    plist_cap = need;
     return CW_OK;
 }
 
@@ -1654,12 +1738,12 @@ int lattice_subsweep(cw_lattice_s *l) {
     PassScratch S;
     S.claim[0] = l->claim;
     S.claim[1] = l->claim + l->ncells;
-    S.list = (Attempt *)l->plist;
+    S.list = l->plist;
     S.mail = l->pmail;
     S.idx = l->pidx;
     S.link = l->pidx + l->plist_cap;
     S.count = l->pcount;
-    S.chain = l->plist_cap < (1ll << 30) ? l->pchain : nullptr;
+    S.chain = l->pchain;
     S.useg = l->useg;
     S.seg = (uint32_t)l->pass_seg;
     S.ncells = l->ncells;
@@ -1682,7 +1766,7 @@ int lattice_subsweep(cw_lattice_s *l) {
     cfg.stream = stream();
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CW_CUDA(cudaLaunchKernelExC(&cfg, (const void *)k_cpm_sweep, args));
+    CW_CUDA(cudaLaunchKernelExC(&cfg, l->lean ? (const void *)k_cpm_sweep<true> : (const void *)k_cpm_sweep<false>, args));
     count_launch(1);
     return CW_OK;
 }

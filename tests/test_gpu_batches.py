@@ -98,3 +98,26 @@ def test_a_pass_of_many_turns():
     lat = cw.CpmLattice.from_grids([grid], [rec], 10.0, J3, 1, seeds=[5])
     lat.monte_carlo_step(2)
     same_as_the_oracle(lat, 0, grid, rec, 1, 2, 5)
+
+
+@pytest.mark.parametrize("shape,side,order,surface", [((150, 131, 1), 7, 2, False), ((150, 131, 1), 7, 1, True),
+                                                      ((40, 33, 36), 5, 2, True)])
+def test_passes_without_room_for_the_cells_lists(shape, side, order, surface):
+    # so many records that their lists would take a third of the device: every
+    # pass by rounds, its attempts' constants read from the records
+    grid, rec = packed(shape, side, 3)
+    lat = cw.CpmLattice.from_grids([grid], [rec], 10.0, J3, order, seeds=[21], capacity=120_000_000)
+    t, v, tg, lam = rec.arrays()
+    d, h, w = grid.shape
+    o = O.Lattice(grid, (w, h, d), len(rec), J3, 10.0, order)
+    o.type[:], o.volume[:], o.target[:], o.lam[:] = t, v, tg, lam
+    if surface:
+        ts, ls = np.full(len(rec), 40, np.int32), np.full(len(rec), 0.3)
+        o.enable_surface(ts, ls)
+        lat.set_surface(ts, ls)
+    lat.monte_carlo_step(4)
+    o.mcs_checkerboard(21, 0, 4)
+    np.testing.assert_array_equal(lat.grid().reshape(-1), o.grid)
+    np.testing.assert_array_equal(lat.cells(len(rec))["volume"][1:], o.volume[1:])
+    if surface:
+        np.testing.assert_array_equal(lat.surfaces(len(rec))[1:], o.surface[1:])
