@@ -60,11 +60,13 @@ struct Part {
     int32_t g[3];          // tiles along x, y, z
     int32_t k;             // half-sweeps a round (even)
     int32_t most;          // volumes: pixels of a colour in its largest window
+    int64_t shift;         // pixel i of the batch stands at other[i - shift]
 };
 
 struct Args {
     FieldView fv;
-    double *other;                // the second buffer of the exchange
+    double *other;                // the second buffer of the exchange: of each history the run of pixels that its
+                                  // windows read
     const Part *parts;
     int nparts;
     RelaxState *st;
@@ -211,7 +213,7 @@ __device__ __forceinline__ Part part_of(const Args &a) {
 // A history's solve, by all its blocks: rounds of pt.k half-sweeps and a
 // meeting.  load(src, halo): the window's pixels (halo: all but the interior's
 // free ones) from a buffer, ready to be swept when it returns; store(dst): the
-// interior out to a buffer; sweep(n): n sweeps of the window, each warp's
+// interior's free ones out to a buffer; sweep(n): n sweeps of the window, each warp's
 // maxima into S.part (the changes, then from MAX_S the residuals) before its
 // last block barrier or this function's first; worst(): the interior's
 // largest residual.
@@ -222,6 +224,7 @@ __device__ __forceinline__ void solve_rounds(const Args &a, const Part &pt, Load
     const double tol = a.st[h].tol;
     uint32_t *arrivals = a.arrivals + h;
     unsigned long long *slots = a.slots + (size_t)h * 3 * SLOTS;
+    double *const other = a.other - pt.shift;
     long long taken = 0;
     uint32_t meetings = 0;
     int cur = 0, settled = 0;
@@ -234,7 +237,7 @@ __device__ __forceinline__ void solve_rounds(const Args &a, const Part &pt, Load
     for (int round = 0; taken < a.max_sweeps; ++round) {
         const int n = (int)min((long long)(pt.k / 2), a.max_sweeps - taken);
         sweep(n);
-        store(cur ? a.fv.c : a.other);
+        store(cur ? a.fv.c : other);
         __syncthreads();
         unsigned long long *set = slots + (round % 3) * SLOTS;
         if (tid < SLOTS && ((tid < n) || (RES && tid >= MAX_S && tid - MAX_S < n))) {
@@ -246,7 +249,7 @@ __device__ __forceinline__ void solve_rounds(const Args &a, const Part &pt, Load
         if (tid < SLOTS) S.all[tid] = __ldcg(set + tid);
         // last read before the meeting that has just ended
         if (b == 0 && tid < SLOTS) slots[((round + 2) % 3) * SLOTS + tid] = 0ull;
-        load(cur ? a.fv.c : a.other, true);
+        load(cur ? a.fv.c : other, true);
         int s = 0;
         for (; s < n; ++s) {
             change = __longlong_as_double((long long)S.all[s]);
@@ -262,7 +265,7 @@ __device__ __forceinline__ void solve_rounds(const Args &a, const Part &pt, Load
             // the round again from its start, as far as the sweep that settled;
             // where that start is the field itself, every block has read it
             // before any writes it
-            load(cur ? a.other : a.fv.c, false);
+            load(cur ? other : a.fv.c, false);
             if (cur == 0 && !met()) return;
             sweep(kept);
             store(a.fv.c);
@@ -496,6 +499,15 @@ __global__ void __launch_bounds__(RT, 1) k_relax64_plane(Args a) {
     };
     __syncthreads();  // the published rows' zeros
     load(fv.c, false);
+    // the window's held pixels into the other buffer too, before the first meeting
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        const int gy = gy0 + j;
+        double *p = a.other - pt.shift + off + (int64_t)gy * dm.x + gx;
+        const bool iny = gy >= 0 && gy < dm.y;
+        if (iny && inx && !((free_a >> j) & 1u)) p[0] = va[j];
+        if (iny && inx1 && !((free_b >> j) & 1u)) p[1] = vb[j];
+    }
     solve_rounds<RES>(a, pt, load, store, sweep, [&]() {
         unsigned long long worst = 0ull;
         residual(Red(), worst);
@@ -677,7 +689,6 @@ __global__ void __launch_bounds__(RT, 1) k_relax64_volume(Args a) {
         own(0, it0, at0, mine0, cur0, up0);
         own(1, it1, at1, mine1, cur1, up1);
     }
-    // (held pixels are read once, above)
     auto take = [&](const double *src, bool halo, auto &it, auto &place, unsigned mine, auto &cur) {
 #pragma unroll
         for (int j = 0; j < PP; ++j)
@@ -894,6 +905,8 @@ namespace cw {
 // exchange, the tilings of its histories and the words they meet on.
 struct Resident64 {
     double *other = nullptr;
+    size_t other_size = 0;         // its numbers, and those the tilings need
+    size_t other_need = 0;
     Part *parts = nullptr;
     uint32_t *words = nullptr;     // arrivals, whether a meeting failed, then the slots
     std::vector<Part> host;
@@ -946,6 +959,7 @@ static int resident64_plan(cw_field_s *f, Resident64 *r, const FieldView &fv, co
         ++live;
     }
     if (live == 0 || live > r->nsm) return CW_OK;
+    int64_t rows = 0;  // planes: a window's rows
     // a block for each history, the others by size
     std::vector<Part> parts;
     std::vector<int> blocks;
@@ -994,19 +1008,38 @@ static int resident64_plan(cw_field_s *f, Resident64 *r, const FieldView &fv, co
         }
         if (best.empty()) return CW_OK;
         parts = best;
+        rows = with.R * (with.threads / with.G);
         r->threads = with.threads;
         r->smem = plane_smem(with, gen, fv.pr, fv.up);
         r->kern[0] = gen ? plane_of<false, true>(with) : plane_of<false, false>(with);
         r->kern[1] = gen ? plane_of<true, true>(with) : plane_of<true, false>(with);
     }
     int first = 0;
+    r->other_need = 0;
     for (Part &p : parts) {
         p.first = first;
         first += p.nblocks;
+        // a volume's free slices, a plane's rows from the first of a window to the
+        // last (`rows` of them below the window's first)
+        const int64_t w = f->g.w[p.h], h = f->g.h[p.h];
+        int64_t from, to;
+        if (volume) {
+            from = (int64_t)p.lo[2] * h * w;
+            to = (int64_t)(p.lo[2] + p.n[2]) * h * w;
+        } else {
+            from = std::max(p.lo[1] - 2, 0) * w;
+            to = std::min<int64_t>(p.lo[1] + p.n[1] + rows, h) * w;
+        }
+        p.shift = f->g.off[p.h] + from - (int64_t)r->other_need;
+        r->other_need += (size_t)(to - from);
     }
     r->host = parts;
-    int rc;
-    if (!r->parts && (rc = dalloc(&r->parts, f->g.nh)) != CW_OK) return rc;
+    if (!r->parts && cudaMalloc((void **)&r->parts, sizeof(Part) * f->g.nh) != cudaSuccess) {
+        r->parts = nullptr;
+        (void)cudaGetLastError();
+        r->spans.clear();  // (tried again by the next solve)
+        return CW_OK;
+    }
     CW_CUDA(cudaMemcpyAsync(r->parts, r->host.data(), sizeof(Part) * r->host.size(), cudaMemcpyHostToDevice, stream()));
     r->served = true;
     return CW_OK;
@@ -1034,18 +1067,21 @@ int relax64_resident(cw_field_s *f, const cw_relax_opts &o, const std::vector<Sp
     if (rc != CW_OK || !r->served) return rc;
     const size_t slots = ((size_t)nh + 2) & ~(size_t)1;  // (64-bit words)
     const size_t words = slots + 2 * (size_t)nh * 3 * SLOTS;
-    if (!r->other || !r->words) {
-        // a device without room for the scratch serves the solve by launches
-        if (!r->other && cudaMalloc((void **)&r->other, sizeof(double) * (size_t)f->g.total) != cudaSuccess) {
+    // a device without room for the scratch serves the solve by launches
+    if (r->other_need > r->other_size) {
+        dfree(r->other);
+        r->other_size = 0;
+        if (cudaMalloc((void **)&r->other, sizeof(double) * r->other_need) != cudaSuccess) {
             r->other = nullptr;
             (void)cudaGetLastError();
             return CW_OK;
         }
-        if (!r->words && cudaMalloc((void **)&r->words, sizeof(uint32_t) * words) != cudaSuccess) {
-            r->words = nullptr;
-            (void)cudaGetLastError();
-            return CW_OK;
-        }
+        r->other_size = r->other_need;
+    }
+    if (!r->words && cudaMalloc((void **)&r->words, sizeof(uint32_t) * words) != cudaSuccess) {
+        r->words = nullptr;
+        (void)cudaGetLastError();
+        return CW_OK;
     }
     const bool res = o.stop == CW_STOP_RESIDUAL;
     const Resident kern = r->kern[res ? 1 : 0];
@@ -1083,8 +1119,6 @@ int relax64_resident(cw_field_s *f, const cw_relax_opts &o, const std::vector<Sp
         }
         a.max_sweeps = std::min<long long>(LAUNCH_SWEEPS, o.max_sweeps - taken);
         CW_CUDA(cudaMemsetAsync(r->words, 0, sizeof(uint32_t) * words, stream()));
-        CW_CUDA(cudaMemcpyAsync(r->other, f->c, sizeof(double) * (size_t)f->g.total, cudaMemcpyDeviceToDevice,
-                                stream()));
         const cudaError_t launched = cudaLaunchKernelExC(&cfg, (const void *)kern, args);
         if (launched == cudaErrorCooperativeLaunchTooLarge && taken == 0) {
             // fewer SMs for this process than the device has: by launches

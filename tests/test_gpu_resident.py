@@ -149,3 +149,55 @@ def test_a_solve_of_more_sweeps_than_a_launch_takes_carries_on():
     o = O.Field(*shapes[0], 0.2, 0.0, 0.0)
     o.held[:], o.values[:], o.uptake[:] = ps[0][0], wants[0][0], ps[0][2]
     assert st[0]["residual"] == o.residual()
+
+
+def test_a_small_tissue_in_a_large_box_takes_little_beside_its_field():
+    torch = pytest.importorskip("torch")
+
+    def tissue(n, z0):
+        free = np.zeros((n, n, n), bool)
+        free[z0:z0 + 20, 40:60, 30:70] = True
+        held = (~free).reshape(-1).astype(np.uint8)
+        values = np.random.default_rng(1).uniform(0.0, 1.0, n**3)
+        return held, values, np.where(held, 0.0, 1e-4)
+
+    shape = (256, 256, 256)
+    small = field((100, 100, 100), tissue(100, 40))
+    small.relax(1e-6, 1000, omega=1.7)  # the kernel loaded
+    p = tissue(256, 100)
+    g = field(shape, p)
+    before = torch.cuda.mem_get_info()[0]
+    counts = [g.relax(1e-6, 1000, omega=1.7)]
+    taken = before - torch.cuda.mem_get_info()[0]
+    # 20 of 256 slices of 8 bytes a voxel (10.5 MB), a few allocations of 2 MB
+    assert taken <= 20 * 256 * 256 * 8 + (8 << 20)
+    # and the tissue moves, to slices that buffer has not held
+    moved = tissue(256, 180)
+    for held, values, uptake in (p, moved):
+        g.set_held(held)
+        g.set_values(values)
+        g.set_uptake_array(uptake)
+        counts.append(g.relax(1e-6, 1000, omega=1.7))
+        want, sweeps = solved(shape, (held, values, uptake), 1.7, 1e-6)
+        assert counts[-1] == sweeps
+        np.testing.assert_array_equal(bits(g.values()), bits(want))
+    assert counts[0] == counts[1]
+
+
+def test_a_tissue_that_moves_through_a_plane_is_solved_as_the_oracles():
+    # rows of the second buffer that no solve has held, windows cut by the box's
+    # border, a larger and a smaller tissue in turn
+    shape = (900, 700, 1)
+    g = cw.ScalarField([shape], 0.2, 0.0, 0.0)
+    rng = np.random.default_rng(2)
+    for x, y, w, h in ((400, 300, 60, 40), (700, 640, 200, 60), (0, 0, 90, 30), (100, 200, 500, 160), (450, 690, 8, 10)):
+        free = np.zeros((700, 900), bool)
+        free[y:y + h, x:x + w] = rng.random((h, w)) < 0.97
+        held = (~free).reshape(-1).astype(np.uint8)
+        p = held, np.where(held, rng.uniform(0.5, 1.0, held.size), rng.uniform(0.0, 1.0, held.size)), np.where(held, 0.0, 1e-4)
+        g.set_held(p[0])
+        g.set_values(p[1])
+        g.set_uptake_array(p[2])
+        want, sweeps = solved(shape, p, 1.8)
+        assert g.relax(1e-7, 100_000, omega=1.8) == sweeps
+        np.testing.assert_array_equal(bits(g.values()), bits(want))
