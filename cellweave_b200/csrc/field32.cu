@@ -84,8 +84,10 @@ __device__ __forceinline__ void half_sweep(float (&d0)[ROWS], float (&d1)[ROWS],
     }
 }
 
+// (src not restricted: an overlapped launch's blocks are there while the launch
+// before still writes it, which the read-only path does not allow for)
 template <int DEPTH>
-__global__ void __launch_bounds__(32 * WARPS) k_sor32_tb(const float *__restrict__ src, float *__restrict__ dst,
+__global__ void __launch_bounds__(32 * WARPS) k_sor32_tb(const float *src, float *__restrict__ dst,
                                                          const float *__restrict__ rhs, const float *__restrict__ inv,
                                                          const int4 *__restrict__ dims,
                                                          const int64_t *__restrict__ off,
