@@ -446,6 +446,7 @@ struct cw_field_s {
     void *stats = nullptr;           // per-history solve state (device)
     cw::Span *d_span = nullptr;
     void *dc_cache = nullptr;        // plans and solver of the FP32 solve (field.cu)
+    uint32_t *waits = nullptr;       // whether a wait of its FP32 sweeps, of its residuals, ran out
     cw::Resident64 *resident = nullptr;  // tilings and scratch of the FP64 solve on chip (field64.cu)
     cw_field_s *adjoint = nullptr;   // twin of cw_field_relax_adjoint, made on its first call
     cw::Plan inflow_plan;            // every site, for the inflow enqueued inside a step

@@ -497,6 +497,10 @@ int cw_field_s::alloc_fp32() {
     if (r32) return CW_OK;
     int rc;
     int64_t n = g.total;
+    if (!waits) {
+        if ((rc = dalloc(&waits, 2)) != CW_OK) return rc;
+        CW_CUDA(cudaMemsetAsync(waits, 0, 2 * sizeof(uint32_t), stream()));
+    }
     if ((rc = dalloc(&r32, n)) != CW_OK) return rc;
     if ((rc = dalloc(&d32a, n)) != CW_OK) return rc;
     if ((rc = dalloc(&d32b, n)) != CW_OK) return rc;
@@ -629,7 +633,6 @@ constexpr int RT_MAX_STAGES = 6;
 constexpr int RT_MAPS = 5;                         // per history: values, held, sink, production, uptake
 constexpr int RT_SMEM = 100 * 1024;                // two blocks per SM: the stages of a block fit in this
 
-__device__ int g_rt_wait_failed;
 
 // A tile as the host lays it out: its history, corner and the history's
 // shape and first pixel.
@@ -652,6 +655,7 @@ struct RtArgs {
     int stage;                // bytes of one stage
     int o_held, o_ks, o_pr, o_up;  // offsets in a stage, -1 for an absent array
     uint32_t tx;              // bytes one stage receives
+    uint32_t *failed;         // set where a wait ran out
 };
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
@@ -718,7 +722,7 @@ __global__ void __launch_bounds__(RT_THREADS, 2)
                         if (a.o_pr >= 0) tma_load_2d(stage + a.o_pr, m + 3, bar, v.t.x0, v.t.y0);
                         if (a.o_up >= 0) tma_load_2d(stage + a.o_up, m + 4, bar, v.t.x0, v.t.y0);
                     } else {
-                        atomicExch(&g_rt_wait_failed, 1);
+                        atomicExch(a.failed, 1u);
                     }
                 }
                 ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -733,7 +737,7 @@ __global__ void __launch_bounds__(RT_THREADS, 2)
                         s_tile[slot].t.h = -1;
                         mbar_arrive(sh_addr(&full[slot]));
                     } else {
-                        atomicExch(&g_rt_wait_failed, 1);
+                        atomicExch(a.failed, 1u);
                     }
                 }
                 stop = true;
@@ -745,7 +749,7 @@ __global__ void __launch_bounds__(RT_THREADS, 2)
     for (int it = 0;; ++it) {
         const int slot = it % a.stages;
         if (!mbar_wait_bounded(sh_addr(&full[slot]), (uint32_t)(it / a.stages) & 1u)) {
-            atomicExch(&g_rt_wait_failed, 1);
+            atomicExch(a.failed, 1u);
             break;
         }
         const RtStaged v = s_tile[slot];
@@ -908,6 +912,7 @@ static int rt_prepare(cw_field_s *f, ResTiles &rt) {
     CW_CUDA(cudaStreamSynchronize(stream()));
     a.maps = rt.maps;
     a.tiles = rt.tiles;
+    a.failed = f->waits + 1;
     a.ntiles = (int)tiles.size();
     rt.grid = std::min<int>(a.ntiles, per_sm * nsm);
     const void *on[RT_MAPS] = {fv.c, fv.held, fv.ks, fv.pr, fv.up};
@@ -916,23 +921,16 @@ static int rt_prepare(cw_field_s *f, ResTiles &rt) {
     return CW_OK;
 }
 
-static int rt_wait_failed();
-
-// Whether a staged copy of the FP32 sweeps or of the residual timed out.
-static int dc_waits_failed() {
-    int rc = sor32_wait_failed();
-    return rc != CW_OK ? rc : rt_wait_failed();
-}
-
-static int rt_wait_failed() {
-    int v = 0;
-    CW_CUDA(cudaMemcpyFromSymbol(&v, g_rt_wait_failed, sizeof v));
-    if (v) {
-        const int zero = 0;
-        CW_CUDA(cudaMemcpyToSymbol(g_rt_wait_failed, &zero, sizeof zero));
-        return fail(CW_ERR_TIMEOUT, "a residual tile's copy did not land in time");
-    }
-    return CW_OK;
+// Whether a staged copy of the field's FP32 sweeps or of its residuals timed out
+// (and clears the record).
+static int dc_waits_failed(cw_field_s *f) {
+    uint32_t v[2] = {0u, 0u};
+    CW_CUDA(cudaMemcpyAsync(v, f->waits, sizeof v, cudaMemcpyDeviceToHost, stream()));
+    CW_CUDA(cudaStreamSynchronize(stream()));
+    if (!v[0] && !v[1]) return CW_OK;
+    CW_CUDA(cudaMemsetAsync(f->waits, 0, sizeof v, stream()));
+    return fail(CW_ERR_TIMEOUT, v[0] ? "an FP32 SOR block waited too long for its window's TMA copies"
+                                     : "a residual tile's copy did not land in time");
 }
 
 // Launch plans and the FP32 solver of the defect-correction solve, built on a
@@ -1068,7 +1066,7 @@ static int relax_fp32dc(cw_field_s *f, const cw_relax_opts &o, RelaxState *d_st,
             if ((rc = dc_outer(f, c, d_st, inner, o.max_sweeps, start)) != CW_OK) return rc;
         CW_CUDA(cudaMemcpyAsync(hs.data(), d_st, sizeof(RelaxState) * nh, cudaMemcpyDeviceToHost, stream()));
         CW_CUDA(cudaStreamSynchronize(stream()));
-        if ((rc = dc_waits_failed()) != CW_OK) return rc;
+        if ((rc = dc_waits_failed(f)) != CW_OK) return rc;
         bool all = true;
         for (uint32_t k = 0; k < nh; ++k) all = all && hs[k].done;
         if (all) break;
@@ -1142,7 +1140,7 @@ int field_relax_collect(cw_field_s *f, std::vector<cw_relax_stats> &out, bool &a
     std::vector<RelaxState> hs(nh);
     CW_CUDA(cudaMemcpyAsync(hs.data(), f->stats, sizeof(RelaxState) * nh, cudaMemcpyDeviceToHost, stream()));
     CW_CUDA(cudaStreamSynchronize(stream()));
-    int rc = dc_waits_failed();
+    int rc = dc_waits_failed(f);
     if (rc != CW_OK) return rc;
     out.resize(nh);
     all_settled = true;
@@ -1194,7 +1192,7 @@ int cw_field_destroy(cw_field f) {
     if (!f) return CW_OK;
     CW_SCOPE(f);
     dfree(f->c); dfree(f->held); dfree(f->uptake); dfree(f->production); dfree(f->lin_sink);
-    dfree(f->r32); dfree(f->d32a); dfree(f->d32b); dfree(f->inv32); dfree(f->tmp64); dfree(f->d_span);
+    dfree(f->r32); dfree(f->d32a); dfree(f->d32b); dfree(f->inv32); dfree(f->waits); dfree(f->tmp64); dfree(f->d_span);
     if (f->dc_cache) {
         DcCache *c = (DcCache *)f->dc_cache;
         c->solver.release();
@@ -1631,7 +1629,7 @@ extern "C" int cw_field_time_inner(cw_field f, int32_t sweeps, int32_t depth, in
     f->last_inner = solver.result();
     solver.release();
     prow.release();
-    return dc_waits_failed();
+    return dc_waits_failed(f);
 }
 
 extern "C" int cw_field_inner_correction(cw_field f, uint32_t hist, float *out) {

@@ -191,7 +191,6 @@ constexpr int WROWS = 16;            // rows per warp; a window has WROWS rows p
 constexpr size_t wide_smem(int warps) {
     return (size_t)3 * WX * WROWS * warps * sizeof(float) + (size_t)2 * (warps + 2) * 2 * (WX / 4) * sizeof(float4);
 }
-__device__ int g_wide_wait_failed;
 
 // One half-sweep of colour C over a lane's WROWS rows x 4 columns.  Column c
 // of row j has colour (c + j) mod 2 (windows start at even x and y): colour C
@@ -254,7 +253,8 @@ __global__ void __launch_bounds__(32 * WWARPS, WWARPS * WROWS == 64 ? 2 : 1)
                  const int4 *__restrict__ tiles, int ntiles, const int4 *__restrict__ dims,
                  const int64_t *__restrict__ off, const float *__restrict__ omega, const int32_t *done,
                  int done_stride, int nhalf, int zero_start, double *__restrict__ apply_c,
-                 int floor, unsigned long long wait_ns, int skip_copies, unsigned long long *corr, int corr_stride) {
+                 int floor, unsigned long long wait_ns, int skip_copies, unsigned long long *corr, int corr_stride,
+                 uint32_t *failed) {
     constexpr int WY = WROWS * WWARPS;  // window rows
     constexpr int STAGE = WX * WY;      // floats per array of the staged window
     extern __shared__ __align__(128) float smem[];
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(32 * WWARPS, WWARPS * WROWS == 64 ? 2 : 1)
             // leave no copy in flight into this block's shared memory
             if (threadIdx.x == 0) {
                 mbar_wait_bounded(bar, parity, wait_ns);
-                atomicExch(&g_wide_wait_failed, 1);
+                atomicExch(failed, 1u);
             }
             return;
         }
@@ -762,7 +762,7 @@ typedef void (*TbKernel)(const float *, float *, const float *, const float *, c
                          const uint8_t *, int);
 typedef void (*WideKernel)(const CUtensorMap *, int, float *, const int4 *, int, const int4 *, const int64_t *,
                            const float *, const int32_t *, int, int, int, double *, int, unsigned long long,
-                           int, unsigned long long *, int);
+                           int, unsigned long long *, int, uint32_t *);
 
 TbKernel tb_kernel(int depth) {
     switch (depth) {
@@ -1036,7 +1036,7 @@ int Sor32::sweeps(cw_field_s *f, int n, const int32_t *done, int done_stride, fl
                                  f->g.d_off, omega, done, done_stride, dd, done_half == 0 ? 1 : 0,
                                  apply && last ? f->c : nullptr, f->floor ? 1 : 0,
                                  test_faults().wait_ns ? test_faults().wait_ns : TMA_WAIT_NS, test_faults().skip_tma,
-                                 apply && last ? corr : nullptr, corr_stride));
+                                 apply && last ? corr : nullptr, corr_stride, f->waits));
         } else {
             CW_CUDA(launch_after(done_half > 0, tb_kernel(depth), tiles.nblocks, 32 * WARPS, 0, stream(), a, b,
                                  f->r32, f->inv32, f->g.d_dims, f->g.d_off, tiles.d_blk, f->g.nh, omega, done,
@@ -1063,17 +1063,6 @@ void Sor32::release() {
     wide = false;
     dfree(vtiles);
     vol = false;
-}
-
-// Whether a wide-kernel block gave up waiting for its window (and clears the record).
-int sor32_wait_failed() {
-    int v = 0, zero = 0;
-    CW_CUDA(cudaMemcpyFromSymbol(&v, g_wide_wait_failed, sizeof v));
-    if (v) {
-        CW_CUDA(cudaMemcpyToSymbol(g_wide_wait_failed, &zero, sizeof zero));
-        return fail(CW_ERR_TIMEOUT, "an FP32 SOR block waited too long for its window's TMA copies");
-    }
-    return CW_OK;
 }
 
 }  // namespace cw

@@ -111,6 +111,5 @@ struct Sor32 {
 
 // CW_ERR_TIMEOUT if a wide-kernel block gave up waiting for its window since
 // the last call (synchronous; clears the record).
-int sor32_wait_failed();
 
 }  // namespace cw
