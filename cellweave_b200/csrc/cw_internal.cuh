@@ -66,8 +66,9 @@ class Join {
 // Failure-test settings (cw_test_faults): all off by default.  wait_ns
 // shortens every bounded device wait (grid barriers, meetings, TMA copies) from
 // its 2 s; withhold_block keeps one block of a pass from arriving at its grid
-// barriers, and of a resident FP64 relax at its meetings; max_rounds caps a pass's priority rounds; skip_tma makes the
-// FP32 sweep kernels issue no copy, so that their waits run out.
+// barriers, and of a resident FP64 relax at its meetings; max_rounds caps a
+// pass's priority rounds or its chains' depth; skip_tma makes the FP32 sweep
+// kernels issue no copy, so that their waits run out.
 struct TestFaults {
     unsigned long long wait_ns = 0;
     int32_t withhold_block = -1;

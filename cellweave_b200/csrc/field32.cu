@@ -877,8 +877,8 @@ int wide_init(Sor32 &s, cw_field_s *f, int warps) {
 
 // The volume kernel's tiles: VX x vy columns (halo VD) by chunks of vz slices,
 // an even number: the count of chunks whose waves of tiles march the fewest
-// slices, halo and pipeline included (256^3: 440 tiles of 32 slices, three full
-// waves of 148).
+// slices, halo and pipeline included (256^3: 275 tiles of 52 slices, two waves of
+// 148, 66 steps each).
 int vol_init(Sor32 &s, cw_field_s *f, int window) {
     s.vol = false;
     const Geom &g = f->g;

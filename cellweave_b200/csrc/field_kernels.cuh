@@ -97,7 +97,9 @@ struct Sor32 {
     float *omega = nullptr;
     float *ping = nullptr, *pong = nullptr, *out = nullptr;
     int init(cw_field_s *f, int depth, const std::vector<double> &omega_per_history, int window = CW_WINDOW_AUTO);
-    // n sweeps from the zeroed correction buffer `start` (or the last result);
+    // n sweeps.  Blocked and volume sweeps start from zero, reading neither
+    // buffer; one half-sweep per launch starts from what `start` (or, without it,
+    // the buffer in turn) holds, which the caller has zeroed.
     // `apply` (blocked sweeps): the last launch adds the correction to the field's
     // values instead of writing it, and result() is null
     // corr (optional, apply only): per history, with stride corr_stride, the
@@ -108,8 +110,5 @@ struct Sor32 {
     float *result() const { return out; }
     void release();
 };
-
-// CW_ERR_TIMEOUT if a wide-kernel block gave up waiting for its window since
-// the last call (synchronous; clears the record).
 
 }  // namespace cw

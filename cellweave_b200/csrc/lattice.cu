@@ -10,7 +10,8 @@
 // only through the volume and surface records of cells they share.  A pass
 // runs its attempts as the sequence in a per-pass priority order would (each
 // seeing the records every earlier one left): attempts that share no cell run
-// at once, the others in rounds, in priority order (k_cpm_sweep).  So a pass is
+// at once, those that share one in priority order, each handing the cell's
+// records to the next, or in rounds (k_cpm_sweep).  So a pass is
 // deterministic whatever the thread schedule, and keeps the sequential
 // sweep's volume statistics.  The colours are swept in an order shuffled anew
 // every step.
@@ -582,7 +583,7 @@ __device__ __forceinline__ int plan_find(const int32_t *plan, int nh, int vb) {
 
 // occupied_span (cpm.rs:774-793) of every volume history, at the start of a
 // Monte Carlo step: min and max of x, y, z over the pixels that are not
-// medium (the obstacle counts), reduced per warp, one atomic a warp; then one
+// medium (the obstacle counts), reduced by blocks (span_blocks); then one
 // pixel wider on every side, clipped, or empty (x0 > x1) when all is medium.
 __global__ void k_span_reset(int32_t *span, int nh) {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1689,8 +1690,7 @@ int lattice_recount(cw_lattice_s *l, int32_t *vol_out, int32_t *surf_out) {
 }
 
 // One Monte Carlo step of every history (no host synchronisation): the
-// colour order, then one cooperative launch of every colour's pass (their
-// rounds meet at a grid barrier).
+// colour order, then one cooperative launch of every colour's pass.
 int lattice_span_enqueue(cw_lattice_s *l) {
     if (!l->d_span) return CW_OK;
     Plan &p = l->site_plan;
@@ -1772,7 +1772,8 @@ int lattice_subsweep(cw_lattice_s *l) {
 }
 
 // CW_ERR_TIMEOUT (or CW_ERR_SIMULATION) if a pass gave up since the last
-// call: a grid barrier that waited too long, or more rounds than allowed.
+// call: a grid barrier that waited too long, or more rounds (a deeper chain)
+// than allowed.
 int lattice_pass_error(cw_lattice_s *l) {
     uint32_t e = 0;
     CW_CUDA(cudaMemcpy(&e, l->pctl + CTL_ERR, sizeof e, cudaMemcpyDeviceToHost));

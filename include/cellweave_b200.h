@@ -98,7 +98,9 @@ uint64_t cw_launch_count(void);
  * TMA-copy wait; withhold_block >= 0 keeps that block of each sublattice pass
  * from arriving at its grid barriers, and of an FP64 relax kept on chip at its
  * meetings (the others give up: CW_ERR_TIMEOUT);
- * max_rounds > 0 caps a pass's priority rounds (past it: CW_ERR_SIMULATION);
+ * max_rounds > 0 caps a pass's priority rounds, or how many of its attempts may
+ * follow one another by the cells they share (past it, 256 by default:
+ * CW_ERR_SIMULATION);
  * skip_tma != 0 makes the FP32 sweeps issue no TMA copy, so their waits run
  * out (CW_ERR_TIMEOUT).  Every call replaces all four; (0, -1, 0, 0) is the
  * default.  Work captured in a CUDA graph keeps the settings of its capture. */
@@ -124,9 +126,10 @@ int cw_lattice_destroy(cw_lattice lat);
 int cw_lattice_count(cw_lattice lat, uint32_t *nh);
 /* The cell records history `hist` holds (its capacity, the medium's included). */
 int cw_lattice_capacity(cw_lattice lat, uint32_t hist, uint32_t *cap);
-/* The most rounds a sublattice pass needed since the last call (a pass runs
- * its attempts that share no cell at once, the others in later rounds);
- * resets the count.  A diagnostic; no counterpart in the reference. */
+/* The most rounds a sublattice pass needed since the last call: the longest
+ * chain of its attempts, each behind one that shares a cell with it (up to 1,023
+ * are told apart); resets the count.  A diagnostic; no counterpart in the
+ * reference. */
 int cw_lattice_pass_rounds(cw_lattice lat, uint32_t *rounds);
 /* ContactEnergy (cpm.rs:30-129) generalised to a K x K table over cell types
  * (K <= 8, symmetric, J[0] the medium-medium 0), and set_contact_order
@@ -192,7 +195,9 @@ int cw_lattice_set_mcs(cw_lattice lat, uint32_t mcs);
 int cw_lattice_get_mcs(cw_lattice lat, uint32_t *mcs);
 /* monte_carlo_step (cpm.rs:748-772) `sweeps` times on every history: one
  * copy attempt per pixel per step, made in sublattice passes so that no two
- * concurrent attempts share a contact neighbourhood. */
+ * concurrent attempts share a contact neighbourhood.  The first step takes the
+ * passes' scratch: 152 bytes a pixel of a colour and 516 a cell record, or 56 a
+ * pixel where the former is more than a quarter of the free memory. */
 int cw_lattice_mcs(cw_lattice lat, uint32_t sweeps);
 /* Delta-H (cpm.rs:841-894) of copying dst[k] into site[k] on history
  * `hist` as it stands, for n proposals: out[6k..6k+5] = contact numerator,
