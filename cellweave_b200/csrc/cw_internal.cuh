@@ -405,7 +405,7 @@ struct cw_lattice_s {
     bool lean = false;                    // every pass by rounds, attempts of 3 uint4, no mailboxes or lists
     uint32_t plans = 0;                   // counts the plans made and the scratch taken: a captured sweep holds both
     int64_t plist_cap = 0;
-    int32_t *d_vplan = nullptr;           // nh + 1: the pass plan (first chunk of each history)
+    int32_t *d_vplan = nullptr;           // nh + 2: the pass plan (first chunk of each history, all, useg)
     uint32_t *pctl = nullptr;             // control words, then 27 pass keys per history (lattice.cu)
     int pass_grid = 0;                    // blocks the device holds at once in a cooperative pass launch
     int pass_blocks = 0;                  // blocks of the pass launch

@@ -495,10 +495,10 @@ struct PassScratch {
     uint32_t *count;               // per cell: the attempts listed (zero between passes)
     unsigned long long *chain;     // per cell: CHAIN entries
     uint32_t seg;
-    int32_t useg;                  // pixels a lane of an item reads (1 to UMAX)
     int64_t ncells;
     uint32_t *ctl;                 // CTL_* below, then the pass keys (history x colour)
-    const int32_t *vplan;          // nh + 1: each history's first chunk of PW items; vplan[nh]: all chunks
+    const int32_t *vplan;          // each history's first chunk of PW items; vplan[nh]: all chunks; vplan[nh + 1]: the
+                                   // pixels a lane of an item reads (useg, 1 to UMAX)
     unsigned long long barrier_ns; // a grid barrier's wait limit
     int32_t withhold;              // a block that never arrives at a barrier (failure tests; -1: none)
     int32_t max_rounds;            // rounds before a pass gives up (CW_ERR_SIMULATION)
@@ -615,27 +615,47 @@ __global__ void k_span_finish(int32_t *span, const int4 *dims, int nh) {
     }
 }
 
+// Whether items of 32 `useg` pixels, `nvb` chunks of them against `least` of 32,
+// give every block four chunks and add no more than an eighth to the slots (a
+// history's last chunk is rounded up).
+__host__ __device__ __forceinline__ bool useg_pays(int64_t nvb, int64_t least, int useg, int blocks) {
+    return nvb * useg * 8 <= least * 9 && nvb >= 4 * blocks;
+}
+
 // The pass plan of every volume history from its span: the chunks of PW items
 // the largest colour of the span holds, as a prefix over the histories
-// (vplan[nh] = all of them).  One block: each thread sums a run of
-// histories, the runs' totals are scanned, then each run is written.
-__global__ void __launch_bounds__(1024) k_pass_plan(const int32_t *span, int nh, int period, int useg,
+// (vplan[nh] = all of them), for the largest useg up to `most` that pays.  One
+// block: each thread sums a run of histories, the runs' totals are scanned, then
+// each run is written.  (With the whole box's useg, a tissue of 84^3 in a box of
+// 256^3 had 36 chunks for 148 blocks: 676 us a Monte Carlo step, now 600.)
+__global__ void __launch_bounds__(1024) k_pass_plan(const int32_t *span, int nh, int period, int most, int blocks,
                                                     int32_t *vplan) {
-    __shared__ int32_t s_run[1024];
+    __shared__ int32_t s_run[1024], s_all[UMAX + 1];
     const int per = (nh + blockDim.x - 1) / blockDim.x;
     const int h0 = threadIdx.x * per, h1 = min(h0 + per, nh);
+    int useg = 1;
     auto chunks = [&](int h) -> int32_t {
         const int32_t *s = span + 6 * h;
         const int64_t n = colour_items(s[3] - s[0] + 1, s[4] - s[1] + 1, s[5] - s[2] + 1, period, useg);
         return (int32_t)((n + PW - 1) / PW);
     };
-    int32_t tot = 0;
-    for (int h = h0; h < h1; ++h) tot += chunks(h);
-    s_run[threadIdx.x] = tot;
+    auto mine = [&]() {
+        int32_t tot = 0;
+        for (int h = h0; h < h1; ++h) tot += chunks(h);
+        return tot;
+    };
+    if (threadIdx.x <= UMAX) s_all[threadIdx.x] = 0;
+    __syncthreads();
+    for (useg = 1; useg <= most; useg *= 2)
+        if (const int32_t tot = mine()) atomicAdd(s_all + useg, tot);
+    __syncthreads();
+    for (useg = most; useg > 1 && !useg_pays(s_all[useg], s_all[1], useg, blocks);) useg /= 2;
+    s_run[threadIdx.x] = mine();
     __syncthreads();
     if (threadIdx.x == 0) {
+        vplan[nh + 1] = useg;
         int32_t acc = 0;
-        for (int t = 0; t < (int)blockDim.x; ++t) {
+        for (int t = 0; t < min(nh, (int)blockDim.x); ++t) {  // (the runs behind are empty)
             const int32_t v = s_run[t];
             s_run[t] = acc;
             acc += v;
@@ -747,12 +767,12 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < L.K * L.K; i += PT) P.J[i] = tabs.J[i];
     for (int i = threadIdx.x; i < 3 * L.nreach; i += PT) P.reach[i] = tabs.reach[i];
-    const bool plan_shared = nh + 1 <= PLAN_SMEM;
+    const bool plan_shared = nh + 2 <= PLAN_SMEM;
     if (plan_shared)
-        for (int i = threadIdx.x; i <= nh; i += PT) P.plan[i] = S.vplan[i];
+        for (int i = threadIdx.x; i < nh + 2; i += PT) P.plan[i] = S.vplan[i];
     __syncthreads();
     const int32_t *plan = plan_shared ? P.plan : S.vplan;
-    const int nvb = plan[nh];
+    const int nvb = plan[nh], useg = plan[nh + 1];
     const uint32_t mcs = *mcs_cur;
     const uint32_t *pass_key = S.ctl + CTL_KEYS;
     const uint32_t id0 = blockIdx.x * S.seg;  // this block's first attempt
@@ -851,7 +871,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
 #pragma unroll
                     for (int a = 0; a < 6; ++a) box[a] = __ldg(L.span + 6 * h + a);
                 const uint32_t item = (uint32_t)(vb - plan[h]) * PW + (uint32_t)warp;
-                const ColourItems items((uint32_t)(box[3] - box[0] + 1), L.period, S.useg);
+                const ColourItems items((uint32_t)(box[3] - box[0] + 1), L.period, useg);
                 const ColourRows rows(box, L.period, __ldg(perm + h * L.ncol + pass));
                 if (rows.rows == 0u) continue;
                 const int32_t *const hist = L.grid + __ldg(L.off + h);
@@ -863,12 +883,12 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                 int32_t src[UMAX];
                 auto read = [&](auto packed) {
                     constexpr bool PACKED = decltype(packed)::value;
-                    const uint32_t k0 = item * 32u * (uint32_t)S.useg + (uint32_t)lane;
+                    const uint32_t k0 = item * 32u * (uint32_t)useg + (uint32_t)lane;
                     uint32_t row = 0, j0 = 0;
                     int x = 0, y = 0, z = 0, fx = 0, nx = 0;
                     if (!PACKED) {
                         row = item / items.segs;
-                        j0 = k0 - row * items.segs * 32u * (uint32_t)S.useg;
+                        j0 = k0 - row * items.segs * 32u * (uint32_t)useg;
                         if (row < rows.rows) rows.at(row, y, z, fx, nx);
                     }
                     // the lane's pixel u into (x, y, z); false without one
@@ -881,7 +901,7 @@ __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int
                             if (row < rows.rows) rows.at(row, y, z, fx, nx);
                         }
                         x = fx + rows.step * (int)j;
-                        return u < S.useg && (int)j < nx;
+                        return u < useg && (int)j < nx;
                     };
                     if (!L.copy_moore) {
                         int32_t nb[UMAX][6];
@@ -1536,28 +1556,27 @@ int cw_lattice_s::build_plans() {
     // the pass plan: chunks of PW items, as many as the largest colour of each
     // history's box holds (a plane's plan; in a volume a bound of the plan the
     // device takes from the occupied span every Monte Carlo step).  A lane of an
-    // item reads as many pixels (4, 2 or 1) as still give every block four chunks
-    // and add no more than an eighth to the chunks' pixels (a history's last chunk
-    // is rounded up).
-    std::vector<int32_t> vp(g.nh + 1, 0);
-    auto chunks = [&](int per) {
+    // item reads the most pixels (4, 2 or 1) that pay.
+    std::vector<int32_t> vp(g.nh + 2, 0);
+    auto chunks = [&](int per) -> int64_t {
         for (uint32_t k = 0; k < g.nh; ++k) {
             const int64_t items = colour_items(g.w[k], g.h[k], g.d[k], period, per);
             vp[k + 1] = vp[k] + (int32_t)((items + PW - 1) / PW);
         }
-        return (int64_t)vp[g.nh] * per;
+        return vp[g.nh];
     };
     const int64_t least = chunks(1);
-    for (useg = UMAX; useg > 1; useg /= 2)
-        if (chunks(useg) * 8 <= least * 9 && vp[g.nh] >= 4 * pass_grid) break;
-    if (useg == 1) chunks(1);
+    for (useg = UMAX; useg > 1 && !useg_pays(chunks(useg), least, useg, pass_grid);) useg /= 2;
     // the pass scratch: a block's segment holds every pixel of the chunks it
-    // visits, (chunks / blocks launched, rounded up) items of 32 useg
-    const int32_t nvb = vp[g.nh];
-    pass_blocks = std::max(1, std::min(nvb, pass_grid));
-    pass_seg = (int64_t)((nvb + pass_blocks - 1) / pass_blocks) * PW * 32 * useg;
-    if (!d_vplan && (rc = dalloc(&d_vplan, (size_t)g.nh + 1)) != CW_OK) return rc;
-    CW_CUDA(cudaMemcpyAsync(d_vplan, vp.data(), sizeof(int32_t) * (g.nh + 1), cudaMemcpyHostToDevice, stream()));
+    // visits, (chunks / blocks launched, rounded up) items of 32 useg, in a volume
+    // for every useg that a span may be given
+    pass_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(volume ? least : chunks(useg), pass_grid));
+    pass_seg = 0;
+    for (int u = volume ? 1 : useg; u <= useg; u *= 2)
+        pass_seg = std::max(pass_seg, (chunks(u) + pass_blocks - 1) / pass_blocks * PW * 32 * u);
+    vp[g.nh + 1] = useg;  // (the chunks are useg's: the last counted)
+    if (!d_vplan && (rc = dalloc(&d_vplan, (size_t)g.nh + 2)) != CW_OK) return rc;
+    CW_CUDA(cudaMemcpyAsync(d_vplan, vp.data(), sizeof(int32_t) * (g.nh + 2), cudaMemcpyHostToDevice, stream()));
     if (!pctl) {
         if ((rc = dalloc(&pctl, CTL_KEYS + 27 * (size_t)g.nh)) != CW_OK) return rc;
         CW_CUDA(cudaMemsetAsync(pctl, 0, sizeof(uint32_t) * (CTL_KEYS + 27 * (size_t)g.nh), stream()));
@@ -1708,7 +1727,7 @@ int lattice_span_enqueue(cw_lattice_s *l) {
     CW_LAUNCHED();
     k_span_finish<<<(nh + 127) / 128, 128, 0, stream()>>>(l->d_span, l->g.d_dims, nh);
     CW_LAUNCHED();
-    k_pass_plan<<<1, 1024, 0, stream()>>>(l->d_span, nh, l->period, l->useg, l->d_vplan);
+    k_pass_plan<<<1, 1024, 0, stream()>>>(l->d_span, nh, l->period, l->useg, l->pass_blocks, l->d_vplan);
     CW_LAUNCHED();
     return CW_OK;
 }
@@ -1744,7 +1763,6 @@ int lattice_subsweep(cw_lattice_s *l) {
     S.link = l->pidx + l->plist_cap;
     S.count = l->pcount;
     S.chain = l->pchain;
-    S.useg = l->useg;
     S.seg = (uint32_t)l->pass_seg;
     S.ncells = l->ncells;
     S.ctl = l->pctl;
