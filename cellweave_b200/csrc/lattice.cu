@@ -627,7 +627,7 @@ __host__ __device__ __forceinline__ bool useg_pays(int64_t nvb, int64_t least, i
 // (vplan[nh] = all of them), for the largest useg up to `most` that pays.  One
 // block: each thread sums a run of histories, the runs' totals are scanned, then
 // each run is written.  (With the whole box's useg, a tissue of 84^3 in a box of
-// 256^3 had 36 chunks for 148 blocks: 676 us a Monte Carlo step, now 600.)
+// 256^3 had 36 chunks for 148 blocks: 676 us a Monte Carlo step, now 607.)
 __global__ void __launch_bounds__(1024) k_pass_plan(const int32_t *span, int nh, int period, int most, int blocks,
                                                     int32_t *vplan) {
     __shared__ int32_t s_run[1024], s_all[UMAX + 1];
@@ -754,9 +754,10 @@ struct PassShared {
 // Large lattices are bound by the attempts' lines, 128 bytes each, in the
 // proposals and the terms.  Measured against a launch a pass of rounds only, a
 // Monte Carlo step: a 96^3 ball of 125-voxel cells with surfaces (8 passes, 36
-// attempts deep) 1,750 -> 650 us, the 256^3 spheroid 1,830 -> 667, a 300 x 300
-// tissue (4 sub-sweeps of 2 passes) 840 -> 322, 256 x 256 265 -> 109, the 2048 x
-// 2048 cord 757 -> 426, the campaign's 22.3 M pixels 1,490 -> 1,360.
+// attempts deep) 1,740 -> 574 us, the 256^3 spheroid 1,860 -> 607, a 300 x 300
+// tissue (4 sub-sweeps of 2 passes) 990 -> 378, 256 x 256 290 -> 111, the 2048 x
+// 2048 cord 820 -> 403, the campaign's 22.3 M pixels 1,520 -> 1,150; dense 4096^2
+// and 256^3 lattices as said below.
 template <bool LEAN>
 __global__ void __launch_bounds__(PT, 1) k_cpm_sweep(LatView L, Tables tabs, int nh, const int32_t *perm,
                                                      const uint32_t *mcs_cur, PassScratch S) {
