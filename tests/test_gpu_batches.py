@@ -121,3 +121,23 @@ def test_passes_without_room_for_the_cells_lists(shape, side, order, surface):
     np.testing.assert_array_equal(lat.cells(len(rec))["volume"][1:], o.volume[1:])
     if surface:
         np.testing.assert_array_equal(lat.surfaces(len(rec))[1:], o.surface[1:])
+
+
+# tissues that fill their box, a corner of it, or a few cells in the middle: the
+# pixels a lane reads follow the spans
+@pytest.mark.parametrize("order", [1, 2, 3])
+def test_volumes_whose_tissue_is_a_part_of_the_box(order):
+    boxes = [((200, 60, 56), (0, 0, 0), (200, 60, 56)), ((200, 60, 56), (150, 30, 20), (45, 25, 30)),
+             ((130, 70, 66), (60, 30, 28), (12, 8, 8)), ((96, 96, 96), (1, 1, 1), (90, 90, 90))]
+    for some in (boxes, boxes[1:2], boxes[2:3], boxes[3:]):
+        grids, recs = [], []
+        for (w, h, d), (x, y, z), (sw, sh, sd) in some:
+            part, rec = packed((sw, sh, sd), 4, 6)
+            grid = seeding.empty(w, h, d)
+            grid[z:z + sd, y:y + sh, x:x + sw] = part
+            grids.append(grid)
+            recs.append(rec)
+        lat = cw.CpmLattice.from_grids(grids, recs, 10.0, J3, order, seeds=list(range(50, 50 + len(some))))
+        lat.monte_carlo_step(3)
+        for k in range(len(some)):
+            same_as_the_oracle(lat, k, grids[k], recs[k], order, 3, 50 + k)
